@@ -21,11 +21,11 @@ LIB = HERE / "libcuopo_b200.so"
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden",
-              "--expt-relaxed-constexpr", "-I" + str(INCLUDE), "-I" + str(CSRC)]
+              "--expt-relaxed-constexpr", "-I" + str(INCLUDE), "-I" + str(CSRC), "-I" + str(OBJ)]
 CC_FLAGS = ["-O2", "-fPIC", "-std=c11", "-Wall", "-Wextra", "-fvisibility=hidden", "-I" + str(INCLUDE),
             "-I" + str(CSRC)]
 
-CU_SOURCES = ["solver.cu", "noise.cu", "fft_api.cu", "probe.cu", "mlp.cu", "params_dev.cu"]
+CU_SOURCES = ["kern_f64_3eq.cu", "kern_f64_2eq.cu", "kern_f32_2eq.cu", "kern_f32_3eq.cu", "solver.cu", "noise.cu", "fft_api.cu", "probe.cu", "mlp.cu", "params_dev.cu"]
 # per-file nvcc flags: the device set-up keeps the host's float rounding (no FMA contraction)
 CU_EXTRA = {"params_dev.cu": ["-fmad=false"]}
 C_SOURCES = ["params.c", "dat_io.c"]
@@ -43,7 +43,7 @@ def _cc() -> str:
 
 
 def _deps(src: Path) -> list[Path]:
-    return [src] + sorted(CSRC.glob("*.cuh")) + sorted(CSRC.glob("*.h")) + [INCLUDE / "cuopo.h", Path(__file__)]
+    return [src] + sorted(CSRC.glob("*.cuh")) + sorted(CSRC.glob("*.h")) + [TW_TABLE, INCLUDE / "cuopo.h", Path(__file__)]
 
 
 def _stale(out: Path, deps: list[Path]) -> bool:
@@ -64,9 +64,34 @@ def _run(cmd: list[str], verbose: bool) -> None:
         sys.stderr.write(r.stdout + r.stderr)
 
 
+TW_NS = 512
+TW_TABLE = OBJ / "twiddle_table.inc"
+
+
+def twiddle_rows() -> list[tuple[float, float]]:
+    """(tan(phi/2), sin(phi)) of the six rotations of every k of a radix-16
+    stage of length 512 (csrc/fft.cuh, StageRot), rounded once to FP64."""
+    import numpy as np
+    rows = []
+    for k in range(TW_NS):
+        for mult, quarter in ((1, 0), (2, 0), (3, 0), (4, 0), (8, 1), (12, 1 if 2 * k < TW_NS else 2)):
+            # exact in units of 2 pi / (16 * 512 * 4), pi itself to extended precision
+            units = 4 * mult * k - quarter * 16 * TW_NS
+            phi = np.longdouble(units) * (np.arctan(np.longdouble(1)) * 8) / np.longdouble(64 * TW_NS)
+            rows.append((float(np.tan(phi / 2)), float(np.sin(phi))))
+    return rows
+
+
+def write_twiddle_table() -> None:
+    text = "".join(f"CUOPO_TW({t.hex()}, {s.hex()})\n" for t, s in twiddle_rows())
+    if not TW_TABLE.exists() or TW_TABLE.read_text() != text:
+        TW_TABLE.write_text(text)
+
+
 def build(force: bool = False, verbose: bool = False, ptxas_verbose: bool = False) -> Path:
     """Compiles every CUDA/C source of the library for sm_100a and links the .so."""
     OBJ.mkdir(exist_ok=True)
+    write_twiddle_table()
     jobs = []
     objs = []
     for s in CU_SOURCES:

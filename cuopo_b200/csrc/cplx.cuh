@@ -19,32 +19,64 @@ template <> struct real_of<double2> { using type = double; };
 template <typename C, typename R = typename real_of<C>::type>
 __host__ __device__ __forceinline__ C mk(R re, R im) { C c; c.x = re; c.y = im; return c; }
 
-template <typename C> __host__ __device__ __forceinline__ C cadd(C a, C b) { return mk<C>(a.x + b.x, a.y + b.y); }
-template <typename C> __host__ __device__ __forceinline__ C csub(C a, C b) { return mk<C>(a.x - b.x, a.y - b.y); }
-template <typename C> __host__ __device__ __forceinline__ C cmul(C a, C b)
+/* Real operations that round exactly as written: the compiler fuses
+ * a * b + c on its own where it likes, so two kernels sharing these helpers
+ * would otherwise differ in the last bit.  Every product and sum of the
+ * solver's field arithmetic goes through them; kernels that run the same
+ * operations on another thread layout then give the same bits. */
+__device__ __forceinline__ float rmul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double rmul(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float radd(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ double radd(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ float rfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double rfma(double a, double b, double c) { return __fma_rn(a, b, c); }
+
+template <typename C> __device__ __forceinline__ C cadd(C a, C b) { return mk<C>(radd(a.x, b.x), radd(a.y, b.y)); }
+template <typename C> __device__ __forceinline__ C csub(C a, C b) { return mk<C>(radd(a.x, -b.x), radd(a.y, -b.y)); }
+template <typename C> __device__ __forceinline__ C cmul(C a, C b)
 {
-    return mk<C>(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+    return mk<C>(rfma(a.x, b.x, -rmul(a.y, b.y)), rfma(a.x, b.y, rmul(a.y, b.x)));
 }
 /* a * conj(b) */
-template <typename C> __host__ __device__ __forceinline__ C cmulc(C a, C b)
+template <typename C> __device__ __forceinline__ C cmulc(C a, C b)
 {
-    return mk<C>(a.x * b.x + a.y * b.y, a.y * b.x - a.x * b.y);
+    return mk<C>(rfma(a.x, b.x, rmul(a.y, b.y)), rfma(a.y, b.x, -rmul(a.x, b.y)));
 }
-template <typename C> __host__ __device__ __forceinline__ C cconj(C a) { return mk<C>(a.x, -a.y); }
-template <typename C, typename R> __host__ __device__ __forceinline__ C cscale(C a, R s) { return mk<C>(a.x * s, a.y * s); }
-/* a + s*b */
-template <typename C, typename R> __host__ __device__ __forceinline__ C caxpy(C a, R s, C b)
+/* i * a * a */
+template <typename C> __device__ __forceinline__ C cisq(C a)
 {
-    return mk<C>(a.x + s * b.x, a.y + s * b.y);
+    using R = typename real_of<C>::type;
+    return mk<C>(rmul(rmul((R)-2, a.x), a.y), rfma(a.x, a.x, -rmul(a.y, a.y)));
+}
+/* i * a * b */
+template <typename C> __device__ __forceinline__ C cimul(C a, C b)
+{
+    return mk<C>(rfma(-a.x, b.y, -rmul(a.y, b.x)), rfma(a.x, b.x, -rmul(a.y, b.y)));
+}
+/* i * a * conj(b) */
+template <typename C> __device__ __forceinline__ C cimulc(C a, C b)
+{
+    return mk<C>(rfma(a.x, b.y, -rmul(a.y, b.x)), rfma(a.x, b.x, rmul(a.y, b.y)));
+}
+template <typename C, typename R> __device__ __forceinline__ C cscale(C a, R s) { return mk<C>(rmul(a.x, s), rmul(a.y, s)); }
+/* a + s*b */
+template <typename C, typename R> __device__ __forceinline__ C caxpy(C a, R s, C b)
+{
+    return mk<C>(rfma(s, b.x, a.x), rfma(s, b.y, a.y));
+}
+/* a + a * b: the products added one after the other onto a */
+template <typename C> __device__ __forceinline__ C caddmul(C a, C b)
+{
+    return mk<C>(rfma(-a.y, b.y, rfma(a.x, b.x, a.x)), rfma(a.x, b.y, rfma(a.y, b.x, a.y)));
 }
 /* sign * i * a, sign = +1 or -1 (compile time) */
-template <int S, typename C> __host__ __device__ __forceinline__ C cmul_si(C a)
+template <int S, typename C> __device__ __forceinline__ C cmul_si(C a)
 {
     return S > 0 ? mk<C>(-a.y, a.x) : mk<C>(a.y, -a.x);
 }
-template <typename C> __host__ __device__ __forceinline__ double cabs2d(C a)
+template <typename C> __device__ __forceinline__ double cabs2d(C a)
 {
-    return (double)a.x * (double)a.x + (double)a.y * (double)a.y;
+    return rfma((double)a.x, (double)a.x, rmul((double)a.y, (double)a.y));
 }
 
 /*

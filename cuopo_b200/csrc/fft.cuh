@@ -24,12 +24,22 @@
  * changes the power of a field with random phase to first order; a complex
  * multiplication by float-rounded (cos, sin) does (by |w_f|^2 - 1, a few
  * 1e-8, systematically), and over the ~10^6 transforms of a long cavity run
- * that bias moves the steady-state power by ~1e-4.  A radix-16 stage whose
- * sub-transform length is NS needs W^{r k}, W = exp(2 pi i/(16 NS)),
- * k = t mod NS: with r = b + 4a it applies the rotation by W^{b k} and then
- * a rotations by W^{4k}; the four base angles are all below pi/2.  The
- * last stage keeps its four bases in registers, middle stages read theirs
- * from a small shared-memory table; both are formed in FP64.
+ * that bias moves the steady-state power by ~1e-4.
+ *
+ * A radix-16 stage whose sub-transform length is NS needs W^{r k},
+ * W = exp(2 pi i/(16 NS)), k = t mod NS, on input r = b + 4a of the 4 x 4
+ * transform.  W^{4 a k} depends on a only and W^{b k} on b only, so the
+ * first is applied before the inner 4-point transforms over a, and the
+ * second after them (they are linear), together with their own W16^{b q}:
+ * 12 + 12 rotations and 8 constant ones per 16 points, each input rotated
+ * once by each factor.  (Rotating every input by W^{b k} and then a times by
+ * W^{4k} took 36 and 8: 132 multiply-adds of the 16-point stage's 276
+ * against 96 of 240 here, and up to four roundings in a row against two.)
+ * The six angles of a stage are 1, 2, 3 (below 3 pi/8) and 4, 8, 12 (in
+ * [0, 3 pi/2)) times 2 pi k/(16 NS); the last two are brought into
+ * [-pi/2, pi/2] by a quarter turn that is the same for every k (8) or one of
+ * two (12).  The last stage keeps its six angles in registers, middle
+ * stages read theirs from a small shared-memory table.
  */
 #pragma once
 #include "cplx.cuh"
@@ -64,9 +74,9 @@ __device__ __forceinline__ C iq_rt(C x, int m)
 template <typename C, typename R>
 __device__ __forceinline__ C shear_rot(C x, R t, R s)
 {
-    const R x1 = x.x - t * x.y;
-    const R y2 = x.y + s * x1;
-    const R x3 = x1 - t * y2;
+    const R x1 = rfma(-t, x.y, x.x);
+    const R y2 = rfma(s, x1, x.y);
+    const R x3 = rfma(-t, y2, x1);
     return mk<C>(x3, y2);
 }
 
@@ -129,12 +139,40 @@ __device__ __forceinline__ void dft8(C (&v)[8])
     for (int q = 0; q < 8; q++) v[q] = o[q];
 }
 
-/* 16 = 4 x 4: n = b + 4a, k = q1 + 4 q2. */
+/* The six rotations (tan(phi/2), sin(phi)) of one k of a twiddled radix-16
+ * stage: phi = j kappa for b[j-1] (j = 1, 2, 3) and, for a[0..2], 4 kappa,
+ * 8 kappa - pi/2 and 12 kappa - pi/2 (k < NS/2) or - pi (otherwise),
+ * kappa = 2 pi k / (16 NS). */
+template <typename C>
+struct StageRot {
+    C b[3], a[3];
+};
+
+/* x rotated by the quarter turns of the factor W^{12 k}: one (hi = 0) or two
+ * (hi = 1), in the direction S. */
 template <int S, typename C>
-__device__ __forceinline__ void dft16(C (&v)[16])
+__device__ __forceinline__ C iq12(C x, bool hi)
 {
+    if constexpr (S > 0) return mk<C>(-(hi ? x.x : x.y), hi ? -x.y : x.x);
+    else return mk<C>(hi ? -x.x : x.y, -(hi ? x.y : x.x));
+}
+
+/* 16 = 4 x 4: n = b + 4a, k = q1 + 4 q2.  TW: the stage's twiddles (StageRot
+ * w, hi = k >= NS/2) applied on the way. */
+template <int S, bool TW, typename C>
+__device__ __forceinline__ void dft16(C (&v)[16], const StageRot<C> &w, bool hi)
+{
+    using R = typename real_of<C>::type;
+    const R sg = (R)S;
 #pragma unroll
-    for (int b = 0; b < 4; b++) dft4<S>(v[b], v[b + 4], v[b + 8], v[b + 12]);
+    for (int b = 0; b < 4; b++) {
+        if constexpr (TW) {
+            v[b + 4] = shear_rot(v[b + 4], sg * w.a[0].x, sg * w.a[0].y);
+            v[b + 8] = shear_rot(iq<S>(v[b + 8]), sg * w.a[1].x, sg * w.a[1].y);
+            v[b + 12] = shear_rot(iq12<S>(v[b + 12], hi), sg * w.a[2].x, sg * w.a[2].y);
+        }
+        dft4<S>(v[b], v[b + 4], v[b + 8], v[b + 12]);
+    }
     /* u_b[q1] = v[b + 4 q1] *= W16^{b q1} */
     v[5] = tw16<S, 1>(v[5]);
     v[9] = tw16<S, 2>(v[9]);
@@ -145,6 +183,12 @@ __device__ __forceinline__ void dft16(C (&v)[16])
     v[7] = tw16<S, 3>(v[7]);
     v[11] = tw16<S, 6>(v[11]);
     v[15] = tw16<S, 9>(v[15]);
+    if constexpr (TW) {
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+#pragma unroll
+            for (int b = 1; b < 4; b++) v[4 * q + b] = shear_rot(v[4 * q + b], sg * w.b[b - 1].x, sg * w.b[b - 1].y);
+    }
 #pragma unroll
     for (int q = 0; q < 4; q++) dft4<S>(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
     /* X[q1 + 4 q2] = v[4 q1 + q2] */
@@ -163,7 +207,7 @@ __device__ __forceinline__ void dft(C (&v)[RADIX])
     if constexpr (RADIX == 2) dft2<S>(v[0], v[1]);
     else if constexpr (RADIX == 4) dft4<S>(v[0], v[1], v[2], v[3]);
     else if constexpr (RADIX == 8) dft8<S>(v);
-    else dft16<S>(v);
+    else dft16<S, false>(v, StageRot<C>{}, false);
 }
 
 /* Shared-memory index swizzle: XOR of the low bits with the row number so
@@ -194,52 +238,90 @@ struct StagePlan {
     }
 };
 
-/* Shared-memory table of the middle radix-16 stages 1..P-2: for stage p,
- * base j = 1..4 and k < NS_p the rotation (tan(theta/2), sin(theta)),
- * theta = 2 pi j k / (16 NS_p), stored as [p][j][k]. */
+/* Shared-memory table of the middle radix-16 stages 1..P-2: for stage p and
+ * k < NS_p the six rotations of StageRot, stored as [p][k][6] (16-byte
+ * loads, conflict-free for consecutive k). */
 template <int M>
 struct TwTable {
     using SP = StagePlan<M>;
     static constexpr int offset(int p)
     {
         int o = 0;
-        for (int q = 1; q < p; q++) o += 4 * SP::ns(q);
+        for (int q = 1; q < p; q++) o += 6 * SP::ns(q);
         return o;
     }
     static constexpr int size() { return SP::P > 2 ? offset(SP::P - 1) : 0; }
 };
 
+/* The six rotations of stage length 512, [k][6] (tan, sin), formed in
+ * extended precision when the library is built (build.py): those of a shorter
+ * stage are every (512/NS)-th row.  A kernel that formed its own (FP64
+ * sincospi, 6 per thread and 6 NS per table) spent 5 us of each launch on
+ * them. */
+static constexpr int TW_NS = 512;
+__device__ __align__(16) static const float2 g_tw_f32[6 * TW_NS] = {
+#define CUOPO_TW(t, s) {(float)(t), (float)(s)},
+#include "twiddle_table.inc"
+#undef CUOPO_TW
+};
+__device__ __align__(16) static const double2 g_tw_f64[6 * TW_NS] = {
+#define CUOPO_TW(t, s) {t, s},
+#include "twiddle_table.inc"
+#undef CUOPO_TW
+};
+
+/* Row k of a stage of length ns. */
 template <typename C>
-__device__ __forceinline__ C rot_params(int jk, int den)
+__device__ __forceinline__ const C *tw_row(int k, int ns)
 {
-    using R = typename real_of<C>::type;
-    /* theta = 2 pi jk / den in [0, pi/2): t = tan(theta/2), s = sin(theta) */
-    double sh, ch, sn, cs;
-    sincospi((double)jk / (double)den, &sh, &ch);
-    sincospi(2.0 * (double)jk / (double)den, &sn, &cs);
-    return mk<C>((R)(sh / ch), (R)sn);
+    const int i = 6 * k * (TW_NS / ns);
+    if constexpr (sizeof(C) == 8) return g_tw_f32 + i;
+    else return g_tw_f64 + i;
 }
 
 /* Fills the table (all threads of the CTA cooperate; caller syncs). */
 template <int M, typename C>
-__device__ __forceinline__ void fill_twiddle_table(C *tab, int t)
+__device__ __forceinline__ void fill_twiddle_table(C *tab, int t, int nthreads = StagePlan<M>::T)
 {
     using SP = StagePlan<M>;
 #pragma unroll
     for (int p = 1; p + 1 < SP::P; p++) {
         const int ns = SP::ns(p);
         const int off = TwTable<M>::offset(p);
-        for (int idx = t; idx < 4 * ns; idx += SP::T) {
-            const int j = idx / ns + 1, k = idx % ns;
-            tab[off + idx] = rot_params<C>(j * k, 16 * ns);
-        }
+        for (int idx = t; idx < 6 * ns; idx += nthreads) tab[off + idx] = tw_row<C>(idx / 6, ns)[idx % 6];
     }
 }
 
-/* The last radix-16 stage's four base rotations of thread t. */
+/* Six rotations of one table row, as 16-byte loads (rows are 48 or 96 bytes). */
+__device__ __forceinline__ StageRot<float2> load_rot(const float2 *row)
+{
+    const float4 *q = reinterpret_cast<const float4 *>(row);
+    const float4 u = q[0], v = q[1], w = q[2];
+    StageRot<float2> r;
+    r.b[0] = make_float2(u.x, u.y);
+    r.b[1] = make_float2(u.z, u.w);
+    r.b[2] = make_float2(v.x, v.y);
+    r.a[0] = make_float2(v.z, v.w);
+    r.a[1] = make_float2(w.x, w.y);
+    r.a[2] = make_float2(w.z, w.w);
+    return r;
+}
+
+__device__ __forceinline__ StageRot<double2> load_rot(const double2 *row)
+{
+    StageRot<double2> r;
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+        r.b[j] = row[j];
+        r.a[j] = row[3 + j];
+    }
+    return r;
+}
+
+/* The last radix-16 stage's rotations of thread t. */
 template <int M, typename C>
 struct StageTwiddles {
-    C b1, b2, b3, b4;  /* (tan(theta/2), sin(theta)) of W^k, W^2k, W^3k, W^4k */
+    StageRot<C> last;
     const C *tab;      /* shared-memory table of the middle stages */
     __device__ __forceinline__ void init(int t, const C *table)
     {
@@ -247,33 +329,10 @@ struct StageTwiddles {
         tab = table;
         if constexpr (SP::P > 1) {
             const int ns = SP::ns(SP::P - 1);
-            const int k = t % ns;
-            b1 = rot_params<C>(k, 16 * ns);
-            b2 = rot_params<C>(2 * k, 16 * ns);
-            b3 = rot_params<C>(3 * k, 16 * ns);
-            b4 = rot_params<C>(4 * k, 16 * ns);
+            last = load_rot(tw_row<C>(t % ns, ns));
         }
     }
 };
-
-/* v[4a+b] rotated by S (b k + 4 a k) theta: the rotation by W^{bk}, then a
- * rotations by W^{4k}. */
-template <int S, typename C>
-__device__ __forceinline__ void apply_stage_rotations(C (&v)[16], C b1, C b2, C b3, C b4)
-{
-    using R = typename real_of<C>::type;
-    const R sg = (R)S;
-    const C q[4] = {b1, b1, b2, b3};
-#pragma unroll
-    for (int r = 1; r < 16; r++) {
-        const int b = r & 3, a = r >> 2;
-        C x = v[r];
-        if (b) x = shear_rot(x, sg * q[b].x, sg * q[b].y);
-#pragma unroll
-        for (int i = 0; i < a; i++) x = shear_rot(x, sg * b4.x, sg * b4.y);
-        v[r] = x;
-    }
-}
 
 template <int S, int M, int P_IDX, typename C>
 __device__ __forceinline__ void stage_compute(C (&reg)[16], const StageTwiddles<M, C> &tw)
@@ -289,15 +348,12 @@ __device__ __forceinline__ void stage_compute(C (&reg)[16], const StageTwiddles<
         for (int r = 0; r < R; r++) v[r] = reg[b + r * B];
         if constexpr (NS > 1) {
             static_assert(R == 16, "twiddled stages are radix 16");
-            if constexpr (P_IDX + 1 == SP::P) {
-                apply_stage_rotations<S>(v, tw.b1, tw.b2, tw.b3, tw.b4);
-            } else {
-                const int k = threadIdx.x % NS;
-                const C *row = tw.tab + TwTable<M>::offset(P_IDX) + k;
-                apply_stage_rotations<S>(v, row[0], row[NS], row[2 * NS], row[3 * NS]);
-            }
+            const int k = threadIdx.x % NS;
+            if constexpr (P_IDX + 1 == SP::P) dft16<S, true>(v, tw.last, 2 * k >= NS);
+            else dft16<S, true>(v, load_rot(tw.tab + TwTable<M>::offset(P_IDX) + 6 * k), 2 * k >= NS);
+        } else {
+            dft<S, R>(v);
         }
-        dft<S, R>(v);
 #pragma unroll
         for (int r = 0; r < R; r++) reg[b + r * B] = v[r];
     }

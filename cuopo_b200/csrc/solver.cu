@@ -15,7 +15,7 @@
 
 #include "cuopo.h"
 #include "internal.h"
-#include "ssfm.cuh"
+#include "kernels.cuh"
 
 using namespace cuopo;
 
@@ -29,14 +29,14 @@ struct cuopo_plan {
     int cluster;      /* CTAs per instance */
     size_t smem;      /* dynamic shared memory per CTA */
     void *d_disp;     /* [F][CL][M], entry [f][k2][k1] = D_f(k2 + CL k1) */
-    void *d_rk;       /* [(n_z+1)][NCO] */
+    void *d_rk;       /* [(n_z+1)][4] */
     void *d_eom;      /* [N] or NULL */
     float *d_w;       /* [CL][M], same permutation */
     void *d_twN;      /* [N] W_N^q (cluster plans) or NULL */
     double2 *d_frame_u; /* [NFRAME] random frame angles */
     void *d_frame_c;    /* [NFRAME][3] their phasors */
     int *d_status;
-    double h6;
+    double h6, g_last;
 };
 
 /* ---------------------------------------------------------------- errors */
@@ -61,80 +61,7 @@ extern "C" const char *cuopo_version(void) { return "cuopo_b200 0.1.0 (sm_100a)"
 
 /* -------------------------------------------------------- kernel registry */
 
-typedef cudaError_t (*launch_fn)(const LaunchArgs &, int clusters, cudaStream_t);
-typedef int (*occ_fn)(void);
-
-template <typename R, int F, int M, int CL, int HM, int MINB>
-static cudaError_t prepare_kernel()
-{
-    using K = Ssfm<R, F, M, CL, HM>;
-    static cudaError_t st = [] {
-        cudaError_t e = cudaFuncSetAttribute(ssfm_kernel<R, F, M, CL, HM, MINB>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)K::smem_bytes());
-        if (e == cudaSuccess && CL > 8)
-            e = cudaFuncSetAttribute(ssfm_kernel<R, F, M, CL, HM, MINB>,
-                                     cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        return e;
-    }();
-    return st;
-}
-
-template <typename R, int F, int M, int CL, int HM, int MINB>
-static cudaLaunchConfig_t make_config(int clusters, cudaStream_t st, cudaLaunchAttribute *attr)
-{
-    using K = Ssfm<R, F, M, CL, HM>;
-    cudaLaunchConfig_t cfg;
-    std::memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3((unsigned)(clusters * CL));
-    cfg.blockDim = dim3(K::T);
-    cfg.dynamicSmemBytes = K::smem_bytes();
-    cfg.stream = st;
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = CL;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cfg;
-}
-
-template <typename R, int F, int M, int CL, int HM, int MINB>
-static cudaError_t launch_impl(const LaunchArgs &a, int clusters, cudaStream_t st)
-{
-    cudaError_t e = prepare_kernel<R, F, M, CL, HM, MINB>();
-    if (e != cudaSuccess) return e;
-    cudaLaunchAttribute attr[1];
-    cudaLaunchConfig_t cfg = make_config<R, F, M, CL, HM, MINB>(clusters, st, attr);
-    e = cudaLaunchKernelEx(&cfg, ssfm_kernel<R, F, M, CL, HM, MINB>, a);
-    if (e != cudaSuccess) return e;
-    return cudaGetLastError();
-}
-
-/* Clusters (of CL CTAs) of this kernel that can be resident at once (0 on error). */
-template <typename R, int F, int M, int CL, int HM, int MINB>
-static int occupancy_impl()
-{
-    if (prepare_kernel<R, F, M, CL, HM, MINB>() != cudaSuccess) return 0;
-    cudaLaunchAttribute attr[1];
-    cudaLaunchConfig_t cfg = make_config<R, F, M, CL, HM, MINB>(1, 0, attr);
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, ssfm_kernel<R, F, M, CL, HM, MINB>, &cfg) != cudaSuccess) return 0;
-    return n;
-}
-
-struct KernelEntry {
-    int precision, F, M, CL;
-    int home; /* 0, 1: fields in shared memory (1: in place); 2: in global memory */
-    size_t smem;
-    launch_fn fn;
-    occ_fn occ;
-};
-
-#define CUOPO_K(R, PREC, F, M, CL, HM, MINB)                                                  \
-    {PREC, F, M, CL, HM, Ssfm<R, F, M, CL, HM>::smem_bytes(), &launch_impl<R, F, M, CL, HM, MINB>, \
-     &occupancy_impl<R, F, M, CL, HM, MINB>}
-
-/* Built configurations (R, precision, equations, points per CTA, CTAs per
+/* Built configurations (kern_*.cu: R, precision, equations, points per CTA, CTAs per
  * cluster, field placement as Ssfm's HM, minimum CTAs per SM).  Where a grid
  * size has more than one, cuopo_autotune times them and records the winner;
  * without a recorded choice the first entry with M * CL == n_t is used (the
@@ -143,47 +70,16 @@ struct KernelEntry {
  * CTAs per SM, than as 1, 2 and 4 8192-point CTAs, one per SM).  The
  * single-CTA entries stay reachable for callers that need one
  * (crystal_pass_noalloc). */
-static const KernelEntry k_kernels[] = {
-    CUOPO_K(float, CUOPO_F32, 2, 512, 1, false, 1),
-    CUOPO_K(float, CUOPO_F32, 2, 1024, 1, false, 1),
-    CUOPO_K(float, CUOPO_F32, 2, 2048, 1, false, 1),
-    CUOPO_K(float, CUOPO_F32, 2, 4096, 1, false, 2),
-    CUOPO_K(float, CUOPO_F32, 2, 4096, 2, false, 2),
-    CUOPO_K(float, CUOPO_F32, 2, 8192, 1, false, 1),
-    CUOPO_K(float, CUOPO_F32, 2, 4096, 4, false, 2),
-    CUOPO_K(float, CUOPO_F32, 2, 4096, 8, false, 2),
-    CUOPO_K(float, CUOPO_F32, 2, 8192, 2, false, 1),
-    CUOPO_K(float, CUOPO_F32, 2, 8192, 4, false, 1),
-    CUOPO_K(float, CUOPO_F32, 2, 8192, 8, false, 1),
-    CUOPO_K(float, CUOPO_F32, 3, 512, 1, false, 1),
-    CUOPO_K(float, CUOPO_F32, 3, 1024, 1, false, 1),
-    CUOPO_K(float, CUOPO_F32, 3, 2048, 1, false, 1),
-    CUOPO_K(float, CUOPO_F32, 3, 4096, 1, false, 1),
-    CUOPO_K(float, CUOPO_F32, 3, 8192, 1, true, 1),
-    CUOPO_K(float, CUOPO_F32, 3, 4096, 4, false, 1),
-    CUOPO_K(float, CUOPO_F32, 3, 4096, 8, false, 1),
-    CUOPO_K(float, CUOPO_F32, 3, 4096, 16, false, 1),
-    CUOPO_K(float, CUOPO_F32, 3, 8192, 16, true, 1),
-    CUOPO_K(double, CUOPO_F64, 2, 512, 1, false, 1),
-    CUOPO_K(double, CUOPO_F64, 2, 1024, 1, false, 1),
-    CUOPO_K(double, CUOPO_F64, 2, 2048, 1, false, 1),
-    CUOPO_K(double, CUOPO_F64, 2, 4096, 1, false, 1),
-    CUOPO_K(double, CUOPO_F64, 2, 4096, 2, false, 1),
-    CUOPO_K(double, CUOPO_F64, 2, 4096, 4, false, 1),
-    CUOPO_K(double, CUOPO_F64, 2, 4096, 8, false, 1),
-    CUOPO_K(double, CUOPO_F64, 2, 4096, 16, false, 1),
-    CUOPO_K(double, CUOPO_F64, 3, 512, 1, false, 1),
-    CUOPO_K(double, CUOPO_F64, 3, 1024, 1, false, 1),
-    CUOPO_K(double, CUOPO_F64, 3, 2048, 1, false, 1),
-    CUOPO_K(double, CUOPO_F64, 3, 4096, 1, true, 1),
-    CUOPO_K(double, CUOPO_F64, 3, 4096, 2, true, 1),
-    CUOPO_K(double, CUOPO_F64, 3, 2048, 8, false, 1),
-    CUOPO_K(double, CUOPO_F64, 3, 4096, 8, true, 1),
-    CUOPO_K(double, CUOPO_F64, 3, 4096, 16, true, 1),
-    /* 2^17 FP64 points of 3 fields (6 MiB) exceed the shared memory of a
-     * 16-CTA cluster: the fields stay in global memory (L2) */
-    CUOPO_K(double, CUOPO_F64, 3, 8192, 16, 2, 1),
-};
+static const KernelList *const k_lists[] = {&kern_f32_2eq, &kern_f32_3eq, &kern_f64_2eq, &kern_f64_3eq};
+
+/* Calls f(entry) for every built configuration until it returns true. */
+template <typename Fn>
+static void each_kernel(Fn f)
+{
+    for (const KernelList *l : k_lists)
+        for (int i = 0; i < l->n; i++)
+            if (f(l->k[i])) return;
+}
 
 /* Autotuned choices, process-wide: (precision, F, N) -> entry. */
 struct TunedChoice {
@@ -204,31 +100,17 @@ static const KernelEntry *find_kernel(int precision, int F, int N, bool single_c
         for (const TunedChoice &c : g_tuned)
             if (c.precision == precision && c.F == F && c.N == N) return c.k;
     }
-    for (const KernelEntry &k : k_kernels)
-        if (k.precision == precision && k.F == F && k.M * k.CL == N && (!single_cta || k.CL == 1)) return &k;
-    return nullptr;
+    const KernelEntry *found = nullptr;
+    each_kernel([&](const KernelEntry &k) {
+        if (k.precision == precision && k.F == F && k.M * k.CL == N && (!single_cta || k.CL == 1)) found = &k;
+        return found != nullptr;
+    });
+    return found;
 }
 
 /* ------------------------------------------------------------ host tables */
 
 static int is_pow2i(long n) { return n > 0 && (n & (n - 1)) == 0; }
-
-/* Stage times of the RK4 half steps: z_s accumulated as the reference does
- * (cwes2.cuh:142,209: real_t z += dz), stage offsets dz/4 and dz/2
- * (cwes2.cuh:152,157,162). */
-template <typename ZT>
-static void stage_times(const cuopo_params &p, int s_count, std::vector<double> &zs)
-{
-    zs.resize((size_t)s_count * 3);
-    ZT z = 0;
-    const ZT dz = (ZT)p.dz;
-    for (int s = 0; s < s_count; s++) {
-        zs[3 * s + 0] = (double)z;
-        zs[3 * s + 1] = (double)(ZT)(z + dz / 4);
-        zs[3 * s + 2] = (double)(ZT)(z + dz / 2);
-        z += dz;
-    }
-}
 
 /* sin and cos of a phase: in FP64, or (p32) in FP32 after reducing the
  * argument to [-pi, pi] in FP64 -- the CUOPO_F32_PHASE32 variant, the
@@ -247,11 +129,72 @@ static void phase_sc(double ph, bool p32, double &sn, double &cs)
     }
 }
 
+/* A turn by u [turns] as m quarter turns and the rotation (tan(phi/2),
+ * sin(phi)), |phi| <= pi/4, at out[0] and (m, 0) at out[1]. */
+template <typename R>
+static void turn_entry(double u, bool p32, cpx<R> *out)
+{
+    const double m = std::rint(4.0 * u);
+    const double phi = 2.0 * M_PI * (u - 0.25 * m);
+    if (p32) out[0] = mk<cpx<R>>((R)tanf(0.5f * (float)phi), (R)sinf((float)phi));
+    else out[0] = mk<cpx<R>>((R)std::tan(0.5 * phi), (R)std::sin(phi));
+    out[1] = mk<cpx<R>>((R)(double)((((long)m % 4) + 4) % 4), (R)0);
+}
+
+/* The RK4 half steps of every slice in the pump frame (the row layout is
+ * RkConst's comment in ssfm.cuh): rows 0..n_z of co, the pump frame of the
+ * last slice [turns], h6.  Stage times z_s as the reference accumulates them
+ * (cwes2.cuh:142,209: real_t z += dz), offsets dz/4 and dz/2
+ * (cwes2.cuh:152,157,162). */
+template <typename R>
+static void build_rk_rows(const cuopo_params &p, cpx<R> *co, bool p32, double &h6, double &g_last)
+{
+    using C = cpx<R>;
+    const R dz = (R)p.dz;
+    h6 = (double)(R)(dz / 2) / 6.0;
+    R z = 0;
+    double g_prev = 0.0;   /* the laboratory frame */
+    for (int s = 0; s < p.n_z; s++, z += dz) {
+        const double z0 = (double)z, z1 = (double)(R)(z + dz / 4), z2 = (double)(R)(z + dz / 2);
+        C *row = co + 4 * (size_t)s;
+        double g;
+        if (p.n_eqs == 2) {
+            double sn, cs;
+            phase_sc(p.dk * (z1 - z0), p32, sn, cs);
+            row[0] = mk<C>((R)cs, (R)-sn);
+            phase_sc(p.dk * (z2 - z1), p32, sn, cs);
+            row[1] = mk<C>((R)cs, (R)sn);
+            g = -p.dk * z1 / (2.0 * M_PI);
+        } else {
+            /* E(z) + 4 E(z+dz/4) + E(z+dz/2) = a e^{i 2 pi g} */
+            double er = 0, ei = 0;
+            const double zj[3] = {z0, z1, z2}, wgt[3] = {1.0, 4.0, 1.0};
+            for (int j = 0; j < 3; j++) {
+                double sn, cs;
+                phase_sc(p.dk * zj[j], p32, sn, cs);
+                er += wgt[j] * cs;
+                ei += wgt[j] * sn;
+            }
+            const double a = std::hypot(er, ei);
+            row[0] = mk<C>((R)(h6 * p.kp * a), (R)(h6 * p.ks * a));
+            row[1] = mk<C>((R)(h6 * p.ki * a), (R)0);
+            g = std::atan2(ei, er) / (2.0 * M_PI);
+        }
+        turn_entry<R>(g - g_prev, p32, s == 0 ? co + 4 * (size_t)p.n_z + 2 : row - 4 + 2);
+        g_prev = g;
+    }
+    co[4 * (size_t)p.n_z] = co[4 * (size_t)p.n_z + 1] = mk<C>((R)0, (R)0);
+    /* the last slice is followed by no turn */
+    co[4 * (size_t)(p.n_z - 1) + 2] = co[4 * (size_t)(p.n_z - 1) + 3] = mk<C>((R)0, (R)0);
+    g_last = g_prev - std::rint(g_prev);
+}
+
 template <typename R>
 static std::vector<unsigned char> build_tables(const cuopo_params &p, const float *w, const float *T, int CL,
                                                std::vector<unsigned char> &rk_out,
                                                std::vector<unsigned char> &eom_out,
-                                               std::vector<unsigned char> &twn_out, double &h6, bool p32 = false)
+                                               std::vector<unsigned char> &twn_out, double &h6, double &g_last,
+                                               bool p32 = false)
 {
     using C = cpx<R>;
     const int N = p.n_t;
@@ -306,45 +249,8 @@ static std::vector<unsigned char> build_tables(const cuopo_params &p, const floa
             W[q] = mk<C>((R)std::tan(0.5 * phi), (R)std::sin(phi));
         }
     }
-    /* RK4 stage coefficients per slice (one extra zero row at the end). */
-    const int nco = (F == 2) ? 6 : 3;
-    std::vector<double> zs;
-    if (sizeof(R) == 4) stage_times<float>(p, p.n_z, zs);
-    else stage_times<double>(p, p.n_z, zs);
-    rk_out.assign(sizeof(C) * (size_t)(p.n_z + 1) * nco, 0);
-    C *co = reinterpret_cast<C *>(rk_out.data());
-    const double h = (sizeof(R) == 4) ? (double)(float)((float)p.dz / 2) : p.dz / 2;
-    h6 = h / 6.0;
-    for (int s = 0; s < p.n_z; s++) {
-        if (F == 2) {
-            /* dAdz, cwes2.cuh:37-38: i kp e^{+i dk z}, i ks e^{-i dk z} */
-            for (int j = 0; j < 3; j++) {
-                const double ph = p.dk * zs[3 * s + j];
-                double c, sn;
-                phase_sc(ph, p32, sn, c);
-                co[s * 6 + 2 * j + 0] = mk<C>((R)(-p.kp * sn), (R)(p.kp * c));
-                co[s * 6 + 2 * j + 1] = mk<C>((R)(p.ks * sn), (R)(p.ks * c));
-            }
-        } else {
-            /* dAdz, cwes3.cuh:37-39 with k2 = k3 (Q3): the half step is
-             * A += (h/6) i kappa (E(z) + 4 E(z+dz/4) + E(z+dz/2)) P. */
-            double er = 0, ei = 0;
-            const double wgt[3] = {1.0, 4.0, 1.0};
-            for (int j = 0; j < 3; j++) {
-                double c, sn;
-                phase_sc(p.dk * zs[3 * s + j], p32, sn, c);
-                er += wgt[j] * c;
-                ei += wgt[j] * sn;
-            }
-            /* pump: E- = conj(E+) */
-            const double kap[3] = {p.kp, p.ks, p.ki};
-            for (int f = 0; f < 3; f++) {
-                const double sr = er, si = (f == 0) ? -ei : ei;
-                /* h6 * i * kappa * (sr + i si) = h6 kappa (-si + i sr) */
-                co[s * 3 + f] = mk<C>((R)(h6 * kap[f] * -si), (R)(h6 * kap[f] * sr));
-            }
-        }
-    }
+    rk_out.assign(sizeof(C) * (size_t)(p.n_z + 1) * 4, 0);
+    build_rk_rows<R>(p, reinterpret_cast<C *>(rk_out.data()), p32, h6, g_last);
     /* EOM factor exp(i m sin(2 pi fpm T)), functions.cuh:242-253 */
     eom_out.clear();
     if (p.use_eom) {
@@ -387,10 +293,11 @@ extern "C" cuopo_status cuopo_plan_create(cuopo_plan **out, const cuopo_params *
     }
 
     std::vector<unsigned char> disp, rk, eom, twn;
-    double h6 = 0;
+    double h6 = 0, g_last = 0;
     const int CL = k->CL;
-    if (precision == CUOPO_F32) disp = build_tables<float>(*p, w.data(), T.data(), CL, rk, eom, twn, h6, phase32);
-    else disp = build_tables<double>(*p, w.data(), T.data(), CL, rk, eom, twn, h6);
+    if (precision == CUOPO_F32)
+        disp = build_tables<float>(*p, w.data(), T.data(), CL, rk, eom, twn, h6, g_last, phase32);
+    else disp = build_tables<double>(*p, w.data(), T.data(), CL, rk, eom, twn, h6, g_last);
     /* frequency grid in the same per-CTA order as the dispersion table */
     std::vector<float> wp((size_t)p->n_t);
     for (int q = 0; q < p->n_t; q++) wp[(size_t)(q % CL) * (p->n_t / CL) + q / CL] = w[q];
@@ -406,6 +313,7 @@ extern "C" cuopo_status cuopo_plan_create(cuopo_plan **out, const cuopo_params *
     pl->cluster = k->CL;
     pl->smem = k->smem;
     pl->h6 = h6;
+    pl->g_last = g_last;
     cudaError_t e;
     if ((e = cudaMalloc(&pl->d_disp, disp.size())) != cudaSuccess ||
         (e = cudaMalloc(&pl->d_rk, rk.size())) != cudaSuccess ||
@@ -501,6 +409,9 @@ static LaunchArgs base_args(const cuopo_plan *pl)
     a.tab.frame_u = pl->d_frame_u;
     a.tab.frame_c = pl->d_frame_c;
     a.tab.h6 = pl->h6;
+    a.tab.kp = pl->p.kp;
+    a.tab.ks = pl->p.ks;
+    a.tab.g_last = pl->g_last;
     a.tab.inv_n = 1.0 / (double)pl->N;
     a.n_z = pl->p.n_z;
     a.regime = pl->p.regime;
@@ -865,6 +776,9 @@ static cuopo_status batch_build(cuopo_batch **out, const std::vector<cuopo_param
             I.w = pl->d_w;
             I.eom = (p.use_eom && pl->d_eom) ? pl->d_eom : nullptr;
             I.h6 = pl->h6;
+            I.kp = p.kp;
+            I.ks = p.ks;
+            I.g_last = pl->g_last;
             I.st_ps = b->d_ps + i;
             I.st_rt = b->d_rt + i;
             I.st_flag = b->d_flag + i;
@@ -1104,8 +1018,10 @@ extern "C" cuopo_status cuopo_autotune(const cuopo_params *base, int precision, 
     if (!base || count < 1 || n_rt < 1) return cuopo_fail(CUOPO_EINVAL, "autotune: bad argument");
     const int F = base->n_eqs, N = base->n_t;
     std::vector<const KernelEntry *> cand;
-    for (const KernelEntry &k : k_kernels)
+    each_kernel([&](const KernelEntry &k) {
         if (k.precision == precision && k.F == F && k.M * k.CL == N) cand.push_back(&k);
+        return false;
+    });
     if (cand.empty()) return cuopo_fail(CUOPO_EUNSUPPORTED, "autotune: no kernel built for this (precision, n_eqs, n_t)");
     const KernelEntry *best = cand[0];
     double best_ms = -1.0;
@@ -1179,18 +1095,23 @@ extern "C" cuopo_status cuopo_autotune(const cuopo_params *base, int precision, 
 
 extern "C" cuopo_status cuopo_kernel_select(int precision, int n_eqs, int n_t, int points_per_cta, int cluster)
 {
-    for (const KernelEntry &k : k_kernels)
+    const KernelEntry *found = nullptr;
+    each_kernel([&](const KernelEntry &k) {
         if (k.precision == precision && k.F == n_eqs && k.M == points_per_cta && k.CL == cluster &&
-            k.M * k.CL == n_t) {
-            std::lock_guard<std::mutex> lock(g_tune_mu);
-            for (TunedChoice &c : g_tuned)
-                if (c.precision == precision && c.F == n_eqs && c.N == n_t) {
-                    c.k = &k;
-                    return CUOPO_OK;
-                }
-            g_tuned.push_back(TunedChoice{precision, n_eqs, n_t, &k});
-            return CUOPO_OK;
-        }
+            k.M * k.CL == n_t)
+            found = &k;
+        return found != nullptr;
+    });
+    if (found) {
+        std::lock_guard<std::mutex> lock(g_tune_mu);
+        for (TunedChoice &c : g_tuned)
+            if (c.precision == precision && c.F == n_eqs && c.N == n_t) {
+                c.k = found;
+                return CUOPO_OK;
+            }
+        g_tuned.push_back(TunedChoice{precision, n_eqs, n_t, found});
+        return CUOPO_OK;
+    }
     return cuopo_fail(CUOPO_EUNSUPPORTED, "kernel_select: no such built configuration");
 }
 
@@ -1248,13 +1169,13 @@ extern "C" cuopo_status cuopo_crystal_pass_noalloc(const cuopo_params *p, const 
         return cuopo_fail(CUOPO_EINVAL, "crystal_pass_noalloc: n_z must be in [1, 1024]");
     const KernelEntry *k = find_kernel(CUOPO_F32, p->n_eqs, p->n_t, true);
     if (!k) return cuopo_fail(CUOPO_EUNSUPPORTED, "crystal_pass_noalloc: no single-CTA kernel for n_t");
-    const int N = p->n_t, F = p->n_eqs, nco = (F == 2) ? 6 : 3;
+    const int N = p->n_t, F = p->n_eqs;
 
     /* layout of the scratch array (bytes, 256-aligned pieces) */
     auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
     const size_t o_disp = 0;
     const size_t o_rk = o_disp + up(sizeof(float2) * (size_t)F * N);
-    const size_t o_w = o_rk + up(sizeof(float2) * (size_t)(p->n_z + 1) * nco);
+    const size_t o_w = o_rk + up(sizeof(float2) * (size_t)(p->n_z + 1) * 4);
     const size_t o_fu = o_w + up(sizeof(float) * (size_t)N);
     const size_t o_fc = o_fu + up(sizeof(double2) * NFRAME);
     const size_t o_st = o_fc + up(sizeof(float2) * 3 * NFRAME);
@@ -1309,35 +1230,8 @@ extern "C" cuopo_status cuopo_crystal_pass_noalloc(const cuopo_params *p, const 
             Dt[(size_t)f * N + q] = make_float2((float)dre, (float)(a * std::sin(ph)));
         }
     }
-    /* RK4 stage coefficients (z accumulated in float, as the reference) */
-    float2 *co = (float2 *)(H + o_rk);
-    std::memset(co, 0, sizeof(float2) * (size_t)(p->n_z + 1) * nco);
-    const double h6 = (double)(float)((float)p->dz / 2) / 6.0;
-    float z = 0;
-    const float dzf = (float)p->dz;
-    for (int s = 0; s < p->n_z; s++) {
-        const double zj[3] = {(double)z, (double)(float)(z + dzf / 4), (double)(float)(z + dzf / 2)};
-        if (F == 2) {
-            for (int j = 0; j < 3; j++) {
-                const double ph = p->dk * zj[j], c = std::cos(ph), sn = std::sin(ph);
-                co[s * 6 + 2 * j + 0] = make_float2((float)(-p->kp * sn), (float)(p->kp * c));
-                co[s * 6 + 2 * j + 1] = make_float2((float)(p->ks * sn), (float)(p->ks * c));
-            }
-        } else {
-            double er = 0, ei = 0;
-            const double wgt[3] = {1.0, 4.0, 1.0};
-            for (int j = 0; j < 3; j++) {
-                er += wgt[j] * std::cos(p->dk * zj[j]);
-                ei += wgt[j] * std::sin(p->dk * zj[j]);
-            }
-            const double kap[3] = {p->kp, p->ks, p->ki};
-            for (int f = 0; f < 3; f++) {
-                const double si = (f == 0) ? -ei : ei;
-                co[s * 3 + f] = make_float2((float)(h6 * kap[f] * -si), (float)(h6 * kap[f] * er));
-            }
-        }
-        z += dzf;
-    }
+    double h6, g_last;
+    build_rk_rows<float>(*p, (float2 *)(H + o_rk), false, h6, g_last);
     /* random frame table (same fixed sequence as the plans') */
     double2 *fu = (double2 *)(H + o_fu);
     float2 *fc = (float2 *)(H + o_fc);
@@ -1372,6 +1266,9 @@ extern "C" cuopo_status cuopo_crystal_pass_noalloc(const cuopo_params *p, const 
     a.tab.frame_u = (const double2 *)(D + o_fu);
     a.tab.frame_c = D + o_fc;
     a.tab.h6 = h6;
+    a.tab.kp = p->kp;
+    a.tab.ks = p->ks;
+    a.tab.g_last = g_last;
     a.tab.inv_n = 1.0 / (double)N;
     a.n_z = p->n_z;
     a.regime = p->regime;

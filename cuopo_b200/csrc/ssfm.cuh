@@ -32,7 +32,7 @@
  * Quirks kept: RK4 stages use aux = A + s k without the step (Q1); both
  * half steps of a slice use the same z (Q2); in the 3-equation model all
  * stages read the unperturbed fields (Q3), so the half step reduces to
- * A += c(z) * P(A) with one complex coefficient per field and slice.
+ * A += c(z) * P(A) with one coefficient per field and slice.
  */
 #pragma once
 #include <cooperative_groups.h>
@@ -46,13 +46,15 @@ namespace cuopo {
  * index k2 + CL k1. */
 struct Tables {
     const void *disp;   /* [F][CL][M]: slice dispersion x attenuation / N */
-    const void *rk;     /* [n_z + 1][6] (2 eqs) or [n_z + 1][3] (3 eqs) RK4 coefficients */
+    const void *rk;     /* [n_z + 1][4]: RK4 half steps, see RkRow */
     const void *eom;    /* [N]: exp(i m sin(2 pi fpm T)) or NULL */
     const float *w;     /* [CL][M]: angular frequency grid (reference float values) */
     const void *twN;    /* [N]: W_N^q (cross-stage twiddles; CL > 1) */
     const double2 *frame_u; /* [NFRAME]: random frame angles (u_s, u_i) in turns, |u| < 1/8 */
     const void *frame_c;    /* [NFRAME][3]: rotation (tan, sin) for pump, signal, idler */
     double h6;          /* (dz/2)/6 */
+    double kp, ks;      /* 2 eqs: couplings */
+    double g_last;      /* pump frame of the last slice [turns] */
     double inv_n;       /* 1/N */
 };
 
@@ -87,7 +89,7 @@ struct Instance {
      * crystal, wavelengths, length or modulator); NULL disp: the launch's */
     const void *disp, *rk, *eom;
     const float *w;
-    double h6;
+    double h6, kp, ks, g_last;
 };
 
 struct LaunchArgs {
@@ -134,43 +136,62 @@ __device__ __forceinline__ C ldc(const void *p, long i)
     return __ldg(reinterpret_cast<const C *>(p) + i);
 }
 
-/* RK4 half step, 2 equations: cwes2.cuh:30-87 with stage coefficients
- * co = {i kp e^{+i dk z_j}, i ks e^{-i dk z_j}}, z_j = z, z+dz/4, z+dz/2. */
+/*
+ * RK4 half steps in the pump frame.  The stage coefficients of slice s are
+ * i kp e^{+i dk z_j} and i ks e^{-i dk z_j} (z_j = z, z+dz/4, z+dz/2), so with
+ * the pump turned by g_s = -dk (z_s + dz/4) the two middle stages have no
+ * phase at all and the outer two e1 = e^{-i dk dz/4} and e2 = e^{i dk dz/4}
+ * or their conjugates; kp, ks go into the scalars of the updates.  That is
+ * 76 multiply-adds per point and half step against 96 with a complex
+ * coefficient per stage, for one more rotation of the pump per slice (3).
+ * The 3-equation half step (one coefficient h6 i kappa_f (E(z) +
+ * 4 E(z+dz/4) + E(z+dz/2)) per field, E conjugate for the pump) becomes
+ * purely imaginary in the frame of that sum's phase: 18 against 30.  The
+ * kernel's other steps commute with a constant turn of the pump.
+ *
+ * Row s < n_z of the table, 4 complex entries:
+ *   2 eqs: e1, e2;  3 eqs: (c_p, c_s), (c_i, 0) with A_f += i c_f P_f
+ *   (tan(phi/2), sin(phi)) and (m, 0): the turn of the pump from the frame of
+ *   slice s to that of slice s+1 as m quarter turns and a rotation phi;
+ * row n_z holds the turn from the laboratory frame into slice 0's.
+ */
+template <typename R>
+struct RkConst {
+    R hp, hs, fp, fs, gp, gs;   /* kappa/2, kappa, h6 kappa */
+};
+
+/* 2 equations: cwes2.cuh:30-87. */
 template <typename C, typename R>
-__device__ __forceinline__ void rk4_half2(C &Ap, C &As, const C *__restrict__ co, R h6)
+__device__ __forceinline__ void rk4_half2(C &Ap, C &As, C e1, C e2, const RkConst<R> &k)
 {
-    const C k1p = cmul(co[0], cmul(As, As));
-    const C k1s = cmul(co[1], cmulc(Ap, As));
-    C ap = caxpy(Ap, (R)0.5, k1p), as = caxpy(As, (R)0.5, k1s);
-    const C k2p = cmul(co[2], cmul(as, as));
-    const C k2s = cmul(co[3], cmulc(ap, as));
-    ap = caxpy(Ap, (R)0.5, k2p);
-    as = caxpy(As, (R)0.5, k2s);
-    const C k3p = cmul(co[2], cmul(as, as));
-    const C k3s = cmul(co[3], cmulc(ap, as));
-    ap = cadd(Ap, k3p);
-    as = cadd(As, k3s);
-    const C k4p = cmul(co[4], cmul(as, as));
-    const C k4s = cmul(co[5], cmulc(ap, as));
-    const C sp = cadd(cadd(k1p, k4p), cscale(cadd(k2p, k3p), (R)2));
-    const C ss = cadd(cadd(k1s, k4s), cscale(cadd(k2s, k3s), (R)2));
-    Ap = caxpy(Ap, h6, sp);
-    As = caxpy(As, h6, ss);
+    const C g1p = cmul(cisq(As), e1);
+    const C g1s = cmulc(cimulc(Ap, As), e1);
+    C ap = caxpy(Ap, k.hp, g1p), as = caxpy(As, k.hs, g1s);
+    const C g2p = cisq(as);
+    const C g2s = cimulc(ap, as);
+    ap = caxpy(Ap, k.hp, g2p);
+    as = caxpy(As, k.hs, g2s);
+    const C g3p = cisq(as);
+    const C g3s = cimulc(ap, as);
+    ap = caxpy(Ap, k.fp, g3p);
+    as = caxpy(As, k.fs, g3s);
+    const C g4p = cmul(cisq(as), e2);
+    const C g4s = cmulc(cimulc(ap, as), e2);
+    Ap = caxpy(Ap, k.gp, caxpy(cadd(g1p, g4p), (R)2, cadd(g2p, g3p)));
+    As = caxpy(As, k.gs, caxpy(cadd(g1s, g4s), (R)2, cadd(g2s, g3s)));
 }
 
-/* RK4 half step, 3 equations: cwes3.cuh:30-90 with Q3, folded to
- * A_f += co_f * P_f where P = (As Ai, Ap conj(Ai), Ap conj(As)). */
+/* 3 equations: cwes3.cuh:30-90 with Q3, P = (As Ai, Ap conj(Ai), Ap conj(As)). */
 template <typename C>
-__device__ __forceinline__ void rk4_half3(C &Ap, C &As, C &Ai, const C *__restrict__ co)
+__device__ __forceinline__ void rk4_half3(C &Ap, C &As, C &Ai, C c0, C c1)
 {
-    const C Pp = cmul(As, Ai);
-    const C Ps = cmulc(Ap, Ai);
-    const C Pi = cmulc(Ap, As);
-    Ap = cadd(Ap, cmul(co[0], Pp));
-    As = cadd(As, cmul(co[1], Ps));
-    Ai = cadd(Ai, cmul(co[2], Pi));
+    const C Pp = cimul(As, Ai);
+    const C Ps = cimulc(Ap, Ai);
+    const C Pi = cimulc(Ap, As);
+    Ap = caxpy(Ap, c0.x, Pp);
+    As = caxpy(As, c0.y, Ps);
+    Ai = caxpy(Ai, c1.x, Pi);
 }
-
 
 namespace cg = cooperative_groups;
 
@@ -193,7 +214,7 @@ struct Ssfm {
     static constexpr int P = SP::P;
     static constexpr int N = M * CL;
     static constexpr int J = 16 / CL;  /* n1 values per thread in a cross stage */
-    static constexpr int NCO = (F == 2) ? 6 : 3;
+    static constexpr int NCO = 4;      /* entries of a row of the RK4 table */
     static constexpr unsigned ALL = (1u << F) - 1u;
     static_assert(CL == 1 || CL == 2 || CL == 4 || CL == 8 || CL == 16, "cluster size must be 1..16, power of 2");
 
@@ -206,9 +227,10 @@ struct Ssfm {
     struct Ops {
         int inject;         /* pump injection */
         long poff;          /* NS pump window offset of this round trip */
-        const C *rk0, *rk1; /* RK4 half steps to apply (NULL: none) */
+        const C *rk0, *rk1; /* rows of the RK4 half steps to apply (NULL: none) */
+        const C *turn;      /* row whose turn of the pump comes between the two (NULL: none) */
         int eom;            /* intracavity phase modulator */
-        int rotate;         /* frame rotation: quarter turns rq[f], then the shear rotation rf[f] */
+        int rotate;         /* frame rotation: 1 the shear rotations rf[f], 2 quarter turns rq[f] first */
         C rf[3];
         int rq[3];
         int addphase;       /* AddPhase on the resonant fields */
@@ -219,17 +241,15 @@ struct Ssfm {
     };
 
     /* Move to the frame of table entry q (rotation by 2 pi u per field, built
-     * from shears); th accumulates each field's frame angle in turns. */
+     * from shears); th accumulates each field's frame angle in turns
+     * (the pump's starts at the RK4 frame of the last slice). */
     static __device__ __forceinline__ void frame_step(Ops &op, const Tables &tab, int q, double (&th)[3])
     {
         const C *fc = reinterpret_cast<const C *>(tab.frame_c) + 3 * q;
         const double2 u = tab.frame_u[q];
         op.rotate = 1;
 #pragma unroll
-        for (int f = 0; f < 3; f++) {
-            op.rf[f] = fc[f];
-            op.rq[f] = 0;
-        }
+        for (int f = 0; f < 3; f++) op.rf[f] = fc[f];
         th[1] += u.x;
         th[2] += u.y;
         th[0] += (F == 2) ? 2.0 * u.x : u.x + u.y;
@@ -239,7 +259,7 @@ struct Ssfm {
      * residual of at most 1/8 turn, formed in FP64. */
     static __device__ __forceinline__ void frame_back(Ops &op, const double (&th)[3])
     {
-        op.rotate = 1;
+        op.rotate = 2;
 #pragma unroll
         for (int f = 0; f < 3; f++) {
             const double back = -th[f];
@@ -296,35 +316,70 @@ struct Ssfm {
 
     static __device__ __forceinline__ C mul_fp64(C a, double2 f)
     {
-        const double re = (double)a.x * f.x - (double)a.y * f.y;
-        const double im = (double)a.x * f.y + (double)a.y * f.x;
+        const double re = rfma((double)a.x, f.x, -rmul((double)a.y, f.y));
+        const double im = rfma((double)a.x, f.y, rmul((double)a.y, f.x));
         return mk<C>((R)re, (R)im);
     }
 
-    /* co0 / co1: the coefficients of op.rk0 / op.rk1, loaded once per cross
-     * pass (through a pointer they would be reloaded for every point: the
-     * shared-memory stores between points may alias it for the compiler) */
-    static __device__ __forceinline__ void pointwise(C (&A)[3], int n, const Ops &op, const C (&co0)[NCO],
-                                                     const C (&co1)[NCO], const Instance &I, const Tables &tab, R h6,
-                                                     int eom_idler, double &acc)
+    /* Table entries of one cross pass, loaded once (through a pointer they
+     * would be reloaded for every point: the shared-memory stores between
+     * points may alias it for the compiler). */
+    struct Coef {
+        C a0, a1, b0, b1;   /* the two half steps */
+        C turn;             /* turn of the pump between them: rotation, quarter turns */
+        int turn_q;
+        RkConst<R> k;
+    };
+
+    static __device__ __forceinline__ Coef load_coef(const Ops &op, const RkConst<R> &k)
     {
-        if (op.inject) A[0] = I.pump ? ldc<C>(I.pump, op.poff + n) : mk<C>((R)I.ap0, (R)0);
+        Coef c;
+        c.a0 = c.a1 = c.b0 = c.b1 = c.turn = mk<C>((R)0, (R)0);
+        c.turn_q = 0;
+        c.k = k;
         if (op.rk0) {
-            if constexpr (F == 2) rk4_half2(A[0], A[1], co0, h6);
-            else rk4_half3(A[0], A[1], A[2], co0);
+            c.a0 = ldc<C>(op.rk0, 0);
+            c.a1 = ldc<C>(op.rk0, 1);
         }
         if (op.rk1) {
-            if constexpr (F == 2) rk4_half2(A[0], A[1], co1, h6);
-            else rk4_half3(A[0], A[1], A[2], co1);
+            c.b0 = ldc<C>(op.rk1, 0);
+            c.b1 = ldc<C>(op.rk1, 1);
         }
+        if (op.turn) {
+            c.turn = ldc<C>(op.turn, 2);
+            c.turn_q = (int)ldc<C>(op.turn, 3).x;
+        }
+        return c;
+    }
+
+    static __device__ __forceinline__ void half_step(C (&A)[3], C c0, C c1, const RkConst<R> &k)
+    {
+        if constexpr (F == 2) rk4_half2(A[0], A[1], c0, c1, k);
+        else rk4_half3(A[0], A[1], A[2], c0, c1);
+    }
+
+    static __device__ __forceinline__ void pointwise(C (&A)[3], int n, const Ops &op, const Coef &co,
+                                                     const Instance &I, const Tables &tab, int eom_idler, double &acc)
+    {
+        if (op.inject) A[0] = I.pump ? ldc<C>(I.pump, op.poff + n) : mk<C>((R)I.ap0, (R)0);
+        if (op.rk0) half_step(A, co.a0, co.a1, co.k);
+        if (op.turn) {
+            if (co.turn_q) A[0] = iq_rt(A[0], co.turn_q);
+            A[0] = shear_rot(A[0], co.turn.x, co.turn.y);
+        }
+        if (op.rk1) half_step(A, co.b0, co.b1, co.k);
         if (op.eom) {
             const C ef = ldc<C>(tab.eom, n);
             A[1] = cmul(A[1], ef);
             if (F == 3 && eom_idler) A[F - 1] = cmul(A[F - 1], ef);
         }
         if (op.rotate) {
+            if (op.rotate == 2) {
 #pragma unroll
-            for (int f = 0; f < F; f++) A[f] = shear_rot(iq_rt(A[f], op.rq[f]), op.rf[f].x, op.rf[f].y);
+                for (int f = 0; f < F; f++) A[f] = iq_rt(A[f], op.rq[f]);
+            }
+#pragma unroll
+            for (int f = 0; f < F; f++) A[f] = shear_rot(A[f], op.rf[f].x, op.rf[f].y);
         }
         if (op.addphase) {
             /* in FP64 so that sqrt(R) exp(i pi delta) carries no float rounding
@@ -379,16 +434,11 @@ struct Ssfm {
      * reads and writes only its own positions, so these steps need no
      * barrier between them. */
     static __device__ __forceinline__ void cross_global(C *const (&gf)[3], unsigned in_y, unsigned out_y,
-                                                        const Ops &op, const Instance &I, const Tables &tab, R h6,
-                                                        int eom_idler, double &acc, int t, int rank)
+                                                        const Ops &op, const Instance &I, const Tables &tab,
+                                                        const RkConst<R> &rkc, int eom_idler, double &acc, int t, int rank)
     {
         const C *__restrict__ twN = reinterpret_cast<const C *>(tab.twN);
-        C co0[NCO], co1[NCO];
-#pragma unroll
-        for (int k = 0; k < NCO; k++) {
-            co0[k] = op.rk0 ? ldc<C>(op.rk0, k) : mk<C>((R)0, (R)0);
-            co1[k] = op.rk1 ? ldc<C>(op.rk1, k) : mk<C>((R)0, (R)0);
-        }
+        const Coef co = load_coef(op, rkc);
 #pragma unroll 1
         for (int j = 0; j < J; j++) {
             const int n1 = rank * (M / CL) + t + j * T;
@@ -402,7 +452,7 @@ struct Ssfm {
                 C A[3];
 #pragma unroll
                 for (int f = 0; f < F; f++) A[f] = __ldcg(gf[f] + (size_t)c * M + n1);
-                pointwise(A, n1 + M * c, op, co0, co1, I, tab, h6, eom_idler, acc);
+                pointwise(A, n1 + M * c, op, co, I, tab, eom_idler, acc);
 #pragma unroll
                 for (int f = 0; f < F; f++) __stcg(gf[f] + (size_t)c * M + n1, A[f]);
             }
@@ -420,20 +470,15 @@ struct Ssfm {
      * of CTA `rank` owns positions n1 = rank M/CL + t + j T, j < J, in every
      * CTA's home; it reads and writes only those. */
     static __device__ __forceinline__ void cross(C *home, C *const (&gf)[3], unsigned in_y, unsigned out_y,
-                                                 const Ops &op, const Instance &I, const Tables &tab, R h6,
-                                                 int eom_idler, double &acc, int t, int rank)
+                                                 const Ops &op, const Instance &I, const Tables &tab,
+                                                 const RkConst<R> &rkc, int eom_idler, double &acc, int t, int rank)
     {
         if constexpr (GH) {
-            cross_global(gf, in_y, out_y, op, I, tab, h6, eom_idler, acc, t, rank);
+            cross_global(gf, in_y, out_y, op, I, tab, rkc, eom_idler, acc, t, rank);
             return;
         }
         const C *__restrict__ twN = reinterpret_cast<const C *>(tab.twN);
-        C co0[NCO], co1[NCO];
-#pragma unroll
-        for (int k = 0; k < NCO; k++) {
-            co0[k] = op.rk0 ? ldc<C>(op.rk0, k) : mk<C>((R)0, (R)0);
-            co1[k] = op.rk1 ? ldc<C>(op.rk1, k) : mk<C>((R)0, (R)0);
-        }
+        const Coef co = load_coef(op, rkc);
 #pragma unroll 1
         for (int j = 0; j < J; j++) {
             const int n1 = rank * (M / CL) + t + j * T;
@@ -467,7 +512,7 @@ struct Ssfm {
                 C A[3];
 #pragma unroll
                 for (int f = 0; f < F; f++) A[f] = v[f][c];
-                pointwise(A, n1 + M * c, op, co0, co1, I, tab, h6, eom_idler, acc);
+                pointwise(A, n1 + M * c, op, co, I, tab, eom_idler, acc);
 #pragma unroll
                 for (int f = 0; f < F; f++) v[f][c] = A[f];
             }
@@ -518,21 +563,19 @@ struct Ssfm {
         if constexpr (MODE == 0) {
 #pragma unroll
             for (int e = 0; e < 16; e++) {
-                const C x = cscale(reg[e], s_n);
-                reg[e] = cadd(x, cmul(x, __ldg(row + t + e * T)));
+                reg[e] = caddmul(cscale(reg[e], s_n), __ldg(row + t + e * T));
             }
         } else {
 #pragma unroll 4
             for (int e = 0; e < 16; e++) {
                 /* functions.cuh:156-186, formed in FP64 */
                 const double wk = (double)__ldg(w + t + e * T);
-                const double ph = use_tod ? 0.5 * wk * (wk * gdd + wk * wk * tod / 3.0) : 0.5 * wk * wk * gdd;
+                const double ph = use_tod ? 0.5 * wk * rfma(wk, gdd, rmul(wk * wk, tod) / 3.0) : 0.5 * wk * wk * gdd;
                 double sn, cs;
                 sincos(ph, &sn, &cs);
                 /* cos(ph) - 1 = -2 sin^2(ph/2), exact for small ph */
                 const double sh = sin(0.5 * ph);
-                const C x = cscale(reg[e], s_n);
-                reg[e] = cadd(x, cmul(x, mk<C>((R)(-2.0 * sh * sh), (R)sn)));
+                reg[e] = caddmul(cscale(reg[e], s_n), mk<C>((R)(-2.0 * sh * sh), (R)sn));
             }
         }
         local_transform<-1, M, P - 1, INPLACE>(reg, bufA, bufB, tw, t);
@@ -599,10 +642,19 @@ struct Ssfm {
                 tab.rk = I.rk;
                 tab.w = I.w;
                 tab.h6 = I.h6;
+                tab.kp = I.kp;
+                tab.ks = I.ks;
+                tab.g_last = I.g_last;
                 tab.eom = I.eom;
                 use_eom = I.eom != nullptr;
             }
-            const R h6 = (R)tab.h6;
+            RkConst<R> rkc;
+            rkc.hp = (R)(0.5 * tab.kp);
+            rkc.hs = (R)(0.5 * tab.ks);
+            rkc.fp = (R)tab.kp;
+            rkc.fs = (R)tab.ks;
+            rkc.gp = (R)(tab.h6 * tab.kp);
+            rkc.gs = (R)(tab.h6 * tab.ks);
             const C *__restrict__ rk = reinterpret_cast<const C *>(tab.rk);
             const C *__restrict__ disp = reinterpret_cast<const C *>(tab.disp);
             const float *__restrict__ wtab = tab.w + (size_t)rank * M;
@@ -637,7 +689,7 @@ struct Ssfm {
             bool stop = false;
             const C *last_row = rk + (size_t)(a.n_z - 1) * NCO;
             for (int rt = rt_begin; rt < rt_begin + rt_count && !stop; rt++) {
-                double th[3] = {0.0, 0.0, 0.0};
+                double th[3] = {tab.g_last, 0.0, 0.0};
                 {
                     Ops op{};
                     op.inject = !a.pass_only;
@@ -646,9 +698,10 @@ struct Ssfm {
                         const int nrt = I.n_rt_total;
                         op.poff = (rt == 0) ? 0 : ((rt > 0 && rt < nrt - 1) ? (long)rt * N : (long)N * nrt - 1 - N);
                     }
-                    op.rk0 = rk;
+                    op.turn = rk + (size_t)a.n_z * NCO;
+                    op.rk1 = rk;
                     frame_step(op, tab, frame_index(rt, 0), th);
-                    cross(home, gf, 0u, ALL, op, I, tab, h6, a.eom_idler, acc, t, rank);
+                    cross(home, gf, 0u, ALL, op, I, tab, rkc, a.eom_idler, acc, t, rank);
                     xsync();
                 }
                 for (int s = 0; s < a.n_z; s++) {
@@ -660,9 +713,10 @@ struct Ssfm {
                     if (s + 1 < a.n_z) {
                         Ops op{};
                         op.rk0 = rk + (size_t)s * NCO;
+                        op.turn = op.rk0;
                         op.rk1 = rk + (size_t)(s + 1) * NCO;
                         frame_step(op, tab, frame_index(rt, s + 1), th);
-                        cross(home, gf, ALL, ALL, op, I, tab, h6, a.eom_idler, acc, t, rank);
+                        cross(home, gf, ALL, ALL, op, I, tab, rkc, a.eom_idler, acc, t, rank);
                         xsync();
                     }
                 }
@@ -671,7 +725,7 @@ struct Ssfm {
                     Ops op{};
                     op.rk0 = last_row;
                     frame_back(op, th);
-                    cross(home, gf, ALL, 0u, op, I, tab, h6, a.eom_idler, acc, t, rank);
+                    cross(home, gf, ALL, 0u, op, I, tab, rkc, a.eom_idler, acc, t, rank);
                     xsync();
                     break;
                 }
@@ -691,19 +745,19 @@ struct Ssfm {
                     op.rk0 = last_row;
                     op.eom = use_eom;
                     const unsigned res = ALL & ~1u;
-                    cross(home, gf, ALL, res, op, I, tab, h6, a.eom_idler, acc, t, rank);
+                    cross(home, gf, ALL, res, op, I, tab, rkc, a.eom_idler, acc, t, rank);
                     xsync();
                     spectral<1>(fld(1), scratch, nullptr, wtab, I.gdd, I.tod_s, I.use_tod_s, tab.inv_n, tw, t);
                     if constexpr (F == 3)
                         spectral<1>(fld(2), scratch, nullptr, wtab, I.gdd, I.tod_i, I.use_tod_i, tab.inv_n, tw, t);
                     xsync();
                     frame_back(end, th);
-                    cross(home, gf, res, 0u, end, I, tab, h6, a.eom_idler, acc, t, rank);
+                    cross(home, gf, res, 0u, end, I, tab, rkc, a.eom_idler, acc, t, rank);
                 } else {
                     end.rk0 = last_row;
                     end.eom = use_eom;
                     frame_back(end, th);
-                    cross(home, gf, ALL, 0u, end, I, tab, h6, a.eom_idler, acc, t, rank);
+                    cross(home, gf, ALL, 0u, end, I, tab, rkc, a.eom_idler, acc, t, rank);
                 }
                 /* signal power over the cluster, summed in rank order by every CTA */
                 double part = block_sum(acc, red, t);
