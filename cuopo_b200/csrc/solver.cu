@@ -25,14 +25,12 @@ struct cuopo_plan {
     int phase32;      /* CUOPO_F32_PHASE32 plans: phase factors in FP32 */
     int F;            /* number of fields */
     int N;            /* grid points */
-    int threads;      /* CTA size */
-    int cluster;      /* CTAs per instance */
-    size_t smem;      /* dynamic shared memory per CTA */
-    void *d_disp;     /* [F][CL][M], entry [f][k2][k1] = D_f(k2 + CL k1) */
+    const KernelEntry *k;    /* the kernel its tables are laid out for */
+    void *d_disp;     /* [F][N], D_f(q) at [f][freq_slot(k, q)] */
     void *d_rk;       /* [(n_z+1)][4] */
     void *d_eom;      /* [N] or NULL */
-    float *d_w;       /* [CL][M], same permutation */
-    void *d_twN;      /* [N] W_N^q (cluster plans) or NULL */
+    float *d_w;       /* [N], same permutation */
+    void *d_twN;      /* [CL - 1][M] cross-stage twiddles (CL > 1) or NULL */
     double2 *d_frame_u; /* [NFRAME] random frame angles */
     void *d_frame_c;    /* [NFRAME][3] their phasors */
     int *d_status;
@@ -106,6 +104,30 @@ static const KernelEntry *find_kernel(int precision, int F, int N, bool single_c
         return found != nullptr;
     });
     return found;
+}
+
+/* The few-instance kernel with the same arithmetic as k, or NULL. */
+static const KernelEntry *find_wide(const KernelEntry *k)
+{
+    static const KernelList *const lists[] = {&wide_f32_2eq, &wide_f32_3eq, &wide_f64_2eq, &wide_f64_3eq};
+    if (k->home != 2)
+        for (const KernelList *l : lists)
+            for (int i = 0; i < l->n; i++) {
+                const KernelEntry &w = l->k[i];
+                if (w.precision == k->precision && w.F == k->F && w.M == k->M && w.CL == k->CL) return &w;
+            }
+    return nullptr;
+}
+
+/* Place of frequency q = k2 + CL k1 in the kernel's tables: per CTA in the
+ * order of k1, or (wide_kernel) per 256-point transform (k2, r) with its 16
+ * lanes side by side, k1 = r + R0 lane + T e. */
+static size_t freq_slot(const KernelEntry *k, int q)
+{
+    const int k2 = q % k->CL, k1 = q / k->CL;
+    if (!k->wide) return (size_t)k2 * k->M + k1;
+    const int T = k->M / 16, R0 = k->M / 256, e = k1 / T, r = k1 % T % R0, lane = k1 % T / R0;
+    return ((size_t)(k2 * R0 + r) * 16 + e) * 16 + lane;
 }
 
 /* ------------------------------------------------------------ host tables */
@@ -190,7 +212,8 @@ static void build_rk_rows(const cuopo_params &p, cpx<R> *co, bool p32, double &h
 }
 
 template <typename R>
-static std::vector<unsigned char> build_tables(const cuopo_params &p, const float *w, const float *T, int CL,
+static std::vector<unsigned char> build_tables(const cuopo_params &p, const float *w, const float *T,
+                                               const KernelEntry *kern,
                                                std::vector<unsigned char> &rk_out,
                                                std::vector<unsigned char> &eom_out,
                                                std::vector<unsigned char> &twn_out, double &h6, double &g_last,
@@ -217,37 +240,37 @@ static std::vector<unsigned char> build_tables(const cuopo_params &p, const floa
     std::vector<unsigned char> disp(sizeof(C) * (size_t)F * N);
     C *D = reinterpret_cast<C *>(disp.data());
     const double z = p.dz;
-    const int M = N / CL;
+    const int CL = kern->CL;
     for (int f = 0; f < F; f++) {
         const double att = std::exp(-0.5 * al[f] * z) / (double)N;
         for (int k = 0; k < N; k++) {
             const double wk = (double)w[k];
             const double ph = z * wk * (gvm[f] + 0.5 * wk * b2[f] + wk * wk * b3[f] / 6.0);
-            /* frequency k = k2 + CL k1 is entry k1 of CTA k2's row.  Stored as
-             * d = N D - 1 and applied as (A + A d) / N: the factor's float
+            /* stored as d = N D - 1 and applied as (A + A d) / N: the factor's float
              * rounding error then scales with |d| (tiny near w = 0, where CW
              * fields live) instead of biasing every slice by up to half an
              * ulp of att, which would compound over thousands of round trips. */
-            const int k2 = k % CL, k1 = k / CL;
             const double a = att * (double)N;
             double sn, cs;
             phase_sc(ph, p32, sn, cs);
             const double dre = (ph == 0.0) ? a - 1.0 : a * cs - 1.0;
-            D[(size_t)f * N + (size_t)k2 * M + k1] = mk<C>((R)dre, (R)(a * sn));
+            D[(size_t)f * N + freq_slot(kern, k)] = mk<C>((R)dre, (R)(a * sn));
         }
     }
-    /* cross-stage twiddles W_N^q = exp(2 pi i q / N) as a quarter turn
-     * m = round(4q/N) (recomputed in the kernel) and the residual rotation
-     * phi = 2 pi q/N - m pi/2, |phi| <= pi/4, stored as (tan(phi/2), sin(phi)) */
+    /* cross-stage twiddles exp(2 pi i q / N), q = n1 c, at [c - 1][n1], as a
+     * quarter turn m = round(4q/N) (recomputed in the kernel) and the residual
+     * rotation phi = 2 pi q/N - m pi/2, |phi| <= pi/4, stored as (tan(phi/2), sin(phi)) */
     twn_out.clear();
     if (CL > 1) {
-        twn_out.resize(sizeof(C) * (size_t)N);
+        const int M = kern->M;
+        twn_out.resize(sizeof(C) * (size_t)(CL - 1) * M);
         C *W = reinterpret_cast<C *>(twn_out.data());
-        for (long q = 0; q < N; q++) {
-            const long m = (4 * q + N / 2) / N;
-            const double phi = 2.0 * M_PI * (double)(4 * q - m * N) / (4.0 * (double)N);
-            W[q] = mk<C>((R)std::tan(0.5 * phi), (R)std::sin(phi));
-        }
+        for (int c = 1; c < CL; c++)
+            for (long n1 = 0; n1 < M; n1++) {
+                const long q = n1 * c, m = (4 * q + N / 2) / N;
+                const double phi = 2.0 * M_PI * (double)(4 * q - m * N) / (4.0 * (double)N);
+                W[(size_t)(c - 1) * M + n1] = mk<C>((R)std::tan(0.5 * phi), (R)std::sin(phi));
+            }
     }
     rk_out.assign(sizeof(C) * (size_t)(p.n_z + 1) * 4, 0);
     build_rk_rows<R>(p, reinterpret_cast<C *>(rk_out.data()), p32, h6, g_last);
@@ -266,10 +289,9 @@ static std::vector<unsigned char> build_tables(const cuopo_params &p, const floa
     return disp;
 }
 
-extern "C" cuopo_status cuopo_plan_create(cuopo_plan **out, const cuopo_params *p,
-                                          const float *w_host, const float *T_host, int precision)
+static cuopo_status plan_create(cuopo_plan **out, const cuopo_params *p, const float *w_host, const float *T_host,
+                                int precision, const KernelEntry *k)
 {
-    cuopo::Range range_("cuopo_plan_create");
     if (!out || !p) return cuopo_fail(CUOPO_EINVAL, "plan_create: NULL argument");
     *out = nullptr;
     if (p->n_eqs != 2 && p->n_eqs != 3) return cuopo_fail(CUOPO_EINVAL, "n_eqs must be 2 or 3");
@@ -279,7 +301,12 @@ extern "C" cuopo_status cuopo_plan_create(cuopo_plan **out, const cuopo_params *
         return cuopo_fail(CUOPO_EINVAL, "precision must be CUOPO_F32, CUOPO_F64 or CUOPO_F32_PHASE32");
     const bool phase32 = precision == CUOPO_F32_PHASE32;
     if (phase32) precision = CUOPO_F32;
-    const KernelEntry *k = find_kernel(precision, p->n_eqs, p->n_t);
+    if (!k) {
+        /* a plan runs one instance at a time: its few-instance kernel, where there is one */
+        k = find_kernel(precision, p->n_eqs, p->n_t);
+        const KernelEntry *wide = k ? find_wide(k) : nullptr;
+        if (wide) k = wide;
+    }
     if (!k) return cuopo_fail(CUOPO_EUNSUPPORTED, "no kernel built for this (precision, n_eqs, n_t)");
 
     std::vector<float> w((size_t)p->n_t), T((size_t)p->n_t);
@@ -294,13 +321,12 @@ extern "C" cuopo_status cuopo_plan_create(cuopo_plan **out, const cuopo_params *
 
     std::vector<unsigned char> disp, rk, eom, twn;
     double h6 = 0, g_last = 0;
-    const int CL = k->CL;
     if (precision == CUOPO_F32)
-        disp = build_tables<float>(*p, w.data(), T.data(), CL, rk, eom, twn, h6, g_last, phase32);
-    else disp = build_tables<double>(*p, w.data(), T.data(), CL, rk, eom, twn, h6, g_last);
-    /* frequency grid in the same per-CTA order as the dispersion table */
+        disp = build_tables<float>(*p, w.data(), T.data(), k, rk, eom, twn, h6, g_last, phase32);
+    else disp = build_tables<double>(*p, w.data(), T.data(), k, rk, eom, twn, h6, g_last);
+    /* frequency grid in the same order as the dispersion table */
     std::vector<float> wp((size_t)p->n_t);
-    for (int q = 0; q < p->n_t; q++) wp[(size_t)(q % CL) * (p->n_t / CL) + q / CL] = w[q];
+    for (int q = 0; q < p->n_t; q++) wp[freq_slot(k, q)] = w[q];
 
     cuopo_plan *pl = new (std::nothrow) cuopo_plan();
     if (!pl) return cuopo_fail(CUOPO_ENOMEM, "plan_create: out of host memory");
@@ -309,9 +335,7 @@ extern "C" cuopo_status cuopo_plan_create(cuopo_plan **out, const cuopo_params *
     pl->phase32 = phase32;
     pl->F = p->n_eqs;
     pl->N = p->n_t;
-    pl->threads = k->M / 16;
-    pl->cluster = k->CL;
-    pl->smem = k->smem;
+    pl->k = k;
     pl->h6 = h6;
     pl->g_last = g_last;
     cudaError_t e;
@@ -373,6 +397,13 @@ extern "C" cuopo_status cuopo_plan_create(cuopo_plan **out, const cuopo_params *
     return CUOPO_OK;
 }
 
+extern "C" cuopo_status cuopo_plan_create(cuopo_plan **out, const cuopo_params *p,
+                                          const float *w_host, const float *T_host, int precision)
+{
+    cuopo::Range range_("cuopo_plan_create");
+    return plan_create(out, p, w_host, T_host, precision, nullptr);
+}
+
 extern "C" cuopo_status cuopo_plan_destroy(cuopo_plan *pl)
 {
     if (!pl) return CUOPO_OK;
@@ -391,9 +422,9 @@ extern "C" cuopo_status cuopo_plan_destroy(cuopo_plan *pl)
 extern "C" cuopo_status cuopo_plan_config(const cuopo_plan *pl, int *cluster, int *threads, int *smem)
 {
     if (!pl) return cuopo_fail(CUOPO_EINVAL, "plan_config: NULL plan");
-    if (cluster) *cluster = pl->cluster;
-    if (threads) *threads = pl->threads;
-    if (smem) *smem = (int)pl->smem;
+    if (cluster) *cluster = pl->k->ctas;
+    if (threads) *threads = pl->k->threads;
+    if (smem) *smem = (int)pl->k->smem;
     return CUOPO_OK;
 }
 
@@ -438,11 +469,9 @@ static void cavity_factors(const cuopo_params &p, Instance &I, bool p32 = false)
     I.use_tod_i = (p.tod_i != 0 && p.b3i != 0);
 }
 
-static cuopo_status launch(cuopo_plan *pl, const LaunchArgs &a, int grid, void *stream)
+static cuopo_status launch(const KernelEntry *k, const LaunchArgs &a, int clusters, void *stream)
 {
-    const KernelEntry *k = find_kernel(pl->precision, pl->F, pl->N);
-    if (!k) return cuopo_fail(CUOPO_EUNSUPPORTED, "no kernel for plan");
-    cudaError_t e = k->fn(a, grid, (cudaStream_t)stream);
+    cudaError_t e = k->fn(a, clusters, (cudaStream_t)stream);
     if (e != cudaSuccess) return cuda_fail(e, "kernel launch");
     return CUOPO_OK;
 }
@@ -460,7 +489,7 @@ extern "C" cuopo_status cuopo_crystal_pass(cuopo_plan *pl, void *Ap, void *As, v
     a.single.rt_count = 1;
     a.single.save_first = 0;
     a.single.save_count = 0;
-    return launch(pl, a, 1, stream);
+    return launch(pl->k, a, 1, stream);
 }
 
 extern "C" cuopo_status cuopo_round_trips(cuopo_plan *pl, void *Ap, void *As, void *Ai, const void *pump,
@@ -494,7 +523,7 @@ extern "C" cuopo_status cuopo_round_trips(cuopo_plan *pl, void *Ap, void *As, vo
     I.tol = tol;
     I.rt_done = rt_done_dev;
     cavity_factors(pl->p, I, pl->phase32);
-    return launch(pl, a, 1, stream);
+    return launch(pl->k, a, 1, stream);
 }
 
 extern "C" cuopo_status cuopo_plan_status(cuopo_plan *pl, int *status, int reset)
@@ -527,8 +556,17 @@ struct BatchGroup {
     int *d_queue;
     cudaStream_t stream;
     cudaEvent_t done;
+    const KernelEntry *kernel;
     int grid;
 };
+
+/* The kernel of a batch group of `count` instances. */
+static const KernelEntry *pick_batch_kernel(int precision, int F, int n_t, int count)
+{
+    const KernelEntry *k = find_kernel(precision, F, n_t), *wide = find_wide(k);
+    if (!wide || g_force) return k;
+    return count <= wide->occ() ? wide : k;
+}
 
 struct cuopo_batch {
     int count;
@@ -716,6 +754,11 @@ static cuopo_status batch_build(cuopo_batch **out, const std::vector<cuopo_param
         g.n_z = key[2];
         g.eom_idler = key[3];
         g.regime = key[4];
+        int members = 0;
+        for (const cuopo_params &p : prm)
+            members += p.n_eqs == g.F && p.n_t == g.n_t && p.n_z == g.n_z && p.eom_idler == g.eom_idler &&
+                       p.regime == g.regime;
+        g.kernel = pick_batch_kernel(precision, g.F, g.n_t, members);
         std::vector<std::vector<double>> pkeys;
         std::vector<int> plan_of;
         for (int i = 0; i < count; i++) {
@@ -728,7 +771,7 @@ static cuopo_status batch_build(cuopo_batch **out, const std::vector<cuopo_param
             size_t q = std::find(pkeys.begin(), pkeys.end(), pk) - pkeys.begin();
             if (q == pkeys.size()) {
                 cuopo_plan *pl = nullptr;
-                cuopo_status st = cuopo_plan_create(&pl, &p, nullptr, nullptr, precision);
+                cuopo_status st = plan_create(&pl, &p, nullptr, nullptr, precision, g.kernel);
                 if (st != CUOPO_OK) {
                     cuopo_batch_destroy(b);
                     return st;
@@ -738,9 +781,8 @@ static cuopo_status batch_build(cuopo_batch **out, const std::vector<cuopo_param
             }
             plan_of.push_back((int)q);
         }
-        const KernelEntry *k = find_kernel(precision, g.F, g.n_t);
         /* persistent grid: as many clusters as can be resident at once */
-        const int occ = k->occ();
+        const int occ = g.kernel->occ();
         if (occ < 1) {
             cuopo_batch_destroy(b);
             return cuopo_fail(CUOPO_ECUDA, "batch_create: kernel does not fit on the device");
@@ -946,7 +988,7 @@ extern "C" cuopo_status cuopo_batch_step(cuopo_batch *b, int chunk, int max_rt, 
         a.max_rt = max_rt;
         a.tol = tol;
         a.patience = patience;
-        cuopo_status s2 = launch(g.plans[0], a, g.grid, g.stream);
+        cuopo_status s2 = launch(g.kernel, a, g.grid, g.stream);
         if (s2 != CUOPO_OK) return s2;
         if ((e = cudaEventRecord(g.done, g.stream)) != cudaSuccess) return cuda_fail(e, "batch_step");
     }
@@ -1168,6 +1210,7 @@ extern "C" cuopo_status cuopo_crystal_pass_noalloc(const cuopo_params *p, const 
     if (p->n_z < 1 || p->n_z > CUOPO_NOALLOC_MAX_NZ)
         return cuopo_fail(CUOPO_EINVAL, "crystal_pass_noalloc: n_z must be in [1, 1024]");
     const KernelEntry *k = find_kernel(CUOPO_F32, p->n_eqs, p->n_t, true);
+    if (k && find_wide(k)) k = find_wide(k);
     if (!k) return cuopo_fail(CUOPO_EUNSUPPORTED, "crystal_pass_noalloc: no single-CTA kernel for n_t");
     const int N = p->n_t, F = p->n_eqs;
 
@@ -1227,7 +1270,7 @@ extern "C" cuopo_status cuopo_crystal_pass_noalloc(const cuopo_params *p, const 
             const double wk = (double)w[q];
             const double ph = p->dz * wk * (gvm[f] + 0.5 * wk * b2[f] + wk * wk * b3[f] / 6.0);
             const double dre = (ph == 0.0) ? a - 1.0 : a * std::cos(ph) - 1.0;
-            Dt[(size_t)f * N + q] = make_float2((float)dre, (float)(a * std::sin(ph)));
+            Dt[(size_t)f * N + freq_slot(k, q)] = make_float2((float)dre, (float)(a * std::sin(ph)));
         }
     }
     double h6, g_last;

@@ -49,7 +49,8 @@ struct Tables {
     const void *rk;     /* [n_z + 1][4]: RK4 half steps, see RkRow */
     const void *eom;    /* [N]: exp(i m sin(2 pi fpm T)) or NULL */
     const float *w;     /* [CL][M]: angular frequency grid (reference float values) */
-    const void *twN;    /* [N]: W_N^q (cross-stage twiddles; CL > 1) */
+    const void *twN;    /* [CL - 1][M]: W_N^{n1 c} at [c - 1][n1] (cross-stage twiddles; CL > 1): the lanes of a
+                         * warp (consecutive n1) read one run per c (indexed by n1 c they read up to 14 lines) */
     const double2 *frame_u; /* [NFRAME]: random frame angles (u_s, u_i) in turns, |u| < 1/8 */
     const void *frame_c;    /* [NFRAME][3]: rotation (tan, sin) for pump, signal, idler */
     double h6;          /* (dz/2)/6 */
@@ -109,7 +110,7 @@ struct LaunchArgs {
     double tol;
 };
 
-enum { ST_OK = 0, ST_CONVERGED = 1, ST_LIMIT = 2, ST_NONFINITE = 5 };
+enum { ST_OK = 0, ST_CONVERGED = 1, ST_LIMIT = 2, ST_TIMEOUT = 4, ST_NONFINITE = 5 };
 
 /* Random frame rotations.  The coupled-wave equations are invariant under
  * (Ap, As, Ai) -> (Ap e^{i(a+b)}, As e^{ia}, Ai e^{ib}) (and Ap e^{2ia} in the
@@ -229,6 +230,7 @@ struct Ssfm {
         long poff;          /* NS pump window offset of this round trip */
         const C *rk0, *rk1; /* rows of the RK4 half steps to apply (NULL: none) */
         const C *turn;      /* row whose turn of the pump comes between the two (NULL: none) */
+        int frame;          /* entry of the frame table to move to (-1: none) */
         int eom;            /* intracavity phase modulator */
         int rotate;         /* frame rotation: 1 the shear rotations rf[f], 2 quarter turns rq[f] first */
         C rf[3];
@@ -240,13 +242,11 @@ struct Ssfm {
         int power;          /* accumulate |As|^2 */
     };
 
-    /* Move to the frame of table entry q (rotation by 2 pi u per field, built
-     * from shears); th accumulates each field's frame angle in turns
+    /* Move to the frame of a table entry (rotation by 2 pi u per field, built
+     * from the shears fc); th accumulates each field's frame angle in turns
      * (the pump's starts at the RK4 frame of the last slice). */
-    static __device__ __forceinline__ void frame_step(Ops &op, const Tables &tab, int q, double (&th)[3])
+    static __device__ __forceinline__ void frame_step(Ops &op, const C *fc, double2 u, double (&th)[3])
     {
-        const C *fc = reinterpret_cast<const C *>(tab.frame_c) + 3 * q;
-        const double2 u = tab.frame_u[q];
         op.rotate = 1;
 #pragma unroll
         for (int f = 0; f < 3; f++) op.rf[f] = fc[f];
@@ -397,6 +397,31 @@ struct Ssfm {
         if (op.power) acc += cabs2d(A[1]);
     }
 
+    /* The radix-CL stages of one field at position n1: the inverse one (y ->
+     * time) and the forward one, with the cross-stage twiddles W_N^{n1 c}:
+     * quarter turn and residual rotation (tan, sin) from the table. */
+    static __device__ __forceinline__ void cross_inv(C (&v)[CL], int n1, const C *__restrict__ twN)
+    {
+#pragma unroll
+        for (int c = 1; c < CL; c++) {
+            const int q = n1 * c;
+            const C w = __ldg(twN + (c - 1) * M + n1);
+            v[c] = shear_rot(iq_rt(v[c], (-((4 * q + N / 2) / N)) & 3), -w.x, -w.y);
+        }
+        dft<-1, CL>(v);
+    }
+
+    static __device__ __forceinline__ void cross_fwd(C (&v)[CL], int n1, const C *__restrict__ twN)
+    {
+        dft<+1, CL>(v);
+#pragma unroll
+        for (int c = 1; c < CL; c++) {
+            const int q = n1 * c;
+            const C w = __ldg(twN + (c - 1) * M + n1);
+            v[c] = shear_rot(iq_rt(v[c], ((4 * q + N / 2) / N) & 3), w.x, w.y);
+        }
+    }
+
     /* The radix-CL stage of one field at the owned position n1 (S = -1: the
      * inverse cross stage, y -> time; S = +1: the forward one), on global
      * memory. */
@@ -406,23 +431,8 @@ struct Ssfm {
         C v[CL];
 #pragma unroll
         for (int c = 0; c < CL; c++) v[c] = __ldcg(g + (size_t)c * M + n1);
-        if constexpr (S < 0) {
-#pragma unroll
-            for (int c = 1; c < CL; c++) {
-                const long q = (long)n1 * c;
-                const C w = __ldg(twN + q);
-                v[c] = shear_rot(iq_rt(v[c], (-(int)(((4 * q + N / 2) / N) & 3)) & 3), -w.x, -w.y);
-            }
-            dft<-1, CL>(v);
-        } else {
-            dft<+1, CL>(v);
-#pragma unroll
-            for (int c = 1; c < CL; c++) {
-                const long q = (long)n1 * c;
-                const C w = __ldg(twN + q);
-                v[c] = shear_rot(iq_rt(v[c], (int)(((4 * q + N / 2) / N) & 3)), w.x, w.y);
-            }
-        }
+        if constexpr (S < 0) cross_inv(v, n1, twN);
+        else cross_fwd(v, n1, twN);
 #pragma unroll
         for (int c = 0; c < CL; c++) __stcg(g + (size_t)c * M + n1, v[c]);
     }
@@ -495,16 +505,7 @@ struct Ssfm {
             if constexpr (CL > 1) {
 #pragma unroll
                 for (int f = 0; f < F; f++) {
-                    if ((in_y >> f) & 1u) {
-#pragma unroll
-                        for (int c = 1; c < CL; c++) {
-                            const long q = (long)n1 * c;
-                            const C w = __ldg(twN + q);
-                            const int qm = (int)(((4 * q + N / 2) / N) & 3);
-                            v[f][c] = shear_rot(iq_rt(v[f][c], (-qm) & 3), -w.x, -w.y);
-                        }
-                        dft<-1, CL>(v[f]);
-                    }
+                    if ((in_y >> f) & 1u) cross_inv(v[f], n1, twN);
                 }
             }
 #pragma unroll
@@ -519,16 +520,7 @@ struct Ssfm {
             if constexpr (CL > 1) {
 #pragma unroll
                 for (int f = 0; f < F; f++) {
-                    if ((out_y >> f) & 1u) {
-                        dft<+1, CL>(v[f]);
-#pragma unroll
-                        for (int c = 1; c < CL; c++) {
-                            const long q = (long)n1 * c;
-                            const C w = __ldg(twN + q);
-                            const int qm = (int)(((4 * q + N / 2) / N) & 3);
-                            v[f][c] = shear_rot(iq_rt(v[f][c], qm), w.x, w.y);
-                        }
-                    }
+                    if ((out_y >> f) & 1u) cross_fwd(v[f], n1, twN);
                 }
             }
 #pragma unroll
@@ -537,6 +529,23 @@ struct Ssfm {
 #pragma unroll
                 for (int f = 0; f < F; f++) dst[f * M + sm] = v[f][c];
             }
+        }
+    }
+
+    /* reg[e] times the GDD/TOD factor of frequency w[e stride] and 1/N
+     * (functions.cuh:156-186, formed in FP64). */
+    static __device__ __forceinline__ void gdd_factor(C (&reg)[16], const float *__restrict__ w, int stride, double gdd,
+                                                      double tod, int use_tod, R s_n)
+    {
+#pragma unroll 4
+        for (int e = 0; e < 16; e++) {
+            const double wk = (double)__ldg(w + e * stride);
+            const double ph = use_tod ? 0.5 * wk * rfma(wk, gdd, rmul(wk * wk, tod) / 3.0) : 0.5 * wk * wk * gdd;
+            double sn, cs;
+            sincos(ph, &sn, &cs);
+            /* cos(ph) - 1 = -2 sin^2(ph/2), exact for small ph */
+            const double sh = sin(0.5 * ph);
+            reg[e] = caddmul(cscale(reg[e], s_n), mk<C>((R)(-2.0 * sh * sh), (R)sn));
         }
     }
 
@@ -566,17 +575,7 @@ struct Ssfm {
                 reg[e] = caddmul(cscale(reg[e], s_n), __ldg(row + t + e * T));
             }
         } else {
-#pragma unroll 4
-            for (int e = 0; e < 16; e++) {
-                /* functions.cuh:156-186, formed in FP64 */
-                const double wk = (double)__ldg(w + t + e * T);
-                const double ph = use_tod ? 0.5 * wk * rfma(wk, gdd, rmul(wk * wk, tod) / 3.0) : 0.5 * wk * wk * gdd;
-                double sn, cs;
-                sincos(ph, &sn, &cs);
-                /* cos(ph) - 1 = -2 sin^2(ph/2), exact for small ph */
-                const double sh = sin(0.5 * ph);
-                reg[e] = caddmul(cscale(reg[e], s_n), mk<C>((R)(-2.0 * sh * sh), (R)sn));
-            }
+            gdd_factor(reg, w + t, T, gdd, tod, use_tod, s_n);
         }
         local_transform<-1, M, P - 1, INPLACE>(reg, bufA, bufB, tw, t);
         if constexpr (GH) {
@@ -587,94 +586,44 @@ struct Ssfm {
         }
     }
 
-    static __device__ __forceinline__ double block_sum(double v, double *red, int t)
-    {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if ((t & 31) == 0) red[t >> 5] = v;
-        __syncthreads();
-        double s = 0.0;
-#pragma unroll
-        for (int q = 0; q < T / 32; q++) s += red[q];
-        __syncthreads();
-        return s;
-    }
-
-    static __device__ __forceinline__ void run(const LaunchArgs &a)
-    {
-        extern __shared__ __align__(16) unsigned char smem_raw[];
-        C *const sm = reinterpret_cast<C *>(smem_raw);
-        C *home = GH ? nullptr : sm;
-        C *scratch = GH ? sm : (INPLACE ? home : home + (size_t)F * M);
-        __shared__ double red[32];
-        __shared__ double red_cl;
-        __shared__ int next_inst;
-        const int t = threadIdx.x;
-        int rank = 0;
-        if constexpr (CL > 1) rank = (int)cg::this_cluster().block_rank();
-
-        C *twtab = sm + field_elems();
-        fill_twiddle_table<M>(twtab, t);
+    /* The kernel's state of one thread: where its fields live and its twiddles
+     * (the interface drive() runs the round trips through). */
+    struct Engine {
+        using Math = Ssfm;
+        C *home, *scratch;
+        C *gf[3];
         StageTwiddles<M, C> tw;
-        tw.init(t, twtab);
-        __syncthreads();
+        int t, rank;
 
-        bool first = true;
-        for (;;) {
-            int idx;
-            if (a.inst) {
-                if (rank == 0 && t == 0) next_inst = atomicAdd(a.queue, 1);
-                bar();
-                idx = *peer(&next_inst, 0);
-                bar();
-                if (idx >= a.n_inst) break;
-            } else {
-                if (!first) break;
-                idx = 0;
-            }
-            first = false;
-            const Instance &I = a.inst ? a.inst[idx] : a.single;
-            /* this instance's tables: its own where it has them, else the launch's */
-            Tables tab = a.tab;
-            int use_eom = a.use_eom;
-            if (I.disp) {
-                tab.disp = I.disp;
-                tab.rk = I.rk;
-                tab.w = I.w;
-                tab.h6 = I.h6;
-                tab.kp = I.kp;
-                tab.ks = I.ks;
-                tab.g_last = I.g_last;
-                tab.eom = I.eom;
-                use_eom = I.eom != nullptr;
-            }
-            RkConst<R> rkc;
-            rkc.hp = (R)(0.5 * tab.kp);
-            rkc.hs = (R)(0.5 * tab.ks);
-            rkc.fp = (R)tab.kp;
-            rkc.fs = (R)tab.ks;
-            rkc.gp = (R)(tab.h6 * tab.kp);
-            rkc.gs = (R)(tab.h6 * tab.ks);
-            const C *__restrict__ rk = reinterpret_cast<const C *>(tab.rk);
-            const C *__restrict__ disp = reinterpret_cast<const C *>(tab.disp);
-            const float *__restrict__ wtab = tab.w + (size_t)rank * M;
-            int rt_begin = I.rt_begin, rt_count = I.rt_count, patience = I.patience, calm = 0;
-            double tol = I.tol, prev_ps = -1.0;
-            if (I.st_flag) {
-                /* batch instance: resume from its saved state, skip if done */
-                if (*(volatile int *)I.st_flag != 0) continue;
-                rt_begin = *(volatile int *)I.st_rt;
-                rt_count = min(a.chunk, rt_limit(a, I) - rt_begin);
-                prev_ps = rt_begin > 0 ? *(volatile double *)I.st_ps : -1.0;
-                calm = *(volatile int *)I.st_calm;
-                tol = a.tol;
-                patience = a.patience;
-            }
+        __device__ __forceinline__ void init()
+        {
+            extern __shared__ __align__(16) unsigned char smem_raw[];
+            C *const sm = reinterpret_cast<C *>(smem_raw);
+            home = GH ? nullptr : sm;
+            scratch = GH ? sm : (INPLACE ? home : home + (size_t)F * M);
+            t = threadIdx.x;
+            rank = 0;
+            if constexpr (CL > 1) rank = (int)cg::this_cluster().block_rank();
+            C *twtab = sm + field_elems();
+            fill_twiddle_table<M>(twtab, t);
+            tw.init(t, twtab);
+            __syncthreads();
+        }
 
-            C *const gf[3] = {reinterpret_cast<C *>(I.Ap), reinterpret_cast<C *>(I.As),
-                              reinterpret_cast<C *>(I.Ai)};
-            /* the field f of this CTA for the local transforms */
-            auto fld = [&](int f) -> C * { return GH ? gf[f] + (size_t)rank * M : home + (size_t)f * M; };
+        /* every thread of the instance's CTAs */
+        __device__ __forceinline__ void barrier() { bar(); }
+
+        template <typename X>
+        static __device__ __forceinline__ X *cta(X *p, int r)
+        {
+            return peer(p, r);
+        }
+
+        __device__ __forceinline__ void load(const Instance &I)
+        {
+            gf[0] = reinterpret_cast<C *>(I.Ap);
+            gf[1] = reinterpret_cast<C *>(I.As);
+            gf[2] = reinterpret_cast<C *>(I.Ai);
             if constexpr (!GH) {
 #pragma unroll
                 for (int f = 0; f < F; f++)
@@ -683,111 +632,10 @@ struct Ssfm {
                         home[f * M + swz<C>(t + e * T)] = gf[f][(size_t)rank * M + t + e * T];
             }
             xsync();
+        }
 
-            double ps = prev_ps, acc = 0.0;
-            int rts = 0, flag = 0;
-            bool stop = false;
-            const C *last_row = rk + (size_t)(a.n_z - 1) * NCO;
-            for (int rt = rt_begin; rt < rt_begin + rt_count && !stop; rt++) {
-                double th[3] = {tab.g_last, 0.0, 0.0};
-                {
-                    Ops op{};
-                    op.inject = !a.pass_only;
-                    if (a.regime == 1) {
-                        /* ReadPump offsets, functions.cuh:196-210 (Q6) */
-                        const int nrt = I.n_rt_total;
-                        op.poff = (rt == 0) ? 0 : ((rt > 0 && rt < nrt - 1) ? (long)rt * N : (long)N * nrt - 1 - N);
-                    }
-                    op.turn = rk + (size_t)a.n_z * NCO;
-                    op.rk1 = rk;
-                    frame_step(op, tab, frame_index(rt, 0), th);
-                    cross(home, gf, 0u, ALL, op, I, tab, rkc, a.eom_idler, acc, t, rank);
-                    xsync();
-                }
-                for (int s = 0; s < a.n_z; s++) {
-#pragma unroll 1
-                    for (int f = 0; f < F; f++)
-                        spectral<0>(fld(f), scratch, disp + ((size_t)f * CL + rank) * M, nullptr, 0.0, 0.0, 0,
-                                    tab.inv_n, tw, t);
-                    xsync();
-                    if (s + 1 < a.n_z) {
-                        Ops op{};
-                        op.rk0 = rk + (size_t)s * NCO;
-                        op.turn = op.rk0;
-                        op.rk1 = rk + (size_t)(s + 1) * NCO;
-                        frame_step(op, tab, frame_index(rt, s + 1), th);
-                        cross(home, gf, ALL, ALL, op, I, tab, rkc, a.eom_idler, acc, t, rank);
-                        xsync();
-                    }
-                }
-                rts++;
-                if (a.pass_only) {
-                    Ops op{};
-                    op.rk0 = last_row;
-                    frame_back(op, th);
-                    cross(home, gf, ALL, 0u, op, I, tab, rkc, a.eom_idler, acc, t, rank);
-                    xsync();
-                    break;
-                }
-                const bool save = (rt >= I.save_first && rt < I.save_first + I.save_count);
-                Ops end{};
-                end.addphase = 1;
-                end.ph_s = make_double2(I.phase_s[0], I.phase_s[1]);
-                end.ph_i = make_double2(I.phase_i[0], I.phase_i[1]);
-                end.save = save;
-                end.slot = save ? (size_t)(rt - I.save_first) * N : 0;
-                end.power = 1;
-                acc = 0.0;
-                if (I.gdd != 0.0) {
-                    /* GDD / TOD compensation of the resonant fields (cuOPO.cu:521-553):
-                     * signal and idler go to the frequency domain, the pump stays in time */
-                    Ops op{};
-                    op.rk0 = last_row;
-                    op.eom = use_eom;
-                    const unsigned res = ALL & ~1u;
-                    cross(home, gf, ALL, res, op, I, tab, rkc, a.eom_idler, acc, t, rank);
-                    xsync();
-                    spectral<1>(fld(1), scratch, nullptr, wtab, I.gdd, I.tod_s, I.use_tod_s, tab.inv_n, tw, t);
-                    if constexpr (F == 3)
-                        spectral<1>(fld(2), scratch, nullptr, wtab, I.gdd, I.tod_i, I.use_tod_i, tab.inv_n, tw, t);
-                    xsync();
-                    frame_back(end, th);
-                    cross(home, gf, res, 0u, end, I, tab, rkc, a.eom_idler, acc, t, rank);
-                } else {
-                    end.rk0 = last_row;
-                    end.eom = use_eom;
-                    frame_back(end, th);
-                    cross(home, gf, ALL, 0u, end, I, tab, rkc, a.eom_idler, acc, t, rank);
-                }
-                /* signal power over the cluster, summed in rank order by every CTA */
-                double part = block_sum(acc, red, t);
-                if constexpr (CL > 1) {
-                    if (t == 0) red_cl = part;
-                    csync();
-                    part = 0.0;
-#pragma unroll
-                    for (int c = 0; c < CL; c++) part += *peer(&red_cl, c);
-                }
-                ps = part * tab.inv_n;
-                /* single launches record from rt_begin, batch instances by round trip */
-                if (rank == 0 && t == 0 && I.ps_hist) I.ps_hist[I.st_flag ? rt : rt - rt_begin] = ps;
-                if (!(ps == ps) || ps > 1.0e300) {
-                    if (rank == 0 && t == 0 && a.status) atomicCAS(a.status, 0, (int)ST_NONFINITE);
-                    flag = ST_NONFINITE;
-                    stop = true;
-                }
-                /* convergence: relative change of the signal power per rt below
-                 * tol for `patience` consecutive rts (from the second rt on) */
-                if (tol > 0.0 && prev_ps > 0.0 && ps > 0.0 && fabs(ps - prev_ps) < tol * ps) {
-                    if (++calm >= (patience > 0 ? patience : 1) && flag == 0) {
-                        flag = ST_CONVERGED;
-                        stop = true;
-                    }
-                } else {
-                    calm = 0;
-                }
-                prev_ps = ps;
-            }
+        __device__ __forceinline__ void store()
+        {
             if constexpr (!GH) {
 #pragma unroll
                 for (int f = 0; f < F; f++)
@@ -795,26 +643,261 @@ struct Ssfm {
                     for (int e = 0; e < 16; e++)
                         gf[f][(size_t)rank * M + t + e * T] = home[f * M + swz<C>(t + e * T)];
             }
-            if (rank == 0 && t == 0) {
-                if (I.rt_done) *I.rt_done = rts;
-                if (I.ps_out) *I.ps_out = ps;
-                if (I.flag_out) *I.flag_out = flag;
-                if (I.st_flag) {
-                    *I.st_rt = rt_begin + rts;
-                    *I.st_ps = ps;
-                    *I.st_calm = calm;
-                    *I.st_flag = flag != 0 ? flag : (rt_begin + rts >= rt_limit(a, I) ? (int)ST_LIMIT : 0);
-                }
-            }
-            bar();
         }
-    }
+
+        /* the field f of this CTA for the local transforms */
+        __device__ __forceinline__ C *fld(int f) const
+        {
+            return GH ? gf[f] + (size_t)rank * M : home + (size_t)f * M;
+        }
+
+        static constexpr bool STAGED = false;
+        __device__ __forceinline__ void stage(const Ops &, const Tables &) {}
+
+        __device__ __forceinline__ void pass(unsigned in_y, unsigned out_y, Ops &op, const Instance &I,
+                                             const Tables &tab, const RkConst<R> &rkc, int eom_idler, double (&th)[3],
+                                             double &acc)
+        {
+            if (op.frame >= 0)
+                frame_step(op, reinterpret_cast<const C *>(tab.frame_c) + 3 * op.frame, tab.frame_u[op.frame], th);
+            cross(home, gf, in_y, out_y, op, I, tab, rkc, eom_idler, acc, t, rank);
+            if (!op.power) xsync(); /* (power() synchronises) */
+        }
+
+        __device__ __forceinline__ void dispersion(const Tables &tab)
+        {
+            const C *__restrict__ disp = reinterpret_cast<const C *>(tab.disp);
+#pragma unroll 1
+            for (int f = 0; f < F; f++)
+                spectral<0>(fld(f), scratch, disp + ((size_t)f * CL + rank) * M, nullptr, 0.0, 0.0, 0, tab.inv_n, tw,
+                            t);
+            xsync();
+        }
+
+        __device__ __forceinline__ int failed() const { return 0; }
+        __device__ __forceinline__ int error() const { return 0; }
+
+        __device__ __forceinline__ void gdd(const Tables &tab, const Instance &I)
+        {
+            const float *__restrict__ w = tab.w + (size_t)rank * M;
+            spectral<1>(fld(1), scratch, nullptr, w, I.gdd, I.tod_s, I.use_tod_s, tab.inv_n, tw, t);
+            if constexpr (F == 3)
+                spectral<1>(fld(2), scratch, nullptr, w, I.gdd, I.tod_i, I.use_tod_i, tab.inv_n, tw, t);
+            xsync();
+        }
+
+        /* Sum of the threads' acc over the cluster, the same on every CTA.
+         * The order is fixed by the grid alone, not by the thread layout:
+         * each (CTA rank, t) adds its points in order (acc), then 16
+         * consecutive t by xor, then the groups of 16, then the ranks. */
+        __device__ __forceinline__ double power(double acc)
+        {
+            __shared__ double red[32];
+            __shared__ double red_cl;
+            double v = acc;
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if ((t & 15) == 0) red[t >> 4] = v;
+            __syncthreads();
+            double part = 0.0;
+#pragma unroll
+            for (int q = 0; q < T / 16; q++) part += red[q];
+            __syncthreads();
+            if constexpr (CL > 1) {
+                if (t == 0) red_cl = part;
+                csync();
+                part = 0.0;
+#pragma unroll
+                for (int c = 0; c < CL; c++) part += *peer(&red_cl, c);
+            }
+            return part;
+        }
+    };
 };
 
-template <typename R, int F, int M, int CL, int HM, int MINB>
-__global__ void __launch_bounds__(M / 16, MINB) ssfm_kernel(const LaunchArgs a)
+/*
+ * The round trips of the instances of one launch.  Engine: the kernel's thread
+ * layout (where the fields live, how a pass over them is spread over threads
+ * and CTAs); Engine::Math: the arithmetic.  Control flow is uniform over the
+ * threads of an instance.
+ */
+template <typename R, class Engine>
+static __device__ __forceinline__ void drive(const LaunchArgs &a)
 {
-    Ssfm<R, F, M, CL, HM>::run(a);
+    using K = typename Engine::Math;
+    using C = cpx<R>;
+    using Ops = typename K::Ops;
+    constexpr int N = K::N, NCO = K::NCO;
+    constexpr unsigned ALL = K::ALL;
+    __shared__ int next_inst;
+    Engine E;
+    E.init();
+    bool first = true;
+    for (;;) {
+        int idx;
+        if (a.inst) {
+            if (E.rank == 0 && threadIdx.x == 0) next_inst = atomicAdd(a.queue, 1);
+            E.barrier();
+            idx = *E.cta(&next_inst, 0);
+            E.barrier();
+            if (idx >= a.n_inst) break;
+        } else {
+            if (!first) break;
+            idx = 0;
+        }
+        first = false;
+        const bool leader = E.rank == 0 && threadIdx.x == 0;
+        const Instance &I = a.inst ? a.inst[idx] : a.single;
+        /* this instance's tables: its own where it has them, else the launch's */
+        Tables tab = a.tab;
+        int use_eom = a.use_eom;
+        if (I.disp) {
+            tab.disp = I.disp;
+            tab.rk = I.rk;
+            tab.w = I.w;
+            tab.h6 = I.h6;
+            tab.kp = I.kp;
+            tab.ks = I.ks;
+            tab.g_last = I.g_last;
+            tab.eom = I.eom;
+            use_eom = I.eom != nullptr;
+        }
+        RkConst<R> rkc;
+        rkc.hp = (R)(0.5 * tab.kp);
+        rkc.hs = (R)(0.5 * tab.ks);
+        rkc.fp = (R)tab.kp;
+        rkc.fs = (R)tab.ks;
+        rkc.gp = (R)(tab.h6 * tab.kp);
+        rkc.gs = (R)(tab.h6 * tab.ks);
+        const C *__restrict__ rk = reinterpret_cast<const C *>(tab.rk);
+        int rt_begin = I.rt_begin, rt_count = I.rt_count, patience = I.patience, calm = 0;
+        double tol = I.tol, prev_ps = -1.0;
+        if (I.st_flag) {
+            /* batch instance: resume from its saved state, skip if done */
+            if (*(volatile int *)I.st_flag != 0) continue;
+            rt_begin = *(volatile int *)I.st_rt;
+            rt_count = min(a.chunk, K::rt_limit(a, I) - rt_begin);
+            prev_ps = rt_begin > 0 ? *(volatile double *)I.st_ps : -1.0;
+            calm = *(volatile int *)I.st_calm;
+            tol = a.tol;
+            patience = a.patience;
+        }
+        E.load(I);
+
+        double ps = prev_ps, acc = 0.0;
+        int rts = 0, flag = 0;
+        bool stop = false;
+        for (int rt = rt_begin; rt < rt_begin + rt_count && !stop; rt++) {
+            double th[3] = {tab.g_last, 0.0, 0.0};
+            {
+                Ops op{};
+                op.inject = !a.pass_only;
+                if (a.regime == 1) {
+                    /* ReadPump offsets, functions.cuh:196-210 (Q6) */
+                    const int nrt = I.n_rt_total;
+                    op.poff = (rt == 0) ? 0 : ((rt > 0 && rt < nrt - 1) ? (long)rt * N : (long)N * nrt - 1 - N);
+                }
+                op.turn = rk + (size_t)a.n_z * NCO;
+                op.rk1 = rk;
+                op.frame = frame_index(rt, 0);
+                E.stage(op, tab);
+                E.pass(0u, ALL, op, I, tab, rkc, a.eom_idler, th, acc);
+            }
+            /* the pass after the dispersion step of slice s (an engine that
+             * prefetches its coefficients asks for it before that step) */
+            auto between = [&](int s) {
+                Ops op{};
+                op.frame = -1;
+                op.rk0 = rk + (size_t)s * NCO;
+                if (s + 1 < a.n_z) {
+                    op.turn = op.rk0;
+                    op.rk1 = op.rk0 + NCO;
+                    op.frame = frame_index(rt, s + 1);
+                }
+                return op;
+            };
+            for (int s = 0; s < a.n_z; s++) {
+                if constexpr (Engine::STAGED) E.stage(between(s), tab);
+                E.dispersion(tab);
+                if (s + 1 < a.n_z) {
+                    Ops op = between(s);
+                    E.pass(ALL, ALL, op, I, tab, rkc, a.eom_idler, th, acc);
+                }
+            }
+            rts++;
+            Ops end = between(a.n_z - 1);
+            if (a.pass_only) {
+                K::frame_back(end, th);
+                E.pass(ALL, 0u, end, I, tab, rkc, a.eom_idler, th, acc);
+                break;
+            }
+            unsigned in_y = ALL;
+            end.eom = use_eom;
+            if (I.gdd != 0.0) {
+                /* GDD / TOD compensation of the resonant fields (cuOPO.cu:521-553):
+                 * signal and idler go to the frequency domain, the pump stays in time */
+                in_y = ALL & ~1u;
+                E.pass(ALL, in_y, end, I, tab, rkc, a.eom_idler, th, acc);
+                end = Ops{};
+                end.frame = -1;
+                if constexpr (Engine::STAGED) E.stage(end, tab);
+                E.gdd(tab, I);
+            }
+            const bool save = (rt >= I.save_first && rt < I.save_first + I.save_count);
+            end.addphase = 1;
+            end.ph_s = make_double2(I.phase_s[0], I.phase_s[1]);
+            end.ph_i = make_double2(I.phase_i[0], I.phase_i[1]);
+            end.save = save;
+            end.slot = save ? (size_t)(rt - I.save_first) * N : 0;
+            end.power = 1;
+            acc = 0.0;
+            K::frame_back(end, th);
+            E.pass(in_y, 0u, end, I, tab, rkc, a.eom_idler, th, acc);
+            ps = E.power(acc) * tab.inv_n;
+            /* single launches record from rt_begin, batch instances by round trip */
+            if (leader && I.ps_hist) I.ps_hist[I.st_flag ? rt : rt - rt_begin] = ps;
+            if (!(ps == ps) || ps > 1.0e300) {
+                if (leader && a.status) atomicCAS(a.status, 0, (int)ST_NONFINITE);
+                flag = ST_NONFINITE;
+                stop = true;
+            }
+            /* convergence: relative change of the signal power per rt below
+             * tol for `patience` consecutive rts (from the second rt on) */
+            if (tol > 0.0 && prev_ps > 0.0 && ps > 0.0 && fabs(ps - prev_ps) < tol * ps) {
+                if (++calm >= (patience > 0 ? patience : 1) && flag == 0) {
+                    flag = ST_CONVERGED;
+                    stop = true;
+                }
+            } else {
+                calm = 0;
+            }
+            prev_ps = ps;
+            if (E.error()) {
+                flag = ST_TIMEOUT;
+                stop = true;
+            }
+        }
+        E.store();
+        if (threadIdx.x == 0 && E.failed() && a.status) atomicCAS(a.status, 0, (int)ST_TIMEOUT);
+        if (leader) {
+            if (I.rt_done) *I.rt_done = rts;
+            if (I.ps_out) *I.ps_out = ps;
+            if (I.flag_out) *I.flag_out = flag;
+            if (I.st_flag) {
+                *I.st_rt = rt_begin + rts;
+                *I.st_ps = ps;
+                *I.st_calm = calm;
+                *I.st_flag = flag != 0 ? flag : (rt_begin + rts >= K::rt_limit(a, I) ? (int)ST_LIMIT : 0);
+            }
+        }
+        E.barrier();
+    }
+}
+
+template <typename R, int F, int M, int CL, int HM, int MINB>
+__global__ void __launch_bounds__(M / 16, MINB) ssfm_kernel(LaunchArgs a)
+{
+    drive<R, typename Ssfm<R, F, M, CL, HM>::Engine>(a);
 }
 
 }  // namespace cuopo
