@@ -318,6 +318,11 @@ __device__ __forceinline__ StageRot<double2> load_rot(const double2 *row)
     return r;
 }
 
+/* Keeps a value loaded from a constant table in registers: without it the
+ * compiler loads it again wherever it is used. */
+__device__ __forceinline__ void pin(float2 &v) { asm volatile("" : "+f"(v.x), "+f"(v.y)); }
+__device__ __forceinline__ void pin(double2 &v) { asm volatile("" : "+d"(v.x), "+d"(v.y)); }
+
 /* The last radix-16 stage's rotations of thread t. */
 template <int M, typename C>
 struct StageTwiddles {
@@ -330,6 +335,11 @@ struct StageTwiddles {
         if constexpr (SP::P > 1) {
             const int ns = SP::ns(SP::P - 1);
             last = load_rot(tw_row<C>(t % ns, ns));
+#pragma unroll
+            for (int j = 0; j < 3; j++) {
+                pin(last.a[j]);
+                pin(last.b[j]);
+            }
         }
     }
 };
@@ -398,11 +408,17 @@ __device__ __forceinline__ void store_own(C *buf, const C (&reg)[16], int t)
  * Local M-point transform of the registers of the CTA (exponent sign S).
  * Exchange x (counted from X0 within the caller's sequence) goes through
  * buffer (x even ? bufA : bufB).  INPLACE: bufA == bufB, and every
- * exchange is bracketed by two barriers instead of one.
+ * exchange is bracketed by two barriers instead of one.  `early` runs while
+ * the last exchange is under way (its stores are issued, no register holds
+ * data): loads issued there have the barrier and the last stage to arrive.
  */
-template <int S, int M, int X0, bool INPLACE, int P_IDX = 0, typename C>
+struct NoEarly {
+    __device__ __forceinline__ void operator()() const {}
+};
+
+template <int S, int M, int X0, bool INPLACE, int P_IDX = 0, typename C, typename Early = NoEarly>
 __device__ __forceinline__ void local_transform(C (&reg)[16], C *bufA, C *bufB,
-                                                const StageTwiddles<M, C> &tw, int t)
+                                                const StageTwiddles<M, C> &tw, int t, const Early &early = Early())
 {
     constexpr int P = StagePlan<M>::P;
     stage_compute<S, M, P_IDX>(reg, tw);
@@ -410,10 +426,26 @@ __device__ __forceinline__ void local_transform(C (&reg)[16], C *bufA, C *bufB,
         C *buf = ((X0 + P_IDX) % 2 == 0) ? bufA : bufB;
         if constexpr (INPLACE) __syncthreads();
         stage_store<M, P_IDX>(buf, reg, t);
+        if constexpr (P_IDX + 2 == P) early();
         __syncthreads();
         load_own<M>(buf, reg, t);
-        local_transform<S, M, X0, INPLACE, P_IDX + 1>(reg, bufA, bufB, tw, t);
+        local_transform<S, M, X0, INPLACE, P_IDX + 1>(reg, bufA, bufB, tw, t, early);
     }
+}
+
+/* Read-only loads that stay where they are written (the compiler moves __ldg
+ * down to its use when registers are short, and every use then waits). */
+__device__ __forceinline__ float2 ld_now(const float2 *p)
+{
+    float2 v;
+    asm volatile("ld.global.nc.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ double2 ld_now(const double2 *p)
+{
+    double2 v;
+    asm volatile("ld.global.nc.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
+    return v;
 }
 
 }  // namespace cuopo

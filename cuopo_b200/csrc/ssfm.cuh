@@ -331,24 +331,50 @@ struct Ssfm {
         RkConst<R> k;
     };
 
-    static __device__ __forceinline__ Coef load_coef(const Ops &op, const RkConst<R> &k)
+    /* The coefficients of the next pass in shared memory: the last warp loads
+     * them before the dispersion step (one entry per lane, in flight
+     * meanwhile) and writes them before a barrier in it, so that no pass
+     * waits for them. */
+    struct Staged {
+        C c[9];      /* rk0: 2, turn: 2, rk1: 2, frame rotations: 3 */
+        double2 u;   /* frame angles */
+    };
+
+    struct Stager {
+        C pf;
+        double2 pf_u;
+
+        /* lane l >= 0 of the last warp */
+        __device__ __forceinline__ void load(int l, const Ops &op, const Tables &tab)
+        {
+            const C *src = nullptr;
+            pf = mk<C>((R)0, (R)0);
+            if (l < 0) return;
+            if (l < 2) src = op.rk0 ? op.rk0 + l : nullptr;
+            else if (l < 4) src = op.turn ? op.turn + l : nullptr;
+            else if (l < 6) src = op.rk1 ? op.rk1 + (l - 4) : nullptr;
+            else if (l < 9 && op.frame >= 0) src = reinterpret_cast<const C *>(tab.frame_c) + 3 * op.frame + (l - 6);
+            if (src) pf = __ldg(src);
+            if (l == 9 && op.frame >= 0) pf_u = tab.frame_u[op.frame];
+        }
+
+        __device__ __forceinline__ void write(int l, Staged *s) const
+        {
+            if (l >= 0 && l < 9) s->c[l] = pf;
+            if (l == 9) s->u = pf_u;
+        }
+    };
+
+    static __device__ __forceinline__ Coef coef(const Staged *s, const RkConst<R> &k)
     {
         Coef c;
-        c.a0 = c.a1 = c.b0 = c.b1 = c.turn = mk<C>((R)0, (R)0);
-        c.turn_q = 0;
         c.k = k;
-        if (op.rk0) {
-            c.a0 = ldc<C>(op.rk0, 0);
-            c.a1 = ldc<C>(op.rk0, 1);
-        }
-        if (op.rk1) {
-            c.b0 = ldc<C>(op.rk1, 0);
-            c.b1 = ldc<C>(op.rk1, 1);
-        }
-        if (op.turn) {
-            c.turn = ldc<C>(op.turn, 2);
-            c.turn_q = (int)ldc<C>(op.turn, 3).x;
-        }
+        c.a0 = s->c[0];
+        c.a1 = s->c[1];
+        c.turn = s->c[2];
+        c.turn_q = (int)s->c[3].x;
+        c.b0 = s->c[4];
+        c.b1 = s->c[5];
         return c;
     }
 
@@ -445,10 +471,9 @@ struct Ssfm {
      * barrier between them. */
     static __device__ __forceinline__ void cross_global(C *const (&gf)[3], unsigned in_y, unsigned out_y,
                                                         const Ops &op, const Instance &I, const Tables &tab,
-                                                        const RkConst<R> &rkc, int eom_idler, double &acc, int t, int rank)
+                                                        const Coef &co, int eom_idler, double &acc, int t, int rank)
     {
         const C *__restrict__ twN = reinterpret_cast<const C *>(tab.twN);
-        const Coef co = load_coef(op, rkc);
 #pragma unroll 1
         for (int j = 0; j < J; j++) {
             const int n1 = rank * (M / CL) + t + j * T;
@@ -481,14 +506,13 @@ struct Ssfm {
      * CTA's home; it reads and writes only those. */
     static __device__ __forceinline__ void cross(C *home, C *const (&gf)[3], unsigned in_y, unsigned out_y,
                                                  const Ops &op, const Instance &I, const Tables &tab,
-                                                 const RkConst<R> &rkc, int eom_idler, double &acc, int t, int rank)
+                                                 const Coef &co, int eom_idler, double &acc, int t, int rank)
     {
         if constexpr (GH) {
-            cross_global(gf, in_y, out_y, op, I, tab, rkc, eom_idler, acc, t, rank);
+            cross_global(gf, in_y, out_y, op, I, tab, co, eom_idler, acc, t, rank);
             return;
         }
         const C *__restrict__ twN = reinterpret_cast<const C *>(tab.twN);
-        const Coef co = load_coef(op, rkc);
 #pragma unroll 1
         for (int j = 0; j < J; j++) {
             const int n1 = rank * (M / CL) + t + j * T;
@@ -566,14 +590,18 @@ struct Ssfm {
         }
         C *bufA = GH ? scratch : (INPLACE ? home : scratch);
         C *bufB = GH ? scratch : home;
-        local_transform<+1, M, 0, INPLACE>(reg, bufA, bufB, tw, t);
+        C d[16];
+        local_transform<+1, M, 0, INPLACE>(reg, bufA, bufB, tw, t, [&]() {
+            if constexpr (MODE == 0) {
+#pragma unroll
+                for (int e = 0; e < 16; e++) d[e] = ld_now(row + t + e * T);
+            }
+        });
         /* the factor F = 1 + d is applied as (A + A d) / N (1/N is exact) */
         const R s_n = (R)inv_n;
         if constexpr (MODE == 0) {
 #pragma unroll
-            for (int e = 0; e < 16; e++) {
-                reg[e] = caddmul(cscale(reg[e], s_n), __ldg(row + t + e * T));
-            }
+            for (int e = 0; e < 16; e++) reg[e] = caddmul(cscale(reg[e], s_n), d[e]);
         } else {
             gdd_factor(reg, w + t, T, gdd, tod, use_tod, s_n);
         }
@@ -593,14 +621,18 @@ struct Ssfm {
         C *home, *scratch;
         C *gf[3];
         StageTwiddles<M, C> tw;
+        Staged *staged;
+        Stager st;
         int t, rank;
 
         __device__ __forceinline__ void init()
         {
             extern __shared__ __align__(16) unsigned char smem_raw[];
             C *const sm = reinterpret_cast<C *>(smem_raw);
+            __shared__ Staged s_staged;
             home = GH ? nullptr : sm;
             scratch = GH ? sm : (INPLACE ? home : home + (size_t)F * M);
+            staged = &s_staged;
             t = threadIdx.x;
             rank = 0;
             if constexpr (CL > 1) rank = (int)cg::this_cluster().block_rank();
@@ -651,16 +683,23 @@ struct Ssfm {
             return GH ? gf[f] + (size_t)rank * M : home + (size_t)f * M;
         }
 
-        static constexpr bool STAGED = false;
-        __device__ __forceinline__ void stage(const Ops &, const Tables &) {}
+        /* Starts the loads of the next pass's coefficients; `now`: no
+         * dispersion step comes before that pass. */
+        __device__ __forceinline__ void stage(const Ops &op, const Tables &tab, bool now)
+        {
+            st.load(t - (T - 32), op, tab);
+            if (now) {
+                st.write(t - (T - 32), staged);
+                __syncthreads();
+            }
+        }
 
         __device__ __forceinline__ void pass(unsigned in_y, unsigned out_y, Ops &op, const Instance &I,
                                              const Tables &tab, const RkConst<R> &rkc, int eom_idler, double (&th)[3],
                                              double &acc)
         {
-            if (op.frame >= 0)
-                frame_step(op, reinterpret_cast<const C *>(tab.frame_c) + 3 * op.frame, tab.frame_u[op.frame], th);
-            cross(home, gf, in_y, out_y, op, I, tab, rkc, eom_idler, acc, t, rank);
+            if (op.frame >= 0) frame_step(op, staged->c + 6, staged->u, th);
+            cross(home, gf, in_y, out_y, op, I, tab, coef(staged, rkc), eom_idler, acc, t, rank);
             if (!op.power) xsync(); /* (power() synchronises) */
         }
 
@@ -668,9 +707,12 @@ struct Ssfm {
         {
             const C *__restrict__ disp = reinterpret_cast<const C *>(tab.disp);
 #pragma unroll 1
-            for (int f = 0; f < F; f++)
+            for (int f = 0; f < F; f++) {
                 spectral<0>(fld(f), scratch, disp + ((size_t)f * CL + rank) * M, nullptr, 0.0, 0.0, 0, tab.inv_n, tw,
                             t);
+                /* (the next field's exchanges make it visible) */
+                if (f == 0) st.write(t - (T - 32), staged);
+            }
             xsync();
         }
 
@@ -680,6 +722,7 @@ struct Ssfm {
         __device__ __forceinline__ void gdd(const Tables &tab, const Instance &I)
         {
             const float *__restrict__ w = tab.w + (size_t)rank * M;
+            st.write(t - (T - 32), staged);
             spectral<1>(fld(1), scratch, nullptr, w, I.gdd, I.tod_s, I.use_tod_s, tab.inv_n, tw, t);
             if constexpr (F == 3)
                 spectral<1>(fld(2), scratch, nullptr, w, I.gdd, I.tod_i, I.use_tod_i, tab.inv_n, tw, t);
@@ -800,11 +843,10 @@ static __device__ __forceinline__ void drive(const LaunchArgs &a)
                 op.turn = rk + (size_t)a.n_z * NCO;
                 op.rk1 = rk;
                 op.frame = frame_index(rt, 0);
-                E.stage(op, tab);
+                E.stage(op, tab, true);
                 E.pass(0u, ALL, op, I, tab, rkc, a.eom_idler, th, acc);
             }
-            /* the pass after the dispersion step of slice s (an engine that
-             * prefetches its coefficients asks for it before that step) */
+            /* the pass after the dispersion step of slice s */
             auto between = [&](int s) {
                 Ops op{};
                 op.frame = -1;
@@ -817,7 +859,7 @@ static __device__ __forceinline__ void drive(const LaunchArgs &a)
                 return op;
             };
             for (int s = 0; s < a.n_z; s++) {
-                if constexpr (Engine::STAGED) E.stage(between(s), tab);
+                E.stage(between(s), tab, false);
                 E.dispersion(tab);
                 if (s + 1 < a.n_z) {
                     Ops op = between(s);
@@ -840,7 +882,7 @@ static __device__ __forceinline__ void drive(const LaunchArgs &a)
                 E.pass(ALL, in_y, end, I, tab, rkc, a.eom_idler, th, acc);
                 end = Ops{};
                 end.frame = -1;
-                if constexpr (Engine::STAGED) E.stage(end, tab);
+                E.stage(end, tab, false);
                 E.gdd(tab, I);
             }
             const bool save = (rt >= I.save_first && rt < I.save_first + I.save_count);

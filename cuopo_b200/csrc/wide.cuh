@@ -138,23 +138,15 @@ struct Wide {
         __device__ __forceinline__ StageRot<C> rot_3() const { return load_rot(tw_row<C>(lane % R0, R0)); }
     };
 
-    /* Coefficients of one pass, staged in shared memory. */
-    struct Staged {
-        C c[9];      /* rk0: 2, turn: 2, rk1: 2, frame rotations: 3 */
-        double2 u;   /* frame angles */
-    };
-
     struct Engine {
         using Math = Wide::Math;
-        static constexpr bool STAGED = true;
         C *tb;      /* [F][CL][16][Tc]: time side, point t2 + T e + M c at [f][c][e][t2 - rank Tc] */
         C *fb;      /* [F][U][256]: frequency side, entry j of transform (k2, r) */
         C *gf[3];
         unsigned long long *mbar;  /* [3 b + f]: field f of buffer b (0: tb, 1: fb) */
         int *dead;                 /* [0]: a wait of this CTA gave up; [1 + c]: CTA c's, after power() */
-        Staged *staged;
-        C pf;                      /* this lane's staged coefficient on its way */
-        double2 pf_u;
+        typename Math::Staged *staged;
+        typename Math::Stager st;
         unsigned parity;           /* bit 3 b + f: parity of that mbarrier's next phase */
         int tid, rank;
         StageRot<C> w_t, w_1, w_2, w_3; /* HOLD_TW: this thread's rotations */
@@ -164,7 +156,7 @@ struct Wide {
             extern __shared__ __align__(16) unsigned char smem_raw[];
             __shared__ unsigned long long s_mbar[6];
             __shared__ int s_dead[1 + P];
-            __shared__ Staged s_staged;
+            __shared__ typename Math::Staged s_staged;
             tb = reinterpret_cast<C *>(smem_raw);
             fb = tb + buf_elems();
             mbar = s_mbar;
@@ -174,8 +166,6 @@ struct Wide {
             tid = threadIdx.x;
             rank = 0;
             if constexpr (P > 1) rank = (int)cg::this_cluster().block_rank();
-            pf = mk<C>((R)0, (R)0);
-            pf_u = make_double2(0.0, 0.0);
             if (tid <= P) s_dead[tid] = 0;
             if constexpr (P > 1) {
                 if (tid < 6)
@@ -261,19 +251,11 @@ struct Wide {
             return e;
         }
 
-        /* Starts the loads of a pass's coefficients (the last warp: one entry
-         * per lane); pass() writes them to shared memory. */
-        __device__ __forceinline__ void stage(const Ops &op, const Tables &tab)
+        /* Starts the loads of the next pass's coefficients (pass() writes them
+         * to shared memory before its first barrier). */
+        __device__ __forceinline__ void stage(const Ops &op, const Tables &tab, bool)
         {
-            const int l = tid - (NTHR - 32);
-            if (l < 0) return;
-            const C *src = nullptr;
-            if (l < 2) src = op.rk0 ? op.rk0 + l : nullptr;
-            else if (l < 4) src = op.turn ? op.turn + l : nullptr;
-            else if (l < 6) src = op.rk1 ? op.rk1 + (l - 4) : nullptr;
-            else if (l < 9) src = op.frame >= 0 ? reinterpret_cast<const C *>(tab.frame_c) + 3 * op.frame + (l - 6) : nullptr;
-            pf = src ? __ldg(src) : mk<C>((R)0, (R)0);
-            if (l == 9 && op.frame >= 0) pf_u = tab.frame_u[op.frame];
+            st.load(tid - (NTHR - 32), op, tab);
         }
 
         /* index into the global fields of entry i (position and cross index) of the time side */
@@ -308,11 +290,7 @@ struct Wide {
                                              double &acc)
         {
             const C *__restrict__ twN = reinterpret_cast<const C *>(tab.twN);
-            if (tid >= NTHR - 32) {
-                const int l = tid - (NTHR - 32);
-                if (l < 9) staged->c[l] = pf;
-                if (l == 9) staged->u = pf_u;
-            }
+            st.write(tid - (NTHR - 32), staged);
             if (in_y) {
 #pragma unroll 1
                 for (int task = tid; task < NT; task += NTHR) {
@@ -334,14 +312,7 @@ struct Wide {
                 flip(0, in_y);
             }
             __syncthreads();
-            typename Math::Coef co;
-            co.k = rkc;
-            co.a0 = staged->c[0];
-            co.a1 = staged->c[1];
-            co.turn = staged->c[2];
-            co.turn_q = (int)staged->c[3].x;
-            co.b0 = staged->c[4];
-            co.b1 = staged->c[5];
+            const typename Math::Coef co = Math::coef(staged, rkc);
             if (op.frame >= 0) Math::frame_step(op, staged->c + 6, staged->u, th);
             if (out_y) expect(1, out_y);
             if constexpr (SPLIT) {
@@ -456,7 +427,7 @@ struct Wide {
                 C v[16], d[EARLY_ROWS ? 16 : 1];
                 if constexpr (MODE == 0 && EARLY_ROWS) {
 #pragma unroll
-                    for (int e = 0; e < 16; e++) d[e] = __ldg(disp + 16 * e);
+                    for (int e = 0; e < 16; e++) d[e] = ld_now(disp + 16 * e);
                 }
                 wait(1, o.f);
                 /* stage 1 (length R0): butterfly `lane`, k = r */
