@@ -61,12 +61,14 @@ struct Launcher {
     /* Clusters that can be resident at once (0 on error). */
     static int occupancy()
     {
-        if (prepare() != cudaSuccess) return 0;
-        cudaLaunchAttribute attr[1];
-        cudaLaunchConfig_t cfg = config(1, 0, attr);
-        int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, KERNEL, &cfg) != cudaSuccess) return 0;
-        return n;
+        static const int clusters = [] {
+            cudaLaunchAttribute attr[1];
+            cudaLaunchConfig_t cfg = config(1, 0, attr);
+            int n = 0;
+            if (prepare() != cudaSuccess || cudaOccupancyMaxActiveClusters(&n, KERNEL, &cfg) != cudaSuccess) n = 0;
+            return n;
+        }();
+        return clusters;
     }
 };
 
@@ -75,21 +77,26 @@ struct KernelEntry {
     int home;           /* 0, 1: fields in shared memory (1: in place); 2: in global memory */
     int ctas, threads;  /* per instance, per CTA */
     int wide;           /* wide_kernel: its order of the frequency tables (freq_slot) */
+    float us1, us_full; /* measured time per slice [us] with at most one CTA per SM, and with every
+                           resident cluster busy (B200, 1965 MHz); 0: not compared */
     size_t smem;
     launch_fn fn;
     occ_fn occ;
 };
 
-#define CUOPO_K(R, PREC, F, M, CL, HM, MINB)                                                                   \
-    {PREC, F, M, CL, HM, CL, M / 16, 0, Ssfm<R, F, M, CL, HM>::smem_bytes(),                                       \
+#define CUOPO_K(R, PREC, F, M, CL, HM, MINB, US1, USF)                                                         \
+    {PREC, F, M, CL, HM, CL, M / 16, 0, US1, USF, Ssfm<R, F, M, CL, HM>::smem_bytes(),                          \
      &Launcher<&ssfm_kernel<R, F, M, CL, HM, MINB>, CL, M / 16, Ssfm<R, F, M, CL, HM>::smem_bytes()>::launch,    \
      &Launcher<&ssfm_kernel<R, F, M, CL, HM, MINB>, CL, M / 16, Ssfm<R, F, M, CL, HM>::smem_bytes()>::occupancy}
 
-/* The same arithmetic (M, CL) spread over P CTAs of NTHR threads (wide.cuh). */
-#define CUOPO_W(R, PREC, F, M, CL, P, NTHR)                                                                    \
-    {PREC, F, M, CL, 0, P, NTHR, 1, Wide<R, F, M, CL, P, NTHR>::smem_bytes(),                                      \
-     &Launcher<&wide_kernel<R, F, M, CL, P, NTHR>, P, NTHR, Wide<R, F, M, CL, P, NTHR>::smem_bytes()>::launch,   \
-     &Launcher<&wide_kernel<R, F, M, CL, P, NTHR>, P, NTHR, Wide<R, F, M, CL, P, NTHR>::smem_bytes()>::occupancy}
+/* The same arithmetic (M, CL) spread over P CTAs of NTHR threads, at least
+ * MINB on an SM (wide.cuh). */
+#define CUOPO_W(R, PREC, F, M, CL, P, NTHR, MINB, US1, USF)                                                    \
+    {PREC, F, M, CL, 0, P, NTHR, 1, US1, USF, Wide<R, F, M, CL, P, NTHR, MINB>::smem_bytes(),                   \
+     &Launcher<&wide_kernel<R, F, M, CL, P, NTHR, MINB>, P, NTHR,                                               \
+               Wide<R, F, M, CL, P, NTHR, MINB>::smem_bytes()>::launch,                                         \
+     &Launcher<&wide_kernel<R, F, M, CL, P, NTHR, MINB>, P, NTHR,                                               \
+               Wide<R, F, M, CL, P, NTHR, MINB>::smem_bytes()>::occupancy}
 
 /* Configurations of one precision and number of equations. */
 struct KernelList {

@@ -106,17 +106,40 @@ static const KernelEntry *find_kernel(int precision, int F, int N, bool single_c
     return found;
 }
 
-/* The few-instance kernel with the same arithmetic as k, or NULL. */
-static const KernelEntry *find_wide(const KernelEntry *k)
+/* Measured time per slice of `count` instances on kernel k: its resident
+ * clusters work through them in waves. */
+static double slice_time(const KernelEntry &k, int count)
+{
+    const int occ = k.occ();
+    if (occ < 1 || k.us1 <= 0) return 1e30;
+    const int waves = count / occ, rest = count % occ;
+    return waves * (double)k.us_full + (rest == 0 ? 0.0 : rest * k.ctas <= 148 ? (double)k.us1 : (double)k.us_full);
+}
+
+/* The layout of k's arithmetic (same M and CL: the same results bit for bit)
+ * that runs `count` instances fastest.  A 2^12-point instance, for example,
+ * takes 11.1 us per slice on one CTA and 3.1 spread over 16, but only 14 of
+ * those clusters are resident against 296 CTAs, so between 15 and 33
+ * instances 4 CTAs each are best (4.2 us), then 2 each (7.1) up to 74, then
+ * one.  A kernel chosen by hand (cuopo_kernel_select) keeps its M and CL; one
+ * that the autotuner is timing runs as it is. */
+static const KernelEntry *pick_layout(const KernelEntry *k, int count)
 {
     static const KernelList *const lists[] = {&wide_f32_2eq, &wide_f32_3eq, &wide_f64_2eq, &wide_f64_3eq};
-    if (k->home != 2)
-        for (const KernelList *l : lists)
-            for (int i = 0; i < l->n; i++) {
-                const KernelEntry &w = l->k[i];
-                if (w.precision == k->precision && w.F == k->F && w.M == k->M && w.CL == k->CL) return &w;
+    if (!k || k == g_force || k->home == 2) return k;
+    const KernelEntry *best = k;
+    double t = slice_time(*k, count);
+    for (const KernelList *l : lists)
+        for (int i = 0; i < l->n; i++) {
+            const KernelEntry &w = l->k[i];
+            if (w.precision != k->precision || w.F != k->F || w.M != k->M || w.CL != k->CL) continue;
+            const double tw = slice_time(w, count);
+            if (tw < t) {
+                best = &w;
+                t = tw;
             }
-    return nullptr;
+        }
+    return best;
 }
 
 /* Place of frequency q = k2 + CL k1 in the kernel's tables: per CTA in the
@@ -124,9 +147,11 @@ static const KernelEntry *find_wide(const KernelEntry *k)
  * lanes side by side, k1 = r + R0 lane + T e. */
 static size_t freq_slot(const KernelEntry *k, int q)
 {
-    const int k2 = q % k->CL, k1 = q / k->CL;
+    /* (M, CL and R0 are powers of 2) */
+    const int k2 = q & (k->CL - 1), k1 = q >> __builtin_ctz((unsigned)k->CL);
     if (!k->wide) return (size_t)k2 * k->M + k1;
-    const int T = k->M / 16, R0 = k->M / 256, e = k1 / T, r = k1 % T % R0, lane = k1 % T / R0;
+    const int T = k->M >> 4, R0 = k->M >> 8, t = k1 & (T - 1);
+    const int e = k1 >> __builtin_ctz((unsigned)T), r = t & (R0 - 1), lane = t >> __builtin_ctz((unsigned)R0);
     return ((size_t)(k2 * R0 + r) * 16 + e) * 16 + lane;
 }
 
@@ -302,10 +327,8 @@ static cuopo_status plan_create(cuopo_plan **out, const cuopo_params *p, const f
     const bool phase32 = precision == CUOPO_F32_PHASE32;
     if (phase32) precision = CUOPO_F32;
     if (!k) {
-        /* a plan runs one instance at a time: its few-instance kernel, where there is one */
-        k = find_kernel(precision, p->n_eqs, p->n_t);
-        const KernelEntry *wide = k ? find_wide(k) : nullptr;
-        if (wide) k = wide;
+        /* a plan runs one instance at a time */
+        k = pick_layout(find_kernel(precision, p->n_eqs, p->n_t), 1);
     }
     if (!k) return cuopo_fail(CUOPO_EUNSUPPORTED, "no kernel built for this (precision, n_eqs, n_t)");
 
@@ -560,14 +583,6 @@ struct BatchGroup {
     int grid;
 };
 
-/* The kernel of a batch group of `count` instances. */
-static const KernelEntry *pick_batch_kernel(int precision, int F, int n_t, int count)
-{
-    const KernelEntry *k = find_kernel(precision, F, n_t), *wide = find_wide(k);
-    if (!wide || g_force) return k;
-    return count <= wide->occ() ? wide : k;
-}
-
 struct cuopo_batch {
     int count;
     int precision;
@@ -746,6 +761,8 @@ static cuopo_status batch_build(cuopo_batch **out, const std::vector<cuopo_param
         return x[1] != y[1] ? x[1] > y[1] : x < y;
     });
     b->h_inst.resize((size_t)count);
+    long batch_ctas = 0;
+    for (const cuopo_params &p : prm) batch_ctas += find_kernel(precision, p.n_eqs, p.n_t)->ctas;
     for (const std::array<int, 5> &key : keys) {
         b->groups.push_back(BatchGroup{});
         BatchGroup &g = b->groups.back();
@@ -754,11 +771,10 @@ static cuopo_status batch_build(cuopo_batch **out, const std::vector<cuopo_param
         g.n_z = key[2];
         g.eom_idler = key[3];
         g.regime = key[4];
-        int members = 0;
-        for (const cuopo_params &p : prm)
-            members += p.n_eqs == g.F && p.n_t == g.n_t && p.n_z == g.n_z && p.eom_idler == g.eom_idler &&
-                       p.regime == g.regime;
-        g.kernel = pick_batch_kernel(precision, g.F, g.n_t, members);
+        /* the groups share the chip: as many instances of this group as would
+         * need the CTAs of all of them */
+        const KernelEntry *k = find_kernel(precision, g.F, g.n_t);
+        g.kernel = pick_layout(k, (int)((batch_ctas + k->ctas - 1) / k->ctas));
         std::vector<std::vector<double>> pkeys;
         std::vector<int> plan_of;
         for (int i = 0; i < count; i++) {
@@ -1067,8 +1083,9 @@ extern "C" cuopo_status cuopo_autotune(const cuopo_params *base, int precision, 
     if (cand.empty()) return cuopo_fail(CUOPO_EUNSUPPORTED, "autotune: no kernel built for this (precision, n_eqs, n_t)");
     const KernelEntry *best = cand[0];
     double best_ms = -1.0;
-    if (cand.size() > 1) {
-        if (F != 2 || base->regime != CUOPO_CW)
+    /* (3-equation grids: the built-in choice, no timing runs) */
+    if (cand.size() > 1 && F == 2) {
+        if (base->regime != CUOPO_CW)
             return cuopo_fail(CUOPO_EUNSUPPORTED, "autotune: timing runs use CW 2-equation batches");
         /* `count` copies of the base instance, seeded noise, n_rt round trips
          * with the convergence test off (fixed work), per candidate */
@@ -1210,7 +1227,7 @@ extern "C" cuopo_status cuopo_crystal_pass_noalloc(const cuopo_params *p, const 
     if (p->n_z < 1 || p->n_z > CUOPO_NOALLOC_MAX_NZ)
         return cuopo_fail(CUOPO_EINVAL, "crystal_pass_noalloc: n_z must be in [1, 1024]");
     const KernelEntry *k = find_kernel(CUOPO_F32, p->n_eqs, p->n_t, true);
-    if (k && find_wide(k)) k = find_wide(k);
+    k = pick_layout(k, 1);
     if (!k) return cuopo_fail(CUOPO_EUNSUPPORTED, "crystal_pass_noalloc: no single-CTA kernel for n_t");
     const int N = p->n_t, F = p->n_eqs;
 

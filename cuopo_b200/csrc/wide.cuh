@@ -89,7 +89,7 @@ __device__ __forceinline__ bool mbar_test(unsigned mbar, unsigned parity)
     return ok != 0;
 }
 
-template <typename R, int F, int M, int CL, int P, int NTHR>
+template <typename R, int F, int M, int CL, int P, int NTHR, int MINB>
 struct Wide {
     using Math = Ssfm<R, F, M, CL, 0>;
     using C = cpx<R>;
@@ -110,8 +110,8 @@ struct Wide {
     static_assert(R0 % P == 0 && P <= 16 && NTHR % 32 == 0 && NT % 16 == 0, "cluster size divides the first radix");
 
     /* stage rotations and dispersion rows kept in registers */
-    static constexpr bool HOLD_TW = sizeof(R) == 4 && NT <= NTHR && NTHR <= 256;
-    static constexpr bool EARLY_ROWS = NTHR <= 256;
+    static constexpr bool HOLD_TW = sizeof(R) == 4 && NT <= NTHR && NTHR * MINB <= 256;
+    static constexpr bool EARLY_ROWS = NTHR * MINB <= 256;
 
     static constexpr size_t buf_elems() { return (size_t)F * CL * NP; }
     static constexpr size_t smem_bytes() { return sizeof(C) * 2 * buf_elems(); }
@@ -527,10 +527,10 @@ struct Wide {
     };
 };
 
-template <typename R, int F, int M, int CL, int P, int NTHR>
-__global__ void __launch_bounds__(NTHR, 1) wide_kernel(LaunchArgs a)
+template <typename R, int F, int M, int CL, int P, int NTHR, int MINB>
+__global__ void __launch_bounds__(NTHR, MINB) wide_kernel(LaunchArgs a)
 {
-    drive<R, typename Wide<R, F, M, CL, P, NTHR>::Engine>(a);
+    drive<R, typename Wide<R, F, M, CL, P, NTHR, MINB>::Engine>(a);
 }
 
 }  // namespace cuopo
