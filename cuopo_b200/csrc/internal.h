@@ -19,6 +19,19 @@ cuopo_status cuopo_fail(cuopo_status st, const char *msg);
 void cuopo_noise_pair_host(uint64_t seed, uint64_t stream_id, uint64_t i, double sigma,
                            float *re, float *im);
 
+/* Noise of one batch instance: n values at element `offset` of the signal
+ * buffer (stream 0) and, with 3 fields, of the idler buffer (stream 1). */
+typedef struct {
+    long offset;
+    int n, fields;
+    uint64_t seed;
+} cuopo_noise_item;
+
+/* The values cuopo_noise_device gives, for every instance in one launch;
+ * items in device memory, n_max the largest n. */
+cuopo_status cuopo_noise_batch(void *signal, void *idler, const cuopo_noise_item *items, int count, int n_max,
+                               double sigma, void *stream);
+
 #ifdef __cplusplus
 }
 

@@ -68,7 +68,38 @@ __global__ void noise_kernel(float2 *out, long n, double sigma, uint64_t seed, u
     }
 }
 
+/* Every instance of a batch: one row of blocks per instance (blockIdx.y, by
+ * steps of gridDim.y), the signal's stream and then the idler's.  A launch
+ * per instance and field cost 2.7 us each, 0.9 ms before a sweep of 333. */
+__global__ void noise_batch_kernel(float2 *signal, float2 *idler, const cuopo_noise_item *items, int count,
+                                   double sigma)
+{
+    for (int k = blockIdx.y; k < count; k += gridDim.y) {
+        const cuopo_noise_item it = items[k];
+        const int total = it.fields == 3 ? 2 * it.n : it.n;
+        for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < total; j += gridDim.x * blockDim.x) {
+            const int s = j >= it.n, i = s ? j - it.n : j;
+            float re, im;
+            noise_pair(it.seed, (uint64_t)s, (uint64_t)i, sigma, &re, &im);
+            (s ? idler : signal)[it.offset + i] = make_float2(re, im);
+        }
+    }
+}
+
 }  // namespace
+
+extern "C" cuopo_status cuopo_noise_batch(void *signal, void *idler, const cuopo_noise_item *items, int count,
+                                          int n_max, double sigma, void *stream)
+{
+    const int threads = 256;
+    /* one field of the largest instance per row of blocks */
+    const dim3 grid((unsigned)((n_max + threads - 1) / threads), (unsigned)(count < 65535 ? count : 65535));
+    noise_batch_kernel<<<grid, threads, 0, (cudaStream_t)stream>>>((float2 *)signal, (float2 *)idler, items, count,
+                                                                  sigma);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return cuopo_fail(CUOPO_ECUDA, cudaGetErrorString(e));
+    return CUOPO_OK;
+}
 
 extern "C" void cuopo_noise_pair_host(uint64_t seed, uint64_t stream_id, uint64_t i, double sigma, float *re,
                                       float *im)

@@ -588,6 +588,7 @@ struct cuopo_batch {
     int precision;
     std::vector<int> n_t, F;
     std::vector<uint64_t> seed;
+    cuopo_noise_item *d_noise;    /* per instance: place, size and seed of its noise */
     std::vector<size_t> offset;   /* element offset of each instance's fields */
     size_t total;                 /* total signal elements */
     void *d_pump;                 /* pump-field work buffers (n_t per instance) */
@@ -628,6 +629,7 @@ extern "C" cuopo_status cuopo_batch_destroy(cuopo_batch *b)
     cudaFree(b->d_rt);
     cudaFree(b->d_flag);
     cudaFree(b->d_calm);
+    cudaFree(b->d_noise);
     delete b;
     return CUOPO_OK;
 }
@@ -700,6 +702,7 @@ static cuopo_status batch_build(cuopo_batch **out, const std::vector<cuopo_param
         (e = cudaMalloc(&b->d_rt, sizeof(int) * count)) != cudaSuccess ||
         (e = cudaMalloc(&b->d_flag, sizeof(int) * count)) != cudaSuccess ||
         (e = cudaMalloc(&b->d_calm, sizeof(int) * count)) != cudaSuccess ||
+        (e = cudaMalloc(&b->d_noise, sizeof(cuopo_noise_item) * count)) != cudaSuccess ||
         (e = cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming)) != cudaSuccess) {
         cuopo_batch_destroy(b);
         return e == cudaErrorMemoryAllocation ? cuopo_fail(CUOPO_ENOMEM, "batch_create: device allocation failed")
@@ -713,6 +716,16 @@ static cuopo_status batch_build(cuopo_batch **out, const std::vector<cuopo_param
     cudaMemset(b->d_flag, 0, sizeof(int) * count);
     cudaMemset(b->d_calm, 0, sizeof(int) * count);
     if (b->d_hist) cudaMemset(b->d_hist, 0, sizeof(double) * hist_total);
+    {
+        std::vector<cuopo_noise_item> items((size_t)count);
+        for (int i = 0; i < count; i++)
+            items[(size_t)i] = {(long)b->offset[(size_t)i], b->n_t[(size_t)i], b->F[(size_t)i], seeds[(size_t)i]};
+        if ((e = cudaMemcpy(b->d_noise, items.data(), sizeof(cuopo_noise_item) * items.size(),
+                            cudaMemcpyHostToDevice)) != cudaSuccess) {
+            cuopo_batch_destroy(b);
+            return cuda_fail(e, "batch_create: noise seeds");
+        }
+    }
     /* nanosecond pump windows (cuOPO.cu:164-175,243-248), built on the host as
      * the reference does, one per nanosecond instance */
     std::vector<size_t> win_off((size_t)count, 0);
@@ -928,15 +941,8 @@ extern "C" cuopo_status cuopo_batch_seed_noise(cuopo_batch *b, double sigma, voi
         if (js != CUOPO_OK) return js;
     }
     if (b->precision != CUOPO_F32) return cuopo_fail(CUOPO_EUNSUPPORTED, "batch_seed_noise: F32 batches only");
-    for (int i = 0; i < b->count; i++) {
-        cuopo_status st = cuopo_noise_device((char *)b->d_signal + 8 * b->offset[(size_t)i], b->n_t[(size_t)i], sigma,
-                                             b->seed[(size_t)i], 0, stream);
-        if (st == CUOPO_OK && b->F[(size_t)i] == 3)
-            st = cuopo_noise_device((char *)b->d_idler + 8 * b->offset[(size_t)i], b->n_t[(size_t)i], sigma,
-                                    b->seed[(size_t)i], 1, stream);
-        if (st != CUOPO_OK) return st;
-    }
-    return CUOPO_OK;
+    return cuopo_noise_batch(b->d_signal, b->d_idler, b->d_noise, b->count,
+                             *std::max_element(b->n_t.begin(), b->n_t.end()), sigma, stream);
 }
 
 extern "C" cuopo_status cuopo_batch_set_signal(cuopo_batch *b, const void *src, int on_device, void *stream)
