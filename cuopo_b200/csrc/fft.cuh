@@ -433,6 +433,21 @@ __device__ __forceinline__ void local_transform(C (&reg)[16], C *bufA, C *bufB,
     }
 }
 
+/* Loads that stay where they are written; in-place transforms read data
+ * that the kernel writes elsewhere, so not through the read-only path. */
+__device__ __forceinline__ float2 ld_stream(const float2 *p)
+{
+    float2 v;
+    asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ double2 ld_stream(const double2 *p)
+{
+    double2 v;
+    asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
+    return v;
+}
+
 /* Read-only loads that stay where they are written (the compiler moves __ldg
  * down to its use when registers are short, and every use then waits). */
 __device__ __forceinline__ float2 ld_now(const float2 *p)

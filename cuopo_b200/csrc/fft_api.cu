@@ -15,6 +15,20 @@ using namespace cuopo;
 
 namespace {
 
+/* The buffers of an M-point transform leave room for one CTA per SM (2^13
+ * FP32, 2^12 FP64 points). */
+template <typename R, int M>
+constexpr bool one_per_sm()
+{
+    return 2 * M * sizeof(cpx<R>) > 114 * 1024;
+}
+
+/* Transforms blockIdx.x, + gridDim.x, ...  With one CTA per SM the grid is
+ * persistent and the next transform's points are loaded into registers
+ * before the current one is computed; otherwise the loads wait for the
+ * previous transform's stores and nothing is in flight meanwhile.  With
+ * several CTAs per SM these overlap one another, and the extra registers
+ * would cost some of them. */
 template <typename R, int M, int S>
 __global__ void __launch_bounds__(M / 16) fft_kernel(const cpx<R> *in, cpx<R> *out, int batch)
 {
@@ -25,16 +39,33 @@ __global__ void __launch_bounds__(M / 16) fft_kernel(const cpx<R> *in, cpx<R> *o
     C *bufB = bufA + M;
     C *tab = bufB + M;
     const int t = threadIdx.x;
+    constexpr bool AHEAD = one_per_sm<R, M>();
+    int b = blockIdx.x;
+    C next[AHEAD ? 16 : 1];
+    if constexpr (AHEAD) {
+#pragma unroll
+        for (int e = 0; e < 16; e++) next[e] = ld_stream(in + (size_t)b * M + t + e * T);
+    }
     fill_twiddle_table<M>(tab, t);
     StageTwiddles<M, C> tw;
     tw.init(t, tab);
     __syncthreads();
-    for (int b = blockIdx.x; b < batch; b += gridDim.x) {
-        const C *src = in + (size_t)b * M;
+    for (; b < batch; b += gridDim.x) {
         C *dst = out + (size_t)b * M;
         C reg[16];
+        if constexpr (AHEAD) {
 #pragma unroll
-        for (int e = 0; e < 16; e++) reg[e] = src[t + e * T];
+            for (int e = 0; e < 16; e++) reg[e] = next[e];
+            if (b + (int)gridDim.x < batch) {
+                const C *src = in + (size_t)(b + gridDim.x) * M + t;
+#pragma unroll
+                for (int e = 0; e < 16; e++) next[e] = ld_stream(src + e * T);
+            }
+        } else {
+            const C *src = in + (size_t)b * M + t;
+#pragma unroll
+            for (int e = 0; e < 16; e++) reg[e] = src[e * T];
+        }
         local_transform<S, M, 0, false>(reg, bufA, bufB, tw, t);
 #pragma unroll
         for (int e = 0; e < 16; e++) dst[t + e * T] = reg[e];
@@ -52,7 +83,8 @@ cudaError_t launch_fft(const void *in, void *out, int batch, cudaStream_t st)
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int grid = batch < 8 * sms ? batch : 8 * sms;
+    const int most = one_per_sm<R, M>() ? sms : 8 * sms;
+    const int grid = batch < most ? batch : most;
     fft_kernel<R, M, S><<<grid, M / 16, smem, st>>>((const cpx<R> *)in, (cpx<R> *)out, batch);
     return cudaGetLastError();
 }
