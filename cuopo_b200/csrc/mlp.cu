@@ -6,23 +6,26 @@
  * has no counterpart: it always starts a run from noise
  * (src/headers/functions.cuh:58-71).
  *
- * Every contraction of training and inference is one kernel, tc_gemm_kernel:
- * C[M][N] = A[M][K] B[N][K]^T with A and B row-major BF16 ("K-major"), one
- * 128 x BN output tile per CTA, the K loop pipelined through STAGES
- * shared-memory buffers (one TMA producer thread, one MMA issuer thread,
- * mbarriers in between), the accumulator in tensor memory, and a fused
- * epilogue run by 16 warps (TMEM lanes = tile rows, 4 lane quadrants x up
- * to 4 chunks of 32 columns):
- *   forward    z = A W^T + b, h = GELU(z): stores GELU'(z), h and h^T (BF16);
- *   output     y = A W^T + b (FP32);
+ * Every contraction of training and inference is one kernel body, gemm_tile:
+ * C[M][N] = A[M][K] B[N][K]^T in BF16, one 128 x 128 (or x 64) output tile per
+ * CTA, the K loop pipelined through STAGES shared-memory buffers (one TMA
+ * producer thread, one MMA issuer thread, mbarriers in between), the
+ * accumulator in tensor memory, and a fused epilogue run by 16 warps (TMEM
+ * lanes = tile rows, 4 lane quadrants x up to 4 chunks of 32 columns):
+ *   forward    z = A W^T + b, h = GELU(z): stores h and, for training, GELU'(z);
+ *   output     y = A W^T + b (FP32), or for training the loss and its gradient;
  *   dX         g_prev = (g W) * GELU'(z_prev) (the stored derivative):
- *              stores g_prev, g_prev^T and adds the column sums of g_prev
- *              into the bias gradient;
+ *              stores g_prev and adds its column sums into the bias gradient;
  *   dW         grad_W += g^T act over a K slice (split over the batch,
- *              FP32 atomics).
- * Keeping every activation and gradient in both layouts (row-major and
- * transposed, written by the producing epilogue) makes every GEMM of the
- * backward pass a K-major one as well.
+ *              FP32 atomics), all layers in one launch.
+ * Every matrix is stored once, row-major.  An operand whose K runs along the
+ * rows of its matrix (W in dX; g and the activations in dW) is read as it
+ * lies, "MN-major": the same 64 x 64 TMA boxes, another shared-memory matrix
+ * descriptor.  (Storing every activation, gradient and weight transposed as
+ * well cost each epilogue 32 two-byte stores per thread, and a transpose
+ * kernel per step.)  BF16 tiles leave through shared memory and TMA stores,
+ * and dX's derivative tile arrives by TMA during the K loop: from registers
+ * a thread reads and writes its own row, 16 bytes at a time.
  *
  * Device waits on mbarriers are bounded (about 1 s of %globaltimer); a wait
  * that gives up sets the error word and the kernel finishes without storing
@@ -105,8 +108,8 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *b, uint32_t parity)
     return true;
 }
 
-/* 2-D tiled TMA load (no multicast) of box {64, rows} at (x, y) into dst,
- * completing on mbarrier bar. */
+/* 2-D tiled TMA load (no multicast) of box {64, 64} at (x, y) into dst,
+ * completing on mbarrier bar; and the store of one. */
 __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, int x, int y, uint64_t *bar)
 {
     asm volatile(
@@ -114,6 +117,14 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, i
             smem_u32(dst)),
         "l"((unsigned long long)map), "r"(x), "r"(y), "r"(smem_u32(bar))
         : "memory");
+}
+
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap *map, int x, int y, const void *src)
+{
+    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];" ::"l"(
+                     (unsigned long long)map),
+                 "r"(x), "r"(y), "r"(smem_u32(src))
+                 : "memory");
 }
 
 /* Shared-memory matrix descriptor of a K-major tile whose 128-byte rows are
@@ -126,12 +137,21 @@ __device__ __forceinline__ uint64_t sw128_desc(uint32_t saddr)
            ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
 
-/* Instruction descriptor of kind::f16: D FP32, A and B BF16, both K-major,
- * N >> 3 at bit 17, M >> 4 at bit 24. */
-template <int BN>
-__host__ __device__ constexpr uint32_t idesc_bf16()
+/* The same for an MN-major tile: 64 MN elements (one 128-byte row) x 64 K
+ * rows per box; the next 64 MN elements one box (8192 bytes) further (leading
+ * byte offset), the next 8 K rows 1024 bytes (stride byte offset). */
+__device__ __forceinline__ uint64_t sw128_desc_mn(uint32_t saddr)
 {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+    return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)(8192 >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) |
+           ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
+}
+
+/* Instruction descriptor of kind::f16: D FP32, A and B BF16, bit 15 / 16 for
+ * an MN-major A / B, N >> 3 at bit 17, M >> 4 at bit 24. */
+__device__ __forceinline__ uint32_t idesc_bf16(int bn, bool a_mn, bool b_mn)
+{
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)a_mn << 15) | ((uint32_t)b_mn << 16) |
+           ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
 }
 
 __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc)
@@ -214,44 +234,59 @@ __device__ __forceinline__ void gelu_and_grad(float z, float &h, float &gp)
 
 /* ------------------------------------------------------------ epilogue */
 
+/* What becomes of an output tile. */
+enum EpiMode {
+    EPI_F32,    /* out_f = (or, atomic, +=) C */
+    EPI_GELU,   /* h = GELU(C + bias) -> tile 0 */
+    EPI_GELU_T, /* the same, and GELU'(C + bias) -> tile 1 */
+    EPI_Y,      /* out_f = C + bias, rows < batch */
+    EPI_MSE,    /* loss of C + bias against the target, its gradient -> tile 0, column sums */
+    EPI_DX,     /* C * gp_in -> tile 0, column sums */
+    EPI_DW      /* out_f += C */
+};
+
 struct Epi {
-    int ldo;              /* row stride of the row-major outputs (= N of the GEMM) */
-    int ldt;              /* row stride of the transposed output */
-    const float *bias;    /* [N] added first, or NULL */
-    int act;              /* 0 none, 1 GELU, 2 multiply by gp_in */
-    const bf16 *gp_in;    /* GELU'(z) [M][ldo] for act 2 */
-    bf16 *gp_out;         /* act 1: GELU'(z) of the pre-activation z [M][ldo], or NULL */
-    bf16 *out_bf;         /* [M][ldo], or NULL */
-    bf16 *out_bfT;        /* [N][ldt], or NULL */
-    float *out_f;         /* [M][ldo], or NULL */
-    int atomic;           /* out_f += (split K) instead of = */
-    float *colsum;        /* [N] += column sums of the BF16-rounded result, or NULL */
+    int ldo;              /* row stride of out_f */
+    const float *bias;    /* [N] */
+    float *out_f;
+    int atomic;           /* EPI_F32: += (split K) instead of = */
+    float *colsum;        /* [N] += column sums of the BF16-rounded result */
+    const float *const *target;   /* EPI_MSE: device word holding the target's address ([batch][ldo]) */
+    float *loss;          /* EPI_MSE: += the batch's mean squared error */
+    int batch;
     int *err;             /* bit 0: a bounded wait gave up */
     int hold_done;        /* test hook: the completion barrier is never signalled, so the
                              epilogue's bounded wait runs out (CUOPO_ETIMEOUT path) */
 };
 
-__device__ __forceinline__ void store_bf16x32(bf16 *dst, const float (&v)[32])
+/* 32 columns from `col` of row `row` of a 128 x 128 BF16 tile in shared
+ * memory: two 64-column halves, rows of 128 bytes, the 16-byte pieces of a
+ * row permuted as the TMA's 128-byte swizzle does. */
+__device__ __forceinline__ uint4 *tile_piece(uint8_t *tile, int row, int col, int q)
+{
+    const int piece = ((col & 63) >> 3) + q;
+    return reinterpret_cast<uint4 *>(tile + (col >> 6) * (BM * 128) + row * 128 + ((piece ^ (row & 7)) << 4));
+}
+
+__device__ __forceinline__ void put_bf16x32(uint8_t *tile, int row, int col, const float (&v)[32])
 {
 #pragma unroll
     for (int q = 0; q < 4; q++) {
-        uint4 u;
         uint32_t w[4];
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             __nv_bfloat162 h = __floats2bfloat162_rn(v[8 * q + 2 * j], v[8 * q + 2 * j + 1]);
             w[j] = *reinterpret_cast<uint32_t *>(&h);
         }
-        u.x = w[0]; u.y = w[1]; u.z = w[2]; u.w = w[3];
-        reinterpret_cast<uint4 *>(dst)[q] = u;
+        *tile_piece(tile, row, col, q) = make_uint4(w[0], w[1], w[2], w[3]);
     }
 }
 
-__device__ __forceinline__ void load_bf16x32(const bf16 *src, float (&v)[32])
+__device__ __forceinline__ void get_bf16x32(uint8_t *tile, int row, int col, float (&v)[32])
 {
 #pragma unroll
     for (int q = 0; q < 4; q++) {
-        const uint4 u = reinterpret_cast<const uint4 *>(src)[q];
+        const uint4 u = *tile_piece(tile, row, col, q);
         const uint32_t w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
         for (int j = 0; j < 4; j++) {
@@ -263,89 +298,136 @@ __device__ __forceinline__ void load_bf16x32(const bf16 *src, float (&v)[32])
     }
 }
 
-/* Row `row`, columns col..col+31 of the tile; lane = this thread's lane. */
-__device__ __forceinline__ void epilogue32(const Epi &ep, int row, int col, float (&v)[32], int lane, bool store)
+/* Sum over the warp's lanes of column j, on lane j: the lanes exchange halves
+ * of what is left (31 shuffles for 32 columns; a tree per column takes 160). */
+__device__ __forceinline__ float column_sums(float (&v)[32], int lane)
 {
-    if (ep.bias) {
 #pragma unroll
-        for (int j = 0; j < 32; j++) v[j] += __ldg(ep.bias + col + j);
+    for (int d = 16; d > 0; d >>= 1) {
+        const bool up = (lane & d) != 0;
+#pragma unroll
+        for (int j = 0; j < d; j++) {
+            const float give = up ? v[j] : v[j + d], keep = up ? v[j + d] : v[j];
+            v[j] = keep + __shfl_xor_sync(0xffffffffu, give, d);
+        }
     }
-    const size_t o = (size_t)row * ep.ldo + col;
-    if (ep.act == 1) {
+    return v[0];
+}
+
+/* Row `row` (of the tile; m0 + row of the matrix), columns n0 + col .. + 31. */
+template <int MODE>
+__device__ __forceinline__ void epilogue32(const Epi &ep, int m0, int row, int n0, int col, float (&v)[32], int lane,
+                                           uint8_t *tile0, uint8_t *tile1, float &loss)
+{
+    if constexpr (MODE == EPI_GELU || MODE == EPI_GELU_T || MODE == EPI_Y || MODE == EPI_MSE) {
+        const float4 *b = reinterpret_cast<const float4 *>(ep.bias + n0 + col);
+#pragma unroll
+        for (int q = 0; q < 8; q++) {
+            const float4 w = __ldg(b + q);
+            v[4 * q] += w.x;
+            v[4 * q + 1] += w.y;
+            v[4 * q + 2] += w.z;
+            v[4 * q + 3] += w.w;
+        }
+    }
+    if constexpr (MODE == EPI_GELU || MODE == EPI_GELU_T) {
         float gp[32];
 #pragma unroll
         for (int j = 0; j < 32; j++) gelu_and_grad(v[j], v[j], gp[j]);
-        if (ep.gp_out && store) store_bf16x32(ep.gp_out + o, gp);
-    } else if (ep.act == 2) {
-        float gp[32];
-        load_bf16x32(ep.gp_in + o, gp);
-#pragma unroll
-        for (int j = 0; j < 32; j++) v[j] *= gp[j];
+        put_bf16x32(tile0, row, col, v);
+        if constexpr (MODE == EPI_GELU_T) put_bf16x32(tile1, row, col, gp);
     }
-    if (ep.out_f && store) {
-        float4 *d = reinterpret_cast<float4 *>(ep.out_f + o);
-        if (ep.atomic) {
+    if constexpr (MODE == EPI_MSE) {
+        const float scale = 2.0f / ((float)ep.batch * (float)ep.ldo);
+        if (m0 + row < ep.batch) {
+            const float *t = *ep.target + (size_t)(m0 + row) * ep.ldo + n0 + col;
+            if (((uintptr_t)t & 15) == 0) {
 #pragma unroll
-            for (int q = 0; q < 8; q++) {
-                atomicAdd(&d[q].x, v[4 * q]);
-                atomicAdd(&d[q].y, v[4 * q + 1]);
-                atomicAdd(&d[q].z, v[4 * q + 2]);
-                atomicAdd(&d[q].w, v[4 * q + 3]);
+                for (int q = 0; q < 8; q++) {
+                    const float4 w = reinterpret_cast<const float4 *>(t)[q];
+                    v[4 * q] -= w.x;
+                    v[4 * q + 1] -= w.y;
+                    v[4 * q + 2] -= w.z;
+                    v[4 * q + 3] -= w.w;
+                }
+            } else {
+#pragma unroll
+                for (int j = 0; j < 32; j++) v[j] -= t[j];
             }
         } else {
 #pragma unroll
-            for (int q = 0; q < 8; q++) d[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+            for (int j = 0; j < 32; j++) v[j] = 0.f;
         }
-    }
-    if (ep.out_bf || ep.out_bfT || ep.colsum) {
-#pragma unroll
-        for (int j = 0; j < 32; j++) v[j] = __bfloat162float(__float2bfloat16_rn(v[j]));
-    }
-    if (ep.out_bf && store) store_bf16x32(ep.out_bf + o, v);
-    if (ep.out_bfT && store) {
-#pragma unroll
-        for (int j = 0; j < 32; j++) ep.out_bfT[(size_t)(col + j) * ep.ldt + row] = __float2bfloat16_rn(v[j]);
-    }
-    if (ep.colsum) {
 #pragma unroll
         for (int j = 0; j < 32; j++) {
-            float s = v[j];
+            loss += v[j] * v[j];
+            v[j] *= scale;
+        }
+    }
+    if constexpr (MODE == EPI_DX) {
+        float gp[32];
+        get_bf16x32(tile1, row, col, gp);
 #pragma unroll
-            for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
-            if (lane == 0 && store) atomicAdd(ep.colsum + col + j, s);
+        for (int j = 0; j < 32; j++) v[j] *= gp[j];
+    }
+    if constexpr (MODE == EPI_MSE || MODE == EPI_DX) {
+#pragma unroll
+        for (int j = 0; j < 32; j++) v[j] = __bfloat162float(__float2bfloat16_rn(v[j]));
+        put_bf16x32(tile0, row, col, v);
+        atomicAdd(ep.colsum + n0 + col + lane, column_sums(v, lane));
+    }
+    if constexpr (MODE == EPI_F32 || MODE == EPI_DW || MODE == EPI_Y) {
+        if (MODE != EPI_Y || m0 + row < ep.batch) {
+            float4 *d = reinterpret_cast<float4 *>(ep.out_f + (size_t)(m0 + row) * ep.ldo + n0 + col);
+            const bool atomic = MODE == EPI_DW || (MODE == EPI_F32 && ep.atomic);
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                const float4 w = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+                if (atomic) atomicAdd(d + q, w);
+                else d[q] = w;
+            }
         }
     }
 }
 
-template <int BN>
-constexpr size_t gemm_smem_bytes()
+constexpr uint32_t OPERAND_BYTES = BM * BK * 2;                 /* one operand's stage: 128 x 64 BF16 */
+constexpr size_t GEMM_TILES = (size_t)STAGES * 2 * OPERAND_BYTES; /* the epilogue's two tiles behind the stages */
+constexpr size_t GEMM_SMEM = 1024 + GEMM_TILES + 2 * (BM * 128 * 2) + (2 * STAGES + 2) * 8 + 16;
+
+/* One operand's stage: the 64 K elements of block kb of its 128 (or 64) rows
+ * from mn0, as boxes of 64 x 64. */
+__device__ __forceinline__ void load_operand(uint8_t *dst, const CUtensorMap *map, bool mn_major, int mn0, int mn, int kb,
+                                             uint64_t *bar)
 {
-    return 1024 + (size_t)STAGES * (BM * BK * 2 + BN * BK * 2) + (2 * STAGES + 1) * 8 + 16;
+    for (int i = 0; i < mn / 64; i++)
+        tma_load_2d(dst + i * 8192, map, mn_major ? mn0 + 64 * i : kb * BK, mn_major ? kb * BK : mn0 + 64 * i, bar);
 }
 
 /*
- * C tile (blockIdx.x, blockIdx.y) over the K slice blockIdx.z * kb_per ..
- * (+kb_per) blocks of 64.  512 threads: thread 0 issues the TMA loads,
- * thread 32 the MMAs; after the last MMA every warp runs the epilogue of
- * one 32 x 32 block of the tile.
+ * The C tile at (m0, n0), 128 rows x bn (64 or 128) columns, over K blocks
+ * kb0 .. kb0 + kb_per.  512 threads: thread 0 issues the TMA loads, thread 32
+ * the MMAs; after the last MMA every warp runs the epilogue of one 32 x 32
+ * block of the tile.  tmO0 / tmO1: where tile 0 (and tile 1) go; EPI_DX reads
+ * tile 1 through tmO1 instead.
  */
-template <int BN>
-__global__ void __launch_bounds__(NTHREADS, 1)
-    tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const Epi ep,
-                   int kb_per)
+template <int MODE, bool A_MN, bool B_MN>
+__device__ __forceinline__ void gemm_tile(const CUtensorMap *tmA, const CUtensorMap *tmB, const CUtensorMap *tmO0,
+                                          const CUtensorMap *tmO1, const Epi &ep, int m0, int n0, int bn, int kb0,
+                                          int kb_per)
 {
-    static_assert(BN == 64 || BN == 128, "tile width: one 32-column chunk per warp and quadrant");
     extern __shared__ uint8_t smem_dyn[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_dyn + 1023) & ~(uintptr_t)1023);
-    constexpr uint32_t A_BYTES = BM * BK * 2, B_BYTES = BN * BK * 2;
     uint8_t *sA = smem;
-    uint8_t *sB = smem + STAGES * A_BYTES;
-    uint64_t *full = (uint64_t *)(sB + STAGES * B_BYTES);
+    uint8_t *sB = smem + STAGES * OPERAND_BYTES;
+    uint8_t *tile0 = smem + GEMM_TILES, *tile1 = tile0 + BM * 128 * 2;
+    uint64_t *full = (uint64_t *)(tile1 + BM * 128 * 2);
     uint64_t *empty = full + STAGES;
     uint64_t *done = empty + STAGES;
-    uint32_t *slot = (uint32_t *)(done + 1);
+    uint64_t *extra = done + 1;
+    uint32_t *slot = (uint32_t *)(extra + 1);
+    __shared__ int s_err;
+    __shared__ float s_loss[NTHREADS / 32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN, kb0 = blockIdx.z * kb_per;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; s++) {
@@ -353,9 +435,11 @@ __global__ void __launch_bounds__(NTHREADS, 1)
             mbar_init(empty + s, 1);
         }
         mbar_init(done, 1);
+        mbar_init(extra, 1);
+        s_err = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 0) tmem_alloc(slot, BN);
+    if (warp == 0) tmem_alloc(slot, 128);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -365,22 +449,26 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     griddep_wait();
     griddep_launch();
 
-    __shared__ int s_err;
-    if (threadIdx.x == 0) s_err = 0;
-    __syncthreads();
     if (threadIdx.x == 0) {
+        const uint32_t bytes = OPERAND_BYTES + (uint32_t)bn * BK * 2;
         for (int kb = 0; kb < kb_per; kb++) {
             const int s = kb % STAGES;
             if (kb >= STAGES && !mbar_wait(empty + s, ((kb / STAGES) & 1) ^ 1)) {
                 atomicOr(&s_err, 1);
                 break;
             }
-            mbar_expect_tx(full + s, A_BYTES + B_BYTES);
-            tma_load_2d(sA + s * A_BYTES, &tmA, (kb0 + kb) * BK, m0, full + s);
-            tma_load_2d(sB + s * B_BYTES, &tmB, (kb0 + kb) * BK, n0, full + s);
+            mbar_expect_tx(full + s, bytes);
+            load_operand(sA + s * OPERAND_BYTES, tmA, A_MN, m0, BM, kb0 + kb, full + s);
+            load_operand(sB + s * OPERAND_BYTES, tmB, B_MN, n0, bn, kb0 + kb, full + s);
+            if (MODE == EPI_DX && kb == min(STAGES, kb_per) - 1) {
+                /* the derivative tile, behind the first operands */
+                mbar_expect_tx(extra, BM * 128 * 2);
+                for (int i = 0; i < 4; i++)
+                    tma_load_2d(tile1 + i * 8192, tmO1, n0 + 64 * (i >> 1), m0 + 64 * (i & 1), extra);
+            }
         }
     } else if (threadIdx.x == 32) {
-        constexpr uint32_t idesc = idesc_bf16<BN>();
+        const uint32_t idesc = idesc_bf16(bn, A_MN, B_MN);
         for (int kb = 0; kb < kb_per; kb++) {
             const int s = kb % STAGES;
             if (!mbar_wait(full + s, (kb / STAGES) & 1)) {
@@ -388,32 +476,92 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                 break;
             }
             tc_fence_after();
-            const uint32_t a0 = smem_u32(sA + s * A_BYTES), b0 = smem_u32(sB + s * B_BYTES);
+            const uint32_t a0 = smem_u32(sA + s * OPERAND_BYTES), b0 = smem_u32(sB + s * OPERAND_BYTES);
 #pragma unroll
-            for (int k = 0; k < BK / 16; k++)
-                umma_bf16(tmem, sw128_desc(a0 + 32 * k), sw128_desc(b0 + 32 * k), idesc, (kb | k) != 0);
+            for (int k = 0; k < BK / 16; k++)   /* 16 K: 32 bytes of every row, or 16 rows */
+                umma_bf16(tmem, A_MN ? sw128_desc_mn(a0 + 2048 * k) : sw128_desc(a0 + 32 * k),
+                          B_MN ? sw128_desc_mn(b0 + 2048 * k) : sw128_desc(b0 + 32 * k), idesc, (kb | k) != 0);
             umma_commit(empty + s);   /* frees the stage once these MMAs have read it */
         }
         if (!ep.hold_done) umma_commit(done);   /* arrives when every MMA above has completed */
     }
     __syncwarp();
     if (!mbar_wait(done, 0)) atomicOr(&s_err, 1);
+    if (MODE == EPI_DX && !mbar_wait(extra, 0)) atomicOr(&s_err, 1);
     /* every role loop and every wait above has ended (all are bounded) */
     __syncthreads();
     tc_fence_after();
     const bool store = s_err == 0;
+    float loss = 0.f;
     /* warp w reads TMEM lane quadrant w % 4 (the lanes it may access) and
      * column chunk w / 4 of 32 */
     const int quad = warp & 3, chunk = warp >> 2;
-    if (chunk < BN / 32) {
+    if (chunk < bn / 32 && store) {
         float v[32];
         tmem_ld32(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(chunk * 32), v);
-        epilogue32(ep, m0 + quad * 32 + lane, n0 + chunk * 32, v, lane, store);
+        epilogue32<MODE>(ep, m0, quad * 32 + lane, n0, chunk * 32, v, lane, tile0, tile1, loss);
+    }
+    if constexpr (MODE == EPI_MSE) {
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, d);
+        if (lane == 0) s_loss[warp] = loss;
     }
     if (!store && threadIdx.x == 0 && ep.err) atomicOr(ep.err, 1);
     tc_fence_before();
+    constexpr bool TILES = MODE == EPI_GELU || MODE == EPI_GELU_T || MODE == EPI_MSE || MODE == EPI_DX;
+    if constexpr (TILES) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
-    if (warp == 0) tmem_dealloc(tmem, BN);
+    if (warp == 0) tmem_dealloc(tmem, 128);
+    if (threadIdx.x == 0 && store) {
+        if constexpr (MODE == EPI_MSE) {
+            float s = 0.f;
+            for (int w = 0; w < NTHREADS / 32; w++) s += s_loss[w];
+            atomicAdd(ep.loss, s / ((float)ep.batch * (float)ep.ldo));
+        }
+        if constexpr (TILES) {
+            for (int i = 0; i < 4; i++) {
+                tma_store_2d(tmO0, n0 + 64 * (i >> 1), m0 + 64 * (i & 1), tile0 + i * 8192);
+                if (MODE == EPI_GELU_T) tma_store_2d(tmO1, n0 + 64 * (i >> 1), m0 + 64 * (i & 1), tile1 + i * 8192);
+            }
+            asm volatile("cp.async.bulk.commit_group;\n\tcp.async.bulk.wait_group 0;" ::: "memory");
+        }
+    }
+}
+
+/* One product: tile (blockIdx.x, blockIdx.y), K slice blockIdx.z. */
+template <int MODE, bool B_MN>
+__global__ void __launch_bounds__(NTHREADS, 1)
+    tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                   const __grid_constant__ CUtensorMap tmO0, const __grid_constant__ CUtensorMap tmO1, const Epi ep,
+                   int bn, int kb_per)
+{
+    gemm_tile<MODE, false, B_MN>(&tmA, &tmB, &tmO0, &tmO1, ep, blockIdx.x * BM, blockIdx.y * bn, bn,
+                                 blockIdx.z * kb_per, kb_per);
+}
+
+/* Weight gradients of every layer, dW_l = g_l^T act_{l-1}: blockIdx.x runs over
+ * the tiles of all layers, blockIdx.y over slices of the batch. */
+constexpr int MAX_LAYERS = 11;
+struct DwArgs {
+    CUtensorMap g[MAX_LAYERS], act[MAX_LAYERS];
+    float *out[MAX_LAYERS];
+    int kp[MAX_LAYERS];           /* columns of dW_l (padded inputs): 64 or a multiple of 128 */
+    int first[MAX_LAYERS + 1];    /* first tile of layer l */
+    int layers, kb_per;
+    int *err;
+};
+
+__global__ void __launch_bounds__(NTHREADS, 1) tc_dw_kernel(const __grid_constant__ DwArgs a)
+{
+    int l = 0;
+    while (l + 1 < a.layers && (int)blockIdx.x >= a.first[l + 1]) l++;
+    const int bn = a.kp[l] % 128 == 0 ? 128 : 64, cols = a.kp[l] / bn, tile = (int)blockIdx.x - a.first[l];
+    Epi ep{};
+    ep.ldo = a.kp[l];
+    ep.out_f = a.out[l];
+    ep.err = a.err;
+    gemm_tile<EPI_DW, true, true>(&a.g[l], &a.act[l], nullptr, nullptr, ep, tile / cols * BM, tile % cols * bn, bn,
+                                  blockIdx.y * a.kb_per, a.kb_per);
 }
 
 /* ------------------------------------------------------- host: TMA maps */
@@ -435,17 +583,17 @@ encode_tiled_fn encoder()
     return fn;
 }
 
-/* Row-major BF16 matrix [rows][cols] read in boxes of 64 columns x box_rows
- * rows with the 128-byte swizzle. */
-cuopo_status encode_bf16(CUtensorMap *m, const void *base, long rows, long cols, int box_rows)
+/* Row-major BF16 matrix [rows][cols] in boxes of 64 columns x 64 rows with
+ * the 128-byte swizzle. */
+cuopo_status encode_bf16(CUtensorMap *m, const void *base, long rows, long cols)
 {
     encode_tiled_fn enc = encoder();
     if (!enc) return cuopo_fail(CUOPO_ECUDA, "mlp: cuTensorMapEncodeTiled unavailable");
-    if (((uintptr_t)base & 15) || (cols * 2) % 16 || cols % 64 || rows % box_rows)
+    if (((uintptr_t)base & 15) || (cols * 2) % 16 || cols % 64 || rows % 64)
         return cuopo_fail(CUOPO_EINVAL, "mlp: matrix not aligned for TMA (16-byte base, 64-column multiples)");
     cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
     cuuint64_t strides[1] = {(cuuint64_t)cols * 2};
-    cuuint32_t box[2] = {64, (cuuint32_t)box_rows};
+    cuuint32_t box[2] = {64, 64};
     cuuint32_t es[2] = {1, 1};
     CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(base), dims, strides, box, es,
                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -480,24 +628,18 @@ cudaError_t launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t sme
     return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 
-template <int BN>
-cudaError_t launch_gemm_bn(const CUtensorMap &a, const CUtensorMap &b, const Epi &ep, int M, int N, int K, int split,
-                           cudaStream_t st)
+/* C = A B^T (B_MN: B stored [K][N]) with tile width bn (64 or 128); K split
+ * into `split` slices.  o0 / o1: the maps of the tiles that MODE writes (reads). */
+template <int MODE, bool B_MN>
+cudaError_t launch_gemm(const CUtensorMap &a, const CUtensorMap &b, const CUtensorMap &o0, const CUtensorMap &o1,
+                        const Epi &ep, int M, int N, int K, int bn, int split, cudaStream_t st)
 {
     cudaError_t attr = prepare_gemm();
     if (attr != cudaSuccess) return attr;
-    dim3 grid((unsigned)(M / BM), (unsigned)(N / BN), (unsigned)split);
-    cudaError_t e = launch_k(tc_gemm_kernel<BN>, grid, dim3(NTHREADS), gemm_smem_bytes<BN>(), st, a, b, ep,
+    dim3 grid((unsigned)(M / BM), (unsigned)(N / bn), (unsigned)split);
+    cudaError_t e = launch_k(tc_gemm_kernel<MODE, B_MN>, grid, dim3(NTHREADS), GEMM_SMEM, st, a, b, o0, o1, ep, bn,
                              (K / BK) / split);
     return e != cudaSuccess ? e : cudaGetLastError();
-}
-
-/* C = A B^T with tile width bn (64 or 128); K split into `split` slices. */
-cudaError_t launch_gemm(const CUtensorMap &a, const CUtensorMap &b, const Epi &ep, int M, int N, int K, int bn,
-                        int split, cudaStream_t st)
-{
-    return bn == 64 ? launch_gemm_bn<64>(a, b, ep, M, N, K, split, st)
-                    : launch_gemm_bn<128>(a, b, ep, M, N, K, split, st);
 }
 
 /* The largest split of K (in blocks of 64, dividing them) that keeps
@@ -513,16 +655,23 @@ int pick_split(int tiles, int kblocks)
     return best;
 }
 
-/* Shared-memory opt-in of both tile widths, outside any stream capture. */
+/* Shared-memory opt-in of every kernel, outside any stream capture. */
+template <typename K>
+cudaError_t opt_in(K *kernel)
+{
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM);
+}
+
 cudaError_t prepare_gemm()
 {
     static cudaError_t st = [] {
-        cudaError_t e = cudaFuncSetAttribute(tc_gemm_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)gemm_smem_bytes<64>());
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(tc_gemm_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)gemm_smem_bytes<128>());
-        return e;
+        cudaError_t r = cudaSuccess;
+        for (cudaError_t e : {opt_in(tc_gemm_kernel<EPI_F32, false>), opt_in(tc_gemm_kernel<EPI_GELU, false>),
+                              opt_in(tc_gemm_kernel<EPI_GELU_T, false>), opt_in(tc_gemm_kernel<EPI_Y, false>),
+                              opt_in(tc_gemm_kernel<EPI_MSE, false>), opt_in(tc_gemm_kernel<EPI_DX, true>),
+                              opt_in(tc_dw_kernel)})
+            if (r == cudaSuccess) r = e;
+        return r;
     }();
     return st;
 }
@@ -546,16 +695,18 @@ cuopo_status cuda_err(cudaError_t e, const char *what)
 /* ------------------------------------------------------- small kernels */
 
 /* Training/inference input: x [batch][n_in] FP32 -> xin [rows][64] BF16
- * (zero padded in both directions) and, when xinT != NULL, xin^T [64][ldt];
- * target t [batch][n_out] -> tgt (rows >= batch zero) when t != NULL.
- * Thread (0,0) also advances the Adam step and forms its scalars. */
+ * (zero padded in both directions).  A training step also clears the
+ * gradients and the loss, leaves the target's address where the captured
+ * kernels find it and, with `step`, advances the Adam step and forms its
+ * scalars. */
 struct PackArgs {
     const float *x;
     const float *t;
+    const float **target;
     bf16 *xin;
-    bf16 *xinT;
-    float *tgt;
-    int batch, rows, n_in, n_out, ldt;
+    float4 *zero;
+    long zeros;       /* float4 values to clear */
+    int batch, rows, n_in;
     int *step;
     float *adam;      /* [lr, 1 - beta1^t, 1 - beta2^t] */
     float lr, beta1, beta2;
@@ -563,18 +714,13 @@ struct PackArgs {
 
 __global__ void pack_kernel(const PackArgs a)
 {
-    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < (long)a.rows * 64) {
-        const int r = (int)(i / 64), c = (int)(i % 64);
-        const float v = (r < a.batch && c < a.n_in) ? a.x[(size_t)r * a.n_in + c] : 0.f;
-        const bf16 b = __float2bfloat16_rn(v);
-        a.xin[i] = b;
-        if (a.xinT) a.xinT[(size_t)c * a.ldt + r] = b;
+    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x, n = (long)gridDim.x * blockDim.x;
+    for (long j = i; j < (long)a.rows * 64; j += n) {
+        const int r = (int)(j / 64), c = (int)(j % 64);
+        a.xin[j] = __float2bfloat16_rn((r < a.batch && c < a.n_in) ? a.x[(size_t)r * a.n_in + c] : 0.f);
     }
-    if (a.t && i < (long)a.rows * a.n_out) {
-        const int r = (int)(i / a.n_out);
-        a.tgt[i] = r < a.batch ? a.t[i] : 0.f;
-    }
+    for (long j = i; j < a.zeros; j += n) a.zero[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (i == 0 && a.target) *a.target = a.t;
     if (i == 0 && a.step) {
         const int t = ++*a.step;
         a.adam[0] = a.lr;
@@ -583,62 +729,12 @@ __global__ void pack_kernel(const PackArgs a)
     }
 }
 
-/* Mean squared error over batch x n_out and its gradient 2 (y - t) / (batch
- * n_out) (zero on rows >= batch), stored as g [rows][n_out] and g^T
- * [n_out][ldt] (BF16); bias gradient += column sums of the BF16 g; loss +=
- * the batch's mean.  Block: n_out threads x MSE_ROWS rows (each thread
- * writes its column's MSE_ROWS values of g^T as 16-byte stores). */
-constexpr int MSE_ROWS = 16;
-__global__ void mse_kernel(const float *y, const float *tgt, bf16 *g, bf16 *gT, float *db, float *loss, int batch,
-                           int n_out, int ldt)
-{
-    griddep_wait();
-    griddep_launch();
-    const int j = threadIdx.x, r0 = blockIdx.x * MSE_ROWS;
-    const float scale = 2.0f / ((float)batch * (float)n_out);
-    float csum = 0.f, lsum = 0.f;
-    uint32_t packed[MSE_ROWS / 2];
-#pragma unroll
-    for (int q = 0; q < MSE_ROWS; q += 2) {
-        float gv[2];
-#pragma unroll
-        for (int u = 0; u < 2; u++) {
-            const int r = r0 + q + u;
-            const size_t o = (size_t)r * n_out + j;
-            float d = 0.f;
-            if (r < batch) d = y[o] - tgt[o];
-            lsum += d * d;
-            const bf16 b = __float2bfloat16_rn(d * scale);
-            g[o] = b;
-            gv[u] = __bfloat162float(b);
-            csum += gv[u];
-        }
-        __nv_bfloat162 h = __floats2bfloat162_rn(gv[0], gv[1]);
-        packed[q / 2] = *reinterpret_cast<uint32_t *>(&h);
-    }
-    uint4 *dst = reinterpret_cast<uint4 *>(gT + (size_t)j * ldt + r0);
-#pragma unroll
-    for (int q = 0; q < MSE_ROWS / 8; q++)
-        dst[q] = make_uint4(packed[4 * q], packed[4 * q + 1], packed[4 * q + 2], packed[4 * q + 3]);
-    atomicAdd(db + j, csum);
-    __shared__ float part[32];
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, d);
-    if ((j & 31) == 0) part[j >> 5] = lsum;
-    __syncthreads();
-    if (j == 0) {
-        float s = 0.f;
-        for (int w = 0; w < (n_out + 31) / 32; w++) s += part[w];
-        atomicAdd(loss, s / ((float)batch * (float)n_out));
-    }
-}
-
 /* Parameter segments of the flat FP32 buffer: weights [N][Kp] (with a BF16
- * copy and its transpose) or biases [N]. */
+ * copy) or biases [N]. */
 struct Seg {
     long off, len;
     int N, Kp;          /* Kp = 0 for a bias */
-    bf16 *w, *wT;
+    bf16 *w;
 };
 constexpr int MAX_SEG = 24;
 struct AdamArgs {
@@ -651,44 +747,42 @@ struct AdamArgs {
     Seg seg[MAX_SEG];
 };
 
+/* Four parameters per thread (every segment starts and ends on a multiple of
+ * 64): 33 MB through L2 as 16-byte accesses. */
 __global__ void adam_kernel(const AdamArgs a, long total)
 {
     griddep_wait();
     griddep_launch();
-    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long i = 4 * ((long)blockIdx.x * blockDim.x + threadIdx.x);
     if (i >= total) return;
-    float p = a.p[i];
+    const float4 p4 = *reinterpret_cast<const float4 *>(a.p + i);
+    float p[4] = {p4.x, p4.y, p4.z, p4.w};
     if (a.update) {
-        const float g = a.g[i] * a.gscale;
-        const float m = a.beta1 * a.m[i] + (1.0f - a.beta1) * g;
-        const float v = a.beta2 * a.v[i] + (1.0f - a.beta2) * g * g;
-        a.m[i] = m;
-        a.v[i] = v;
-        const float mh = m / a.adam[1], vh = v / a.adam[2];
-        p -= a.adam[0] * mh / (sqrtf(vh) + a.eps);
-        a.p[i] = p;
+        const float4 g4 = *reinterpret_cast<const float4 *>(a.g + i);
+        const float4 m4 = *reinterpret_cast<const float4 *>(a.m + i);
+        const float4 v4 = *reinterpret_cast<const float4 *>(a.v + i);
+        const float gr[4] = {g4.x, g4.y, g4.z, g4.w};
+        float m[4] = {m4.x, m4.y, m4.z, m4.w}, v[4] = {v4.x, v4.y, v4.z, v4.w};
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const float g = gr[j] * a.gscale;
+            m[j] = a.beta1 * m[j] + (1.0f - a.beta1) * g;
+            v[j] = a.beta2 * v[j] + (1.0f - a.beta2) * g * g;
+            const float mh = m[j] / a.adam[1], vh = v[j] / a.adam[2];
+            p[j] -= a.adam[0] * mh / (sqrtf(vh) + a.eps);
+        }
+        *reinterpret_cast<float4 *>(a.m + i) = make_float4(m[0], m[1], m[2], m[3]);
+        *reinterpret_cast<float4 *>(a.v + i) = make_float4(v[0], v[1], v[2], v[3]);
+        *reinterpret_cast<float4 *>(a.p + i) = make_float4(p[0], p[1], p[2], p[3]);
     }
     int s = 0;
     while (s + 1 < a.nseg && i >= a.seg[s + 1].off) s++;
     const Seg &sg = a.seg[s];
-    if (sg.Kp > 0) sg.w[i - sg.off] = __float2bfloat16_rn(p);
-}
-
-/* W^T [Kp][N] from W [N][Kp] (BF16) through 32 x 32 shared-memory tiles, so
- * that both the reads and the writes are coalesced; blockIdx.z = weight
- * segment (a.seg[2 l]). */
-__global__ void transpose_weights_kernel(const AdamArgs a)
-{
-    griddep_wait();
-    griddep_launch();
-    __shared__ bf16 tile[32][33];
-    const Seg &sg = a.seg[2 * blockIdx.z];
-    const int n0 = blockIdx.y * 32, k0 = blockIdx.x * 32;
-    if (n0 >= sg.N || k0 >= sg.Kp) return;
-    const int tx = threadIdx.x, ty = threadIdx.y;   /* 32 x 8 */
-    for (int r = ty; r < 32; r += 8) tile[r][tx] = sg.w[(size_t)(n0 + r) * sg.Kp + k0 + tx];
-    __syncthreads();
-    for (int r = ty; r < 32; r += 8) sg.wT[(size_t)(k0 + r) * sg.N + n0 + tx] = tile[tx][r];
+    if (sg.Kp > 0) {
+        const __nv_bfloat162 lo = __floats2bfloat162_rn(p[0], p[1]), hi = __floats2bfloat162_rn(p[2], p[3]);
+        *reinterpret_cast<uint2 *>(sg.w + (i - sg.off)) = make_uint2(*reinterpret_cast<const uint32_t *>(&lo),
+                                                                     *reinterpret_cast<const uint32_t *>(&hi));
+    }
 }
 
 }  /* namespace */
@@ -701,14 +795,15 @@ struct cuopo_mlp {
     std::vector<int> N, K, Kp;                        /* per layer: outputs, inputs, padded inputs */
     std::vector<long> w_off, b_off;                   /* flat offsets (internal, padded layer 0) */
     long P;                                           /* internal parameter count */
-    float *params, *grads, *m, *v, *adam, *loss, *y, *tgt;
+    float *params, *grads, *m, *v, *adam, *loss, *y;   /* loss: the word after the gradients */
+    const float **target;                             /* device word: the current target's address */
     int *err, *step;
-    bf16 *xin, *xinT;
-    std::vector<bf16 *> w_bf, wT_bf;                  /* per layer [N][Kp], [Kp][N] */
-    std::vector<bf16 *> gp, h, hT, g, gT;             /* per hidden layer [rows][width] / [width][rows];
-                                                         gp = GELU'(z) */
-    bf16 *g_out, *g_outT;
-    std::vector<CUtensorMap> mA_fwd, mB_fwd, mA_dW, mB_dW, mA_dX, mB_dX;
+    bf16 *xin;
+    std::vector<bf16 *> w_bf;                         /* per layer [N][Kp] */
+    std::vector<bf16 *> gp, h, g;                     /* per hidden layer [rows][width]; gp = GELU'(z) */
+    bf16 *g_out;
+    CUtensorMap m_xin, m_gout;
+    std::vector<CUtensorMap> m_w, m_h, m_gp, m_g;
     std::vector<void *> allocs;
     AdamArgs adam_args;
     cudaGraphExec_t graph;        /* forward, loss, backward, Adam */
@@ -732,88 +827,78 @@ cuopo_status dalloc(cuopo_mlp *m, T **p, size_t count)
     return CUOPO_OK;
 }
 
-/* The activation feeding layer l (row-major and transposed). */
-bf16 *act_in(cuopo_mlp *m, int l) { return l == 0 ? m->xin : m->h[l - 1]; }
-bf16 *act_inT(cuopo_mlp *m, int l) { return l == 0 ? m->xinT : m->hT[l - 1]; }
-
 cuopo_status launch_check(cudaError_t e, const char *what)
 {
     return e == cudaSuccess ? CUOPO_OK : cuda_err(e, what);
 }
 
-/* Forward pass over `rows_used` rows (a multiple of 128).  train: keep z, h^T. */
-cuopo_status forward(cuopo_mlp *m, int rows_used, bool train, cudaStream_t st)
+/* The map of the activation feeding layer l, and of layer l's gradient. */
+const CUtensorMap &act_map(const cuopo_mlp *m, int l) { return l == 0 ? m->m_xin : m->m_h[(size_t)(l - 1)]; }
+const CUtensorMap &grad_map(const cuopo_mlp *m, int l) { return l == m->L - 1 ? m->m_gout : m->m_g[(size_t)l]; }
+
+/* Forward pass over `rows_used` rows (a multiple of 128).  train: keeps
+ * GELU'(z), and the output layer forms the loss and its gradient; otherwise
+ * its first `batch` rows go to y. */
+cuopo_status forward(cuopo_mlp *m, int batch, int rows_used, bool train, float *y, cudaStream_t st)
 {
     for (int l = 0; l < m->L; l++) {
         Epi ep = epi_none(m->N[l], m->err);
         ep.bias = m->params + m->b_off[l];
-        ep.ldt = m->rows;
+        ep.batch = batch;
+        const CUtensorMap &a = act_map(m, l), &w = m->m_w[l];
+        cudaError_t e;
         if (l < m->L - 1) {
-            ep.act = 1;
-            ep.out_bf = m->h[l];
-            if (train) {
-                ep.gp_out = m->gp[l];
-                ep.out_bfT = m->hT[l];
-            }
+            const CUtensorMap &h = m->m_h[l], &gp = m->m_gp[l];
+            e = train ? launch_gemm<EPI_GELU_T, false>(a, w, h, gp, ep, rows_used, m->N[l], m->Kp[l], 128, 1, st)
+                      : launch_gemm<EPI_GELU, false>(a, w, h, h, ep, rows_used, m->N[l], m->Kp[l], 128, 1, st);
+        } else if (train) {
+            ep.target = m->target;
+            ep.loss = m->loss;
+            ep.colsum = m->grads + m->b_off[l];
+            e = launch_gemm<EPI_MSE, false>(a, w, m->m_gout, m->m_gout, ep, rows_used, m->N[l], m->Kp[l], 128, 1, st);
         } else {
-            ep.out_f = m->y;
+            ep.out_f = y;
+            e = launch_gemm<EPI_Y, false>(a, w, a, a, ep, rows_used, m->N[l], m->Kp[l], 128, 1, st);
         }
-        cuopo_status s = launch_check(launch_gemm(m->mA_fwd[l], m->mB_fwd[l], ep, rows_used, m->N[l], m->Kp[l], 128, 1,
-                                                  st),
-                                      "mlp forward GEMM");
+        cuopo_status s = launch_check(e, "mlp forward GEMM");
         if (s != CUOPO_OK) return s;
     }
     return CUOPO_OK;
 }
 
-cuopo_status zero_grads(cuopo_mlp *m, cudaStream_t st)
+/* Gradients (into m->grads, cleared by pack) over rows_used rows from the
+ * output layer's, which the forward pass has left. */
+cuopo_status backward(cuopo_mlp *m, int rows_used, cudaStream_t st)
 {
-    cudaError_t e = cudaMemsetAsync(m->grads, 0, sizeof(float) * m->P, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(m->loss, 0, sizeof(float), st);
-    return e != cudaSuccess ? cuda_err(e, "mlp: memset") : CUOPO_OK;
-}
-
-/* Loss, gradients (into m->grads) over rows_used rows; `zero`: clear the
- * gradient and loss accumulators first (a captured step clears them before
- * its forward pass, so that its kernels follow one another directly). */
-cuopo_status backward(cuopo_mlp *m, int batch, int rows_used, cudaStream_t st, bool zero = true)
-{
-    cudaError_t e;
-    if (zero) {
-        cuopo_status z = zero_grads(m, st);
-        if (z != CUOPO_OK) return z;
-    }
-    const int Lo = m->L - 1;
-    e = launch_k(mse_kernel, dim3((unsigned)(rows_used / MSE_ROWS)), dim3((unsigned)m->n_out), 0, st,
-                 (const float *)m->y, (const float *)m->tgt, m->g_out, m->g_outT, m->grads + m->b_off[Lo], m->loss,
-                 batch, m->n_out, m->rows);
-    if (e != cudaSuccess || (e = cudaGetLastError()) != cudaSuccess) return cuda_err(e, "mlp: loss kernel");
-    for (int l = Lo; l >= 0; l--) {
-        /* dW_l = g_l^T act_{l-1}: M = N_l, N = Kp_l, K = rows_used */
-        Epi ew = epi_none(m->Kp[l], m->err);
-        ew.out_f = m->grads + m->w_off[l];
-        ew.atomic = 1;
-        const int bn = (m->Kp[l] % 128 == 0) ? 128 : 64;
-        const int tiles = (m->N[l] / BM) * (m->Kp[l] / bn);
-        const int split = pick_split(tiles, rows_used / BK);
-        cuopo_status s = launch_check(launch_gemm(m->mA_dW[l], m->mB_dW[l], ew, m->N[l], m->Kp[l], rows_used, bn,
-                                                  split, st),
-                                      "mlp dW GEMM");
-        if (s != CUOPO_OK) return s;
-        if (l == 0) break;
+    for (int l = m->L - 1; l > 0; l--) {
         /* g_{l-1} = (g_l W_l) * GELU'(z_{l-1}): M = rows_used, N = Kp_l (= width), K = N_l */
         Epi ex = epi_none(m->Kp[l], m->err);
-        ex.ldt = m->rows;
-        ex.act = 2;
-        ex.gp_in = m->gp[l - 1];
-        ex.out_bf = m->g[l - 1];
-        ex.out_bfT = m->gT[l - 1];
         ex.colsum = m->grads + m->b_off[l - 1];
-        s = launch_check(launch_gemm(m->mA_dX[l], m->mB_dX[l], ex, rows_used, m->Kp[l], m->N[l], 128, 1, st),
-                         "mlp dX GEMM");
+        cuopo_status s = launch_check(launch_gemm<EPI_DX, true>(grad_map(m, l), m->m_w[l], m->m_g[l - 1],
+                                                                m->m_gp[l - 1], ex, rows_used, m->Kp[l], m->N[l], 128,
+                                                                1, st),
+                                      "mlp dX GEMM");
         if (s != CUOPO_OK) return s;
     }
-    return CUOPO_OK;
+    /* dW_l = g_l^T act_{l-1} of every layer: M = N_l, N = Kp_l, K = rows_used */
+    DwArgs d;
+    std::memset(&d, 0, sizeof(d));
+    d.layers = m->L;
+    d.err = m->err;
+    int tiles = 0;
+    for (int l = 0; l < m->L; l++) {
+        d.g[l] = grad_map(m, l);
+        d.act[l] = act_map(m, l);
+        d.out[l] = m->grads + m->w_off[l];
+        d.kp[l] = m->Kp[l];
+        d.first[l] = tiles;
+        tiles += (m->N[l] / BM) * (m->Kp[l] / (m->Kp[l] % 128 == 0 ? 128 : 64));
+    }
+    d.first[m->L] = tiles;
+    const int split = pick_split(tiles, rows_used / BK);
+    d.kb_per = rows_used / BK / split;
+    cudaError_t e = launch_k(tc_dw_kernel, dim3((unsigned)tiles, (unsigned)split), dim3(NTHREADS), GEMM_SMEM, st, d);
+    return launch_check(e != cudaSuccess ? e : cudaGetLastError(), "mlp dW GEMM");
 }
 
 cuopo_status run_adam(cuopo_mlp *m, int update, cudaStream_t st, float gscale = 1.0f)
@@ -822,17 +907,8 @@ cuopo_status run_adam(cuopo_mlp *m, int update, cudaStream_t st, float gscale = 
     a.update = update;
     a.gscale = gscale;
     const int tpb = 256;
-    cudaError_t e = launch_k(adam_kernel, dim3((unsigned)((m->P + tpb - 1) / tpb)), dim3(tpb), 0, st, a, m->P);
-    cuopo_status s = launch_check(e != cudaSuccess ? e : cudaGetLastError(), "mlp: adam kernel");
-    if (s != CUOPO_OK) return s;
-    int maxN = 0, maxK = 0;
-    for (int l = 0; l < m->L; l++) {
-        maxN = m->N[l] > maxN ? m->N[l] : maxN;
-        maxK = m->Kp[l] > maxK ? m->Kp[l] : maxK;
-    }
-    e = launch_k(transpose_weights_kernel, dim3((unsigned)(maxK / 32), (unsigned)(maxN / 32), (unsigned)m->L),
-                 dim3(32, 8), 0, st, a);
-    return launch_check(e != cudaSuccess ? e : cudaGetLastError(), "mlp: weight transpose kernel");
+    cudaError_t e = launch_k(adam_kernel, dim3((unsigned)((m->P / 4 + tpb - 1) / tpb)), dim3(tpb), 0, st, a, m->P);
+    return launch_check(e != cudaSuccess ? e : cudaGetLastError(), "mlp: adam kernel");
 }
 
 cuopo_status pack(cuopo_mlp *m, const float *x, const float *t, int batch, int rows_used, bool train, float lr,
@@ -841,21 +917,22 @@ cuopo_status pack(cuopo_mlp *m, const float *x, const float *t, int batch, int r
     PackArgs a;
     std::memset(&a, 0, sizeof(a));
     a.x = x;
-    a.t = t;
     a.xin = m->xin;
-    a.xinT = train ? m->xinT : nullptr;
-    a.tgt = m->tgt;
+    if (train) {
+        a.t = t;
+        a.target = m->target;
+        a.zero = reinterpret_cast<float4 *>(m->grads);
+        a.zeros = m->P / 4 + 1;   /* and the loss behind them */
+    }
     a.batch = batch;
     a.rows = rows_used;
     a.n_in = m->n_in;
-    a.n_out = m->n_out;
-    a.ldt = m->rows;
     a.step = (train && lr > 0) ? m->step : nullptr;
     a.adam = m->adam;
     a.lr = lr;
     a.beta1 = 0.9f;
     a.beta2 = 0.999f;
-    const long n = (long)rows_used * (m->n_out > 64 ? m->n_out : 64);
+    const long n = (long)rows_used * 64 > a.zeros ? (long)rows_used * 64 : a.zeros;
     pack_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(a);
     return launch_check(cudaGetLastError(), "mlp: pack kernel");
 }
@@ -918,54 +995,39 @@ extern "C" cuopo_status cuopo_mlp_create(cuopo_mlp **out, int n_in, int width, i
     };
     cuopo_status s;
     const size_t R = (size_t)m->rows;
-    if ((s = dalloc(m, &m->params, m->P)) || (s = dalloc(m, &m->grads, m->P)) || (s = dalloc(m, &m->m, m->P)) ||
-        (s = dalloc(m, &m->v, m->P)) || (s = dalloc(m, &m->adam, 4)) || (s = dalloc(m, &m->loss, 1)) ||
-        (s = dalloc(m, &m->y, R * n_out)) || (s = dalloc(m, &m->tgt, R * n_out)) || (s = dalloc(m, &m->err, 1)) ||
-        (s = dalloc(m, &m->step, 1)) || (s = dalloc(m, &m->xin, R * 64)) || (s = dalloc(m, &m->xinT, R * 64)) ||
-        (s = dalloc(m, &m->g_out, R * n_out)) || (s = dalloc(m, &m->g_outT, R * n_out)))
+    if ((s = dalloc(m, &m->params, m->P)) || (s = dalloc(m, &m->grads, m->P + 4)) || (s = dalloc(m, &m->m, m->P)) ||
+        (s = dalloc(m, &m->v, m->P)) || (s = dalloc(m, &m->adam, 4)) || (s = dalloc(m, &m->y, R * n_out)) ||
+        (s = dalloc(m, &m->target, 1)) || (s = dalloc(m, &m->err, 1)) || (s = dalloc(m, &m->step, 1)) ||
+        (s = dalloc(m, &m->xin, R * 64)) || (s = dalloc(m, &m->g_out, R * n_out)))
         return fail(s);
+    m->loss = m->grads + m->P;
     m->w_bf.resize(m->L);
-    m->wT_bf.resize(m->L);
+    m->m_w.resize(m->L);
     for (int l = 0; l < m->L; l++)
         if ((s = dalloc(m, &m->w_bf[l], (size_t)m->N[l] * m->Kp[l])) ||
-            (s = dalloc(m, &m->wT_bf[l], (size_t)m->N[l] * m->Kp[l])))
+            (s = encode_bf16(&m->m_w[l], m->w_bf[l], m->N[l], m->Kp[l])))
             return fail(s);
     m->gp.resize(depth);
     m->h.resize(depth);
-    m->hT.resize(depth);
     m->g.resize(depth);
-    m->gT.resize(depth);
+    m->m_gp.resize(depth);
+    m->m_h.resize(depth);
+    m->m_g.resize(depth);
     for (int l = 0; l < depth; l++)
         if ((s = dalloc(m, &m->gp[l], R * width)) || (s = dalloc(m, &m->h[l], R * width)) ||
-            (s = dalloc(m, &m->hT[l], R * width)) || (s = dalloc(m, &m->g[l], R * width)) ||
-            (s = dalloc(m, &m->gT[l], R * width)))
+            (s = dalloc(m, &m->g[l], R * width)) || (s = encode_bf16(&m->m_gp[l], m->gp[l], m->rows, width)) ||
+            (s = encode_bf16(&m->m_h[l], m->h[l], m->rows, width)) ||
+            (s = encode_bf16(&m->m_g[l], m->g[l], m->rows, width)))
             return fail(s);
+    if ((s = encode_bf16(&m->m_xin, m->xin, m->rows, 64)) || (s = encode_bf16(&m->m_gout, m->g_out, m->rows, n_out)))
+        return fail(s);
     cudaError_t e = cudaMemset(m->m, 0, sizeof(float) * m->P);
     if (e == cudaSuccess) e = cudaMemset(m->v, 0, sizeof(float) * m->P);
     if (e == cudaSuccess) e = cudaMemset(m->err, 0, sizeof(int));
     if (e == cudaSuccess) e = cudaMemset(m->step, 0, sizeof(int));
     if (e == cudaSuccess) e = cudaMemset(m->xin, 0, sizeof(bf16) * R * 64);
-    if (e == cudaSuccess) e = cudaMemset(m->xinT, 0, sizeof(bf16) * R * 64);
     if (e != cudaSuccess) return fail(cuda_err(e, "mlp_create: memset"));
 
-    /* tensor maps (every activation buffer has m->rows rows) */
-    m->mA_fwd.resize(m->L);
-    m->mB_fwd.resize(m->L);
-    m->mA_dW.resize(m->L);
-    m->mB_dW.resize(m->L);
-    m->mA_dX.resize(m->L);
-    m->mB_dX.resize(m->L);
-    for (int l = 0; l < m->L; l++) {
-        const int last = l == m->L - 1;
-        if ((s = encode_bf16(&m->mA_fwd[l], act_in(m, l), m->rows, m->Kp[l], BM)) ||
-            (s = encode_bf16(&m->mB_fwd[l], m->w_bf[l], m->N[l], m->Kp[l], 128)) ||
-            (s = encode_bf16(&m->mA_dW[l], last ? m->g_outT : m->gT[l], m->N[l], m->rows, BM)) ||
-            (s = encode_bf16(&m->mB_dW[l], act_inT(m, l), m->Kp[l], m->rows, m->Kp[l] % 128 == 0 ? 128 : 64)))
-            return fail(s);
-        if (l > 0 && ((s = encode_bf16(&m->mA_dX[l], last ? m->g_out : m->g[l], m->rows, m->N[l], BM)) ||
-                      (s = encode_bf16(&m->mB_dX[l], m->wT_bf[l], m->Kp[l], m->N[l], 128))))
-            return fail(s);
-    }
     /* Adam segments */
     AdamArgs &a = m->adam_args;
     std::memset(&a, 0, sizeof(a));
@@ -980,8 +1042,8 @@ extern "C" cuopo_status cuopo_mlp_create(cuopo_mlp **out, int n_in, int width, i
     a.gscale = 1.0f;
     a.nseg = 2 * m->L;
     for (int l = 0; l < m->L; l++) {
-        a.seg[2 * l] = Seg{m->w_off[l], (long)m->N[l] * m->Kp[l], m->N[l], m->Kp[l], m->w_bf[l], m->wT_bf[l]};
-        a.seg[2 * l + 1] = Seg{m->b_off[l], m->N[l], m->N[l], 0, nullptr, nullptr};
+        a.seg[2 * l] = Seg{m->w_off[l], (long)m->N[l] * m->Kp[l], m->N[l], m->Kp[l], m->w_bf[l]};
+        a.seg[2 * l + 1] = Seg{m->b_off[l], m->N[l], m->N[l], 0, nullptr};
     }
     /* initial weights: uniform(-sqrt(6/fan_in), +sqrt(6/fan_in)), zero biases (splitmix64 stream of seed) */
     std::vector<float> host((size_t)m->P, 0.f);
@@ -1074,9 +1136,13 @@ extern "C" cuopo_status cuopo_mlp_forward(cuopo_mlp *m, const float *x, float *y
     if (batch < 1 || batch > m->max_batch) return cuopo_fail(CUOPO_EINVAL, "mlp_forward: batch outside [1, max_batch]");
     cudaStream_t st = (cudaStream_t)stream;
     const int rows = round128(batch);
+    /* the output layer writes y itself where its 16-byte stores may */
+    float *out = ((uintptr_t)y & 15) ? m->y : y;
     cuopo_status s = pack(m, x, nullptr, batch, rows, false, 0.f, st);
-    if (s == CUOPO_OK) s = forward(m, rows, false, st);
-    if (s != CUOPO_OK) return s;
+    g_pdl = 2; /* every kernel from here on waits for the one before it */
+    if (s == CUOPO_OK) s = forward(m, batch, rows, false, out, st);
+    g_pdl = 0;
+    if (s != CUOPO_OK || out == y) return s;
     cudaError_t e = cudaMemcpyAsync(y, m->y, sizeof(float) * (size_t)batch * m->n_out, cudaMemcpyDeviceToDevice, st);
     return e == cudaSuccess ? CUOPO_OK : cuda_err(e, "mlp_forward: copy out");
 }
@@ -1090,8 +1156,8 @@ extern "C" cuopo_status cuopo_mlp_gradients(cuopo_mlp *m, const float *x, const 
     cudaStream_t st = (cudaStream_t)stream;
     const int rows = round128(batch);
     cuopo_status s = pack(m, x, t, batch, rows, true, 0.f, st);
-    if (s == CUOPO_OK) s = forward(m, rows, true, st);
-    if (s == CUOPO_OK) s = backward(m, batch, rows, st);
+    if (s == CUOPO_OK) s = forward(m, batch, rows, true, nullptr, st);
+    if (s == CUOPO_OK) s = backward(m, rows, st);
     if (s != CUOPO_OK) return s;
     cudaError_t e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return cuda_err(e, "mlp_gradients");
@@ -1136,10 +1202,9 @@ cuopo_status capture_step(cuopo_mlp *m, int batch, int rows, cudaStream_t st, bo
         if (own) cudaStreamDestroy(cap);
         return cuda_err(e, "mlp: begin capture");
     }
-    cuopo_status s = zero_grads(m, cap);
     g_pdl = 1;
-    if (s == CUOPO_OK) s = forward(m, rows, true, cap);
-    if (s == CUOPO_OK) s = backward(m, batch, rows, cap, false);
+    cuopo_status s = forward(m, batch, rows, true, nullptr, cap);
+    if (s == CUOPO_OK) s = backward(m, rows, cap);
     if (s == CUOPO_OK && with_adam) s = run_adam(m, 1, cap);
     g_pdl = 0;
     e = cudaStreamEndCapture(cap, &g);
@@ -1251,8 +1316,8 @@ extern "C" cuopo_status cuopo_gemm_bf16(const void *A, const void *B, float *C, 
     cudaError_t pe = prepare_gemm();
     if (pe != cudaSuccess) return cuda_err(pe, "gemm_bf16: kernel attributes");
     CUtensorMap ma, mb;
-    cuopo_status s = encode_bf16(&ma, A, M, K, BM);
-    if (s == CUOPO_OK) s = encode_bf16(&mb, B, N, K, bn);
+    cuopo_status s = encode_bf16(&ma, A, M, K);
+    if (s == CUOPO_OK) s = encode_bf16(&mb, B, N, K);
     if (s != CUOPO_OK) return s;
     Epi ep = epi_none(N, err_dev);
     ep.out_f = C;
@@ -1263,7 +1328,7 @@ extern "C" cuopo_status cuopo_gemm_bf16(const void *A, const void *B, float *C, 
         cudaError_t e = cudaMemsetAsync(C, 0, sizeof(float) * (size_t)M * N, st);
         if (e != cudaSuccess) return cuda_err(e, "gemm_bf16: memset");
     }
-    return launch_check(launch_gemm(ma, mb, ep, M, N, K, bn, split, st), "gemm_bf16");
+    return launch_check(launch_gemm<EPI_F32, false>(ma, mb, ma, ma, ep, M, N, K, bn, split, st), "gemm_bf16");
 }
 
 /* ============================================ warm-start fields <-> modes */
