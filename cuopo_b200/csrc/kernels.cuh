@@ -13,16 +13,21 @@
 
 namespace cuopo {
 
-typedef cudaError_t (*launch_fn)(const LaunchArgs &, int clusters, cudaStream_t);
+typedef cudaError_t (*launch_fn)(const LaunchArgs &, int clusters, bool spread, cudaStream_t);
 typedef int (*occ_fn)(void);
 
-/* Launches of one kernel: CLUSTER CTAs per instance, THREADS per CTA. */
+/* Dynamic shared memory that keeps any two CTAs off one SM (227 KB each). */
+constexpr size_t SPREAD_SMEM = 116 * 1024;
+
+/* Launches of one kernel: CLUSTER CTAs per instance, THREADS per CTA.
+ * spread: one CTA per SM. */
 template <void (*KERNEL)(LaunchArgs), int CLUSTER, int THREADS, size_t SMEM>
 struct Launcher {
     static cudaError_t prepare()
     {
         static cudaError_t st = [] {
-            cudaError_t e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
+            cudaError_t e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 (int)(SMEM > SPREAD_SMEM ? SMEM : SPREAD_SMEM));
             if (e == cudaSuccess && CLUSTER > 8)
                 e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
             return e;
@@ -47,12 +52,13 @@ struct Launcher {
         return cfg;
     }
 
-    static cudaError_t launch(const LaunchArgs &a, int clusters, cudaStream_t st)
+    static cudaError_t launch(const LaunchArgs &a, int clusters, bool spread, cudaStream_t st)
     {
         cudaError_t e = prepare();
         if (e != cudaSuccess) return e;
         cudaLaunchAttribute attr[1];
         cudaLaunchConfig_t cfg = config(clusters, st, attr);
+        if (spread && SMEM < SPREAD_SMEM) cfg.dynamicSmemBytes = SPREAD_SMEM;
         e = cudaLaunchKernelEx(&cfg, KERNEL, a);
         if (e != cudaSuccess) return e;
         return cudaGetLastError();

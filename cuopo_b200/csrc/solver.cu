@@ -106,6 +106,13 @@ static const KernelEntry *find_kernel(int precision, int F, int N, bool single_c
     return found;
 }
 
+/* Clusters of k that are resident with one CTA per SM. */
+static int one_per_sm(const KernelEntry &k)
+{
+    const int occ = k.occ(), per_sm = (occ * k.ctas + 147) / 148;
+    return per_sm > 1 ? occ / per_sm : occ;
+}
+
 /* Measured time per slice of `count` instances on kernel k: its resident
  * clusters work through them in waves. */
 static double slice_time(const KernelEntry &k, int count)
@@ -113,33 +120,89 @@ static double slice_time(const KernelEntry &k, int count)
     const int occ = k.occ();
     if (occ < 1 || k.us1 <= 0) return 1e30;
     const int waves = count / occ, rest = count % occ;
-    return waves * (double)k.us_full + (rest == 0 ? 0.0 : rest * k.ctas <= 148 ? (double)k.us1 : (double)k.us_full);
+    return waves * (double)k.us_full +
+           (rest == 0 ? 0.0 : rest <= one_per_sm(k) ? (double)k.us1 : (double)k.us_full);
 }
 
-/* The layout of k's arithmetic (same M and CL: the same results bit for bit)
- * that runs `count` instances fastest.  A 2^12-point instance, for example,
- * takes 11.1 us per slice on one CTA and 3.1 spread over 16, but only 14 of
- * those clusters are resident against 296 CTAs, so between 15 and 33
- * instances 4 CTAs each are best (4.2 us), then 2 each (7.1) up to 74, then
- * one.  A kernel chosen by hand (cuopo_kernel_select) keeps its M and CL; one
- * that the autotuner is timing runs as it is. */
-static const KernelEntry *pick_layout(const KernelEntry *k, int count)
+/* Every layout of k's arithmetic (same M and CL: the same results bit for
+ * bit), k first.  A kernel chosen by hand (cuopo_kernel_select) keeps its M
+ * and CL; one that the autotuner is timing runs as it is. */
+static std::vector<const KernelEntry *> layouts(const KernelEntry *k)
 {
     static const KernelList *const lists[] = {&wide_f32_2eq, &wide_f32_3eq, &wide_f64_2eq, &wide_f64_3eq};
-    if (!k || k == g_force || k->home == 2) return k;
-    const KernelEntry *best = k;
-    double t = slice_time(*k, count);
+    std::vector<const KernelEntry *> v{k};
+    if (!k || k == g_force || k->us1 <= 0) return v;
     for (const KernelList *l : lists)
         for (int i = 0; i < l->n; i++) {
             const KernelEntry &w = l->k[i];
-            if (w.precision != k->precision || w.F != k->F || w.M != k->M || w.CL != k->CL) continue;
-            const double tw = slice_time(w, count);
-            if (tw < t) {
-                best = &w;
-                t = tw;
-            }
+            if (w.precision == k->precision && w.F == k->F && w.M == k->M && w.CL == k->CL && w.occ() > 0)
+                v.push_back(&w);
         }
+    return v;
+}
+
+/* The layout that runs `count` instances, alone on the chip, fastest.  A
+ * 2^12-point instance, for example, takes 11.1 us per slice on one CTA and
+ * 3.1 spread over 16, but only 14 of those clusters are resident against 296
+ * CTAs, so between 15 and 33 instances 4 CTAs each are best (4.2 us), then 2
+ * each (7.1) up to 74, then one.  packed: only the layouts of the fewest CTAs
+ * per instance (a chip that is full anyway). */
+static const KernelEntry *pick_layout(const KernelEntry *k, int count, bool packed = false)
+{
+    const KernelEntry *best = k;
+    double t = 0;
+    for (const KernelEntry *w : layouts(k)) {
+        if (!w || (packed && w->wide)) continue;
+        const double tw = slice_time(*w, count);
+        if (w == k || tw < t) {
+            best = w;
+            t = tw;
+        }
+    }
     return best;
+}
+
+/* The layouts of groups that share the chip (k: their kernels, n: instances).
+ * Together they finish with the slowest: while the SMs that the layouts take
+ * leave room, the slowest group gets a faster one, and the groups are launched
+ * one CTA per SM (side by side, kernels of two CTAs per SM pair up on some
+ * SMs and leave others idle: 16 instances of 2^12..2^15 took 20 us per slice
+ * that way against 17).  Where even the base kernels fill the chip every group
+ * keeps the one of the least SM time. */
+static std::vector<const KernelEntry *> share_chip(const std::vector<const KernelEntry *> &k,
+                                                   const std::vector<int> &n, bool &spread)
+{
+    spread = false;
+    if (k.size() == 1) return {pick_layout(k[0], n[0])};
+    /* share of the chip that n instances take, one CTA per SM */
+    auto share = [](const KernelEntry *e, int count) {
+        const int occ = one_per_sm(*e);
+        return occ < 1 ? 1e9 : (double)count / occ;
+    };
+    std::vector<const KernelEntry *> pick = k;
+    double used = 0, ctas = 0;
+    for (size_t g = 0; g < k.size(); g++) {
+        used += share(k[g], n[g]);
+        ctas += (double)n[g] * k[g]->ctas;
+    }
+    if (used > 1.0) {
+        for (size_t g = 0; g < k.size(); g++) pick[g] = pick_layout(k[g], (int)(ctas / k[g]->ctas), true);
+        return pick;
+    }
+    spread = true;
+    for (;;) {
+        size_t slow = 0;
+        for (size_t g = 1; g < k.size(); g++)
+            if (pick[g]->us1 > pick[slow]->us1) slow = g;
+        const KernelEntry *next = nullptr;
+        for (const KernelEntry *w : layouts(k[slow]))
+            if (w->us1 < pick[slow]->us1 && (!next || share(w, n[slow]) < share(next, n[slow]))) next = w;
+        if (!next) return pick;
+        const double then = used - share(pick[slow], n[slow]) + share(next, n[slow]);
+        if (then > 1.0) return pick;
+        used = then;
+        pick[slow] = next;
+    }
 }
 
 /* Place of frequency q = k2 + CL k1 in the kernel's tables: per CTA in the
@@ -492,9 +555,9 @@ static void cavity_factors(const cuopo_params &p, Instance &I, bool p32 = false)
     I.use_tod_i = (p.tod_i != 0 && p.b3i != 0);
 }
 
-static cuopo_status launch(const KernelEntry *k, const LaunchArgs &a, int clusters, void *stream)
+static cuopo_status launch(const KernelEntry *k, const LaunchArgs &a, int clusters, void *stream, bool spread = false)
 {
-    cudaError_t e = k->fn(a, clusters, (cudaStream_t)stream);
+    cudaError_t e = k->fn(a, clusters, spread, (cudaStream_t)stream);
     if (e != cudaSuccess) return cuda_fail(e, "kernel launch");
     return CUOPO_OK;
 }
@@ -590,6 +653,7 @@ struct cuopo_batch {
     std::vector<uint64_t> seed;
     cuopo_noise_item *d_noise;    /* per instance: place, size and seed of its noise */
     std::vector<size_t> offset;   /* element offset of each instance's fields */
+    bool spread;                  /* several groups that fit one CTA per SM: launched so */
     size_t total;                 /* total signal elements */
     void *d_pump;                 /* pump-field work buffers (n_t per instance) */
     void *d_signal;               /* signal fields, concatenated */
@@ -774,8 +838,15 @@ static cuopo_status batch_build(cuopo_batch **out, const std::vector<cuopo_param
         return x[1] != y[1] ? x[1] > y[1] : x < y;
     });
     b->h_inst.resize((size_t)count);
-    long batch_ctas = 0;
-    for (const cuopo_params &p : prm) batch_ctas += find_kernel(precision, p.n_eqs, p.n_t)->ctas;
+    std::vector<const KernelEntry *> base;
+    std::vector<int> members;
+    for (const std::array<int, 5> &key : keys) {
+        base.push_back(find_kernel(precision, key[0], key[1]));
+        members.push_back(0);
+        for (const cuopo_params &p : prm)
+            members.back() += std::array<int, 5>{p.n_eqs, p.n_t, p.n_z, p.eom_idler, p.regime} == key;
+    }
+    const std::vector<const KernelEntry *> pick = share_chip(base, members, b->spread);
     for (const std::array<int, 5> &key : keys) {
         b->groups.push_back(BatchGroup{});
         BatchGroup &g = b->groups.back();
@@ -784,10 +855,7 @@ static cuopo_status batch_build(cuopo_batch **out, const std::vector<cuopo_param
         g.n_z = key[2];
         g.eom_idler = key[3];
         g.regime = key[4];
-        /* the groups share the chip: as many instances of this group as would
-         * need the CTAs of all of them */
-        const KernelEntry *k = find_kernel(precision, g.F, g.n_t);
-        g.kernel = pick_layout(k, (int)((batch_ctas + k->ctas - 1) / k->ctas));
+        g.kernel = pick[b->groups.size() - 1];
         std::vector<std::vector<double>> pkeys;
         std::vector<int> plan_of;
         for (int i = 0; i < count; i++) {
@@ -1010,7 +1078,7 @@ extern "C" cuopo_status cuopo_batch_step(cuopo_batch *b, int chunk, int max_rt, 
         a.max_rt = max_rt;
         a.tol = tol;
         a.patience = patience;
-        cuopo_status s2 = launch(g.kernel, a, g.grid, g.stream);
+        cuopo_status s2 = launch(g.kernel, a, g.grid, g.stream, b->spread);
         if (s2 != CUOPO_OK) return s2;
         if ((e = cudaEventRecord(g.done, g.stream)) != cudaSuccess) return cuda_fail(e, "batch_step");
     }
@@ -1344,7 +1412,7 @@ extern "C" cuopo_status cuopo_crystal_pass_noalloc(const cuopo_params *p, const 
     a.single.As = As;
     a.single.Ai = Ai;
     a.single.rt_count = 1;
-    e = k->fn(a, 1, st);
+    e = k->fn(a, 1, false, st);
     if (e != cudaSuccess) return cuda_fail(e, "crystal_pass_noalloc: kernel launch");
     return CUOPO_OK;
 }
