@@ -96,13 +96,13 @@ struct KernelEntry {
      &Launcher<&ssfm_kernel<R, F, M, CL, HM, MINB>, CL, M / 16, Ssfm<R, F, M, CL, HM>::smem_bytes()>::occupancy}
 
 /* The same arithmetic (M, CL) spread over P CTAs of NTHR threads, at least
- * MINB on an SM (wide.cuh). */
-#define CUOPO_W(R, PREC, F, M, CL, P, NTHR, MINB, US1, USF)                                                    \
-    {PREC, F, M, CL, 0, P, NTHR, 1, US1, USF, Wide<R, F, M, CL, P, NTHR, MINB>::smem_bytes(),                   \
-     &Launcher<&wide_kernel<R, F, M, CL, P, NTHR, MINB>, P, NTHR,                                               \
-               Wide<R, F, M, CL, P, NTHR, MINB>::smem_bytes()>::launch,                                         \
-     &Launcher<&wide_kernel<R, F, M, CL, P, NTHR, MINB>, P, NTHR,                                               \
-               Wide<R, F, M, CL, P, NTHR, MINB>::smem_bytes()>::occupancy}
+ * MINB on an SM, Q threads per 16-point transform (wide.cuh). */
+#define CUOPO_W(R, PREC, F, M, CL, P, NTHR, MINB, Q, US1, USF)                                                 \
+    {PREC, F, M, CL, 0, P, NTHR, 1, US1, USF, Wide<R, F, M, CL, P, NTHR, MINB, Q>::smem_bytes(),                \
+     &Launcher<&wide_kernel<R, F, M, CL, P, NTHR, MINB, Q>, P, NTHR,                                            \
+               Wide<R, F, M, CL, P, NTHR, MINB, Q>::smem_bytes()>::launch,                                      \
+     &Launcher<&wide_kernel<R, F, M, CL, P, NTHR, MINB, Q>, P, NTHR,                                            \
+               Wide<R, F, M, CL, P, NTHR, MINB, Q>::smem_bytes()>::occupancy}
 
 /* Configurations of one precision and number of equations. */
 struct KernelList {

@@ -558,11 +558,12 @@ struct Ssfm {
 
     /* reg[e] times the GDD/TOD factor of frequency w[e stride] and 1/N
      * (functions.cuh:156-186, formed in FP64). */
-    static __device__ __forceinline__ void gdd_factor(C (&reg)[16], const float *__restrict__ w, int stride, double gdd,
+    template <int NV>
+    static __device__ __forceinline__ void gdd_factor(C (&reg)[NV], const float *__restrict__ w, int stride, double gdd,
                                                       double tod, int use_tod, R s_n)
     {
 #pragma unroll 4
-        for (int e = 0; e < 16; e++) {
+        for (int e = 0; e < NV; e++) {
             const double wk = (double)__ldg(w + e * stride);
             const double ph = use_tod ? 0.5 * wk * rfma(wk, gdd, rmul(wk * wk, tod) / 3.0) : 0.5 * wk * wk * gdd;
             double sn, cs;

@@ -31,9 +31,14 @@
  * thread of the owner reads its part before it sends, and every thread sends
  * to every CTA.
  *
- * Every 16-point transform is one thread's, all fields at once, so a CTA has
- * F CL 16 R0/P transform threads; the element-wise pass uses all NTHR of the
- * CTA.  The chain per slice is what bounds it (six 16-point transforms, two
+ * A CTA has F CL 16 R0/P 16-point transforms of every stage, all fields at
+ * once; Q threads (1 or 4) do one.  With Q = 4 thread q holds the elements
+ * e = q mod 4: the inner 4-point transforms over a are its own, and their
+ * outputs change places within the quad through shared memory (the outer
+ * ones, over b, then leave it the outputs q mod 4).  That is a quarter of the
+ * instructions in each link of the chain: where a CTA has only a warp or two of
+ * transforms (2^13 points or less on 16 CTAs) the others would idle.  The
+ * element-wise pass uses all NTHR threads of the CTA.  The chain per slice is what bounds it (six 16-point transforms, two
  * exchanges, two RK4 half steps), so whatever does not depend on the fields
  * is loaded ahead: the pass's coefficients by the last warp into shared
  * memory before the dispersion step (stage()), the dispersion rows and the
@@ -89,7 +94,56 @@ __device__ __forceinline__ bool mbar_test(unsigned mbar, unsigned parity)
     return ok != 0;
 }
 
-template <typename R, int F, int M, int CL, int P, int NTHR, int MINB>
+/* dft16 by a quad: v[a] = element q + 4a in, output q + 4a out.  scr: the
+ * warp's 128 entries of shared memory; tw: quarter turns and rotation of
+ * W16^{b q}, b = 1..3 (QuadTw). */
+template <typename C>
+struct QuadTw {
+    C rot[3];
+    int m[3];
+    __device__ __forceinline__ void init(int q)
+    {
+        using R = typename real_of<C>::type;
+#pragma unroll
+        for (int b = 1; b < 4; b++) {
+            /* as tw16: n = b q eighths of pi, nearest quarter turn, rest r pi/8 with r = -1..2 */
+            const int n = b * q, k = (n + 1) / 4, r = n - 4 * k;
+            const double t = r == 0 ? 0.0 : r == 2 ? 0.41421356237309504880 : 0.19891236737965800691;
+            const double sn = r == 0 ? 0.0 : r == 2 ? 0.70710678118654752440 : 0.38268343236508977173;
+            rot[b - 1] = mk<C>((R)(r < 0 ? -t : t), (R)(r < 0 ? -sn : sn));
+            m[b - 1] = k;
+        }
+    }
+};
+
+template <int S, bool TW, typename C>
+__device__ __forceinline__ void dft16_quad(C (&v)[4], const StageRot<C> &w, bool hi, const QuadTw<C> &tw, C *scr)
+{
+    using R = typename real_of<C>::type;
+    const R sg = (R)S;
+    if constexpr (TW) {
+        v[1] = shear_rot(v[1], sg * w.a[0].x, sg * w.a[0].y);
+        v[2] = shear_rot(iq<S>(v[2]), sg * w.a[1].x, sg * w.a[1].y);
+        v[3] = shear_rot(iq12<S>(v[3], hi), sg * w.a[2].x, sg * w.a[2].y);
+    }
+    dft4<S>(v[0], v[1], v[2], v[3]);
+    /* 4 x 4 transpose: (q1, b) at 16 quad + ((4 q1 + b) ^ 4 (quad mod 4)) */
+    const int l = threadIdx.x & 31, q = l & 3, base = (l >> 2) * 16, x = (l >> 2) & 3;
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < 4; j++) scr[base + 4 * (j ^ x) + q] = v[j];
+    __syncwarp();
+#pragma unroll
+    for (int b = 0; b < 4; b++) v[b] = scr[base + 4 * (q ^ x) + b];
+#pragma unroll
+    for (int b = 1; b < 4; b++) {
+        v[b] = shear_rot(iq_rt(v[b], (S * tw.m[b - 1]) & 3), sg * tw.rot[b - 1].x, sg * tw.rot[b - 1].y);
+        if constexpr (TW) v[b] = shear_rot(v[b], sg * w.b[b - 1].x, sg * w.b[b - 1].y);
+    }
+    dft4<S>(v[0], v[1], v[2], v[3]);
+}
+
+template <typename R, int F, int M, int CL, int P, int NTHR, int MINB, int Q>
 struct Wide {
     using Math = Ssfm<R, F, M, CL, 0>;
     using C = cpx<R>;
@@ -108,13 +162,73 @@ struct Wide {
     static constexpr bool SPLIT = CL == 16;
     static_assert(SP::P == 3, "radix R0, 16, 16 only");
     static_assert(R0 % P == 0 && P <= 16 && NTHR % 32 == 0 && NT % 16 == 0, "cluster size divides the first radix");
+    static_assert(Q == 1 || (Q == 4 && 4 * NT <= NTHR && F * U <= 15), "quads: one transform each, a named barrier per 256 points");
+    static constexpr int NV = 16 / Q;        /* elements of a thread */
 
     /* stage rotations and dispersion rows kept in registers */
-    static constexpr bool HOLD_TW = sizeof(R) == 4 && NT <= NTHR && NTHR * MINB <= 256;
-    static constexpr bool EARLY_ROWS = NTHR * MINB <= 256;
+    static constexpr bool HOLD_TW = sizeof(R) == 4 && Q * NT <= NTHR && (NTHR * MINB <= 256 || Q == 4);
+    static constexpr bool EARLY_ROWS = NTHR * MINB <= 256 || Q == 4;
 
     static constexpr size_t buf_elems() { return (size_t)F * CL * NP; }
-    static constexpr size_t smem_bytes() { return sizeof(C) * 2 * buf_elems(); }
+    static constexpr size_t smem_bytes() { return sizeof(C) * (2 * buf_elems() + (Q == 4 ? 4 * NTHR : 0)); }
+
+    /* Places in the two buffers: quads read 8 neighbours of 4 elements e at a
+     * time, so every other element is shifted by half of 16 entries (distinct
+     * banks); in the exchange inside a 256-point transform, row and column of
+     * a 16 x 16 matrix. */
+    static __device__ __forceinline__ int tb_at(int e, int t2l) { return e * Tc + (Q == 4 ? t2l ^ (8 * (e & 1)) : t2l); }
+    static __device__ __forceinline__ int fb_at(int j) { return Q == 4 ? j ^ ((j >> 1) & 8) : j; }
+    static __device__ __forceinline__ int xc_at(int row, int col)
+    {
+        return 16 * row + (col ^ row ^ (Q == 4 ? 8 * (row & 1) : 0));
+    }
+
+    /* A 16-point transform, elements and outputs q + Q a of thread q. */
+    template <int S, bool TW>
+    static __device__ __forceinline__ void dft_q(C (&v)[NV], const StageRot<C> &w, bool hi, const QuadTw<C> &qt, C *scr)
+    {
+        if constexpr (Q == 1) dft16<S, TW>(v, w, hi);
+        else dft16_quad<S, TW>(v, w, hi, qt, scr);
+    }
+
+    /* First forward (S = +1) or inverse stage, radix R0: butterflies i < B over
+     * the elements i + B r.  Output j of thread q is output out_r(j, q) of
+     * butterfly out_i(j, q). */
+    template <int S>
+    static __device__ __forceinline__ void first_stage(C (&v)[NV], const QuadTw<C> &qt, C *scr)
+    {
+        if constexpr (Q == 1) {
+            stage_compute<S, M, 0>(v, StageTwiddles<M, C>{});
+        } else if constexpr (R0 == 16) {
+            dft16_quad<S, false>(v, StageRot<C>{}, false, qt, scr);
+        } else if constexpr (R0 == 8) {
+            /* dft8: b = q / 2, over a in the thread, then with the thread of the other b */
+            dft4<S>(v[0], v[1], v[2], v[3]);
+            const bool odd = (threadIdx.x & 2) != 0;
+            C w[4] = {v[0], tw16<S, 2>(v[1]), tw16<S, 4>(v[2]), tw16<S, 6>(v[3])};
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const C mine = odd ? w[k] : v[k];
+                const C other = mk<C>(__shfl_xor_sync(0xffffffffu, mine.x, 2), __shfl_xor_sync(0xffffffffu, mine.y, 2));
+                v[k] = odd ? csub(other, mine) : cadd(mine, other);
+            }
+        } else if constexpr (R0 == 4) {
+            dft4<S>(v[0], v[1], v[2], v[3]);
+        } else {
+            dft2<S>(v[0], v[2]);
+            dft2<S>(v[1], v[3]);
+        }
+    }
+    static __device__ __forceinline__ int out_i(int j, int q)
+    {
+        if (Q == 1) return j % B;
+        return R0 == 16 ? 0 : R0 == 8 ? (q & 1) : R0 == 4 ? q : q + 4 * (j & 1);
+    }
+    static __device__ __forceinline__ int out_r(int j, int q)
+    {
+        if (Q == 1) return j / B;
+        return R0 == 16 ? q + 4 * j : R0 == 8 ? 4 * (q >> 1) + j : R0 == 4 ? j : j >> 1;
+    }
 
     /* One 16-point transform.  Time side: field, cross index, class;
      * frequency side: field, transform (uk2, r), lane.  The field is the same on
@@ -149,6 +263,9 @@ struct Wide {
         typename Math::Stager st;
         unsigned parity;           /* bit 3 b + f: parity of that mbarrier's next phase */
         int tid, rank;
+        int q;                     /* thread of the transform */
+        QuadTw<C> qt;              /* Q == 4 */
+        C *scr;
         StageRot<C> w_t, w_1, w_2, w_3; /* HOLD_TW: this thread's rotations */
 
         __device__ __forceinline__ void init()
@@ -172,8 +289,11 @@ struct Wide {
                     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&s_mbar[tid])) : "memory");
                 asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
             }
+            q = tid % Q;
+            scr = fb + buf_elems() + (tid >> 5) * 128;
+            if constexpr (Q == 4) qt.init(q);
             if constexpr (HOLD_TW) {
-                const Role o(tid, rank);
+                const Role o(tid / Q, rank);
                 w_t = o.rot_t(rank);
                 w_1 = o.rot_1();
                 w_2 = o.rot_2();
@@ -258,10 +378,18 @@ struct Wide {
             st.load(tid - (NTHR - 32), op, tab);
         }
 
-        /* index into the global fields of entry i (position and cross index) of the time side */
+        /* the threads of one 256-point transform */
+        __device__ __forceinline__ void sync_unit(int uu)
+        {
+            if constexpr (Q == 1) __syncwarp(0xFFFFu << (tid & 16));
+            else asm volatile("bar.sync %0, 64;" ::"r"(1 + uu) : "memory");
+        }
+
+        /* index into the global fields of entry pos (cross index c) of the time side */
         __device__ __forceinline__ int point(int pos, int c) const
         {
-            return rank * Tc + pos % Tc + T * (pos / Tc) + M * c;
+            const int e = pos / Tc;
+            return rank * Tc + tb_at(e, pos % Tc) % Tc + T * e + M * c;
         }
 
         __device__ __forceinline__ void load(const Instance &I)
@@ -293,21 +421,21 @@ struct Wide {
             st.write(tid - (NTHR - 32), staged);
             if (in_y) {
 #pragma unroll 1
-                for (int task = tid; task < NT; task += NTHR) {
+                for (int task = tid / Q; task < NT; task += NTHR / Q) {
                     const Role o(task, rank);
                     if (!((in_y >> o.f) & 1u)) continue;
-                    C *const own = tb + (o.f * CL + o.k2) * NP + o.t2l;
+                    C *const own = tb + (o.f * CL + o.k2) * NP;
                     const int t2 = rank * Tc + o.t2l;
                     StageRot<C> w;
                     if constexpr (HOLD_TW) w = w_t;
                     else w = o.rot_t(rank);
-                    C v[16];
+                    C v[NV];
                     wait(0, o.f);
 #pragma unroll
-                    for (int e = 0; e < 16; e++) v[e] = own[e * Tc];
-                    dft16<-1, true>(v, w, 2 * t2 >= T);
+                    for (int a = 0; a < NV; a++) v[a] = own[tb_at(q + Q * a, o.t2l)];
+                    dft_q<-1, true>(v, w, 2 * t2 >= T, qt, scr);
 #pragma unroll
-                    for (int e = 0; e < 16; e++) own[e * Tc] = v[e];
+                    for (int a = 0; a < NV; a++) own[tb_at(q + Q * a, o.t2l)] = v[a];
                 }
                 flip(0, in_y);
             }
@@ -366,20 +494,20 @@ struct Wide {
             __syncthreads();
             if (!out_y) return;
 #pragma unroll 1
-            for (int task = tid; task < NT; task += NTHR) {
+            for (int task = tid / Q; task < NT; task += NTHR / Q) {
                 const Role o(task, rank);
                 if (!((out_y >> o.f) & 1u)) continue;
-                const C *const own = tb + (o.f * CL + o.k2) * NP + o.t2l;
-                C v[16];
+                const C *const own = tb + (o.f * CL + o.k2) * NP;
+                C v[NV];
 #pragma unroll
-                for (int e = 0; e < 16; e++) v[e] = own[e * Tc];
-                first_stage<+1>(v);
+                for (int a = 0; a < NV; a++) v[a] = own[tb_at(q + Q * a, o.t2l)];
+                first_stage<+1>(v, qt, scr);
 #pragma unroll
-                for (int q = 0; q < R0; q++) /* output q of butterfly i: entry t2 + T i of transform (k2, q) */
-#pragma unroll
-                    for (int i = 0; i < B; i++)
-                        put(fb, 3 + o.f, q / RP, (o.f * U + o.k2 * RP + q % RP) * 256 + rank * Tc + o.t2l + T * i,
-                            v[i + q * B]);
+                for (int j = 0; j < NV; j++) { /* output k of butterfly i: entry t2 + T i of transform (k2, k) */
+                    const int i = out_i(j, q), k = out_r(j, q);
+                    put(fb, 3 + o.f, k / RP,
+                        (o.f * U + o.k2 * RP + k % RP) * 256 + fb_at(rank * Tc + o.t2l + T * i), v[j]);
+                }
             }
             if constexpr (P == 1) __syncthreads();
         }
@@ -402,12 +530,6 @@ struct Wide {
             }
         }
 
-        template <int S>
-        static __device__ __forceinline__ void first_stage(C (&v)[16])
-        {
-            stage_compute<S, M, 0>(v, StageTwiddles<M, C>{});
-        }
-
         /* The frequency side of the fields of mask: two forward stages, the
          * factor, two inverse stages, exchange.  MODE as Ssfm::spectral. */
         template <int MODE>
@@ -415,67 +537,62 @@ struct Wide {
         {
             expect(0, mask);
 #pragma unroll 1
-            for (int task = tid; task < NT; task += NTHR) {
+            for (int task = tid / Q; task < NT; task += NTHR / Q) {
                 const Role o(task, rank);
                 if (!((mask >> o.f) & 1u)) continue;
                 const int r = o.r, lane = o.lane, t2p = r + R0 * lane;
-                const unsigned half = 0xFFFFu << (tid & 16); /* the transform's 16 lanes */
                 C *const u = fb + o.uu * 256;
                 /* row entries of frequencies t2p + T e, [k2][r][e][lane] */
-                const int row = ((o.uk2 * R0 + r) * 16) * 16 + lane;
+                const int row = ((o.uk2 * R0 + r) * 16 + q) * 16 + lane;
                 const C *__restrict__ disp = reinterpret_cast<const C *>(tab.disp) + (size_t)o.f * N + row;
-                C v[16], d[EARLY_ROWS ? 16 : 1];
+                C v[NV], d[EARLY_ROWS ? NV : 1];
                 if constexpr (MODE == 0 && EARLY_ROWS) {
 #pragma unroll
-                    for (int e = 0; e < 16; e++) d[e] = ld_now(disp + 16 * e);
+                    for (int a = 0; a < NV; a++) d[a] = ld_now(disp + 16 * Q * a);
                 }
                 wait(1, o.f);
                 /* stage 1 (length R0): butterfly `lane`, k = r */
 #pragma unroll
-                for (int e = 0; e < 16; e++) v[e] = u[lane + 16 * e];
-                if constexpr (HOLD_TW) dft16<+1, true>(v, w_1, 2 * r >= R0);
-                else dft16<+1, true>(v, o.rot_1(), 2 * r >= R0);
-                __syncwarp(half);
+                for (int a = 0; a < NV; a++) v[a] = u[fb_at(lane + 16 * (q + Q * a))];
+                if constexpr (HOLD_TW) dft_q<+1, true>(v, w_1, 2 * r >= R0, qt, scr);
+                else dft_q<+1, true>(v, o.rot_1(), 2 * r >= R0, qt, scr);
+                sync_unit(o.uu);
 #pragma unroll
-                for (int q = 0; q < 16; q++) u[16 * q + (lane ^ q)] = v[q];
-                __syncwarp(half);
+                for (int a = 0; a < NV; a++) u[xc_at(q + Q * a, lane)] = v[a];
+                sync_unit(o.uu);
                 /* stage 2 (length T): butterfly t2p = r + R0 lane; leaves frequencies t2p + T e */
 #pragma unroll
-                for (int e = 0; e < 16; e++) v[e] = u[16 * lane + (e ^ lane)];
-                if constexpr (HOLD_TW) dft16<+1, true>(v, w_2, 2 * t2p >= T);
-                else dft16<+1, true>(v, o.rot_2(), 2 * t2p >= T);
+                for (int a = 0; a < NV; a++) v[a] = u[xc_at(lane, q + Q * a)];
+                if constexpr (HOLD_TW) dft_q<+1, true>(v, w_2, 2 * t2p >= T, qt, scr);
+                else dft_q<+1, true>(v, o.rot_2(), 2 * t2p >= T, qt, scr);
                 const R s_n = (R)tab.inv_n;
                 if constexpr (MODE == 0) {
 #pragma unroll
-                    for (int e = 0; e < 16; e++)
-                        v[e] = caddmul(cscale(v[e], s_n), EARLY_ROWS ? d[e % (EARLY_ROWS ? 16 : 1)]
-                                                                     : __ldg(disp + 16 * e));
+                    for (int a = 0; a < NV; a++)
+                        v[a] = caddmul(cscale(v[a], s_n), EARLY_ROWS ? d[a % (EARLY_ROWS ? NV : 1)]
+                                                                     : __ldg(disp + 16 * Q * a));
                 } else {
-                    Math::gdd_factor(v, tab.w + row, 16, I->gdd, o.f == 1 ? I->tod_s : I->tod_i,
+                    Math::gdd_factor(v, tab.w + row, 16 * Q, I->gdd, o.f == 1 ? I->tod_s : I->tod_i,
                                      o.f == 1 ? I->use_tod_s : I->use_tod_i, s_n);
                 }
                 /* inverse stage 0 (radix R0) on the same registers */
-                first_stage<-1>(v);
-                __syncwarp(half);
+                first_stage<-1>(v, qt, scr);
+                sync_unit(o.uu);
                 /* to butterfly s = q R0 + r0, element e1: (position R0 j + r0, j = t2p + T i = 16 e1 + r + R0 q) */
 #pragma unroll
-                for (int r0 = 0; r0 < R0; r0++)
+                for (int j = 0; j < NV; j++)
+                    u[xc_at(lane / B + R0 * out_i(j, q), (lane % B) * R0 + out_r(j, q))] = v[j];
+                sync_unit(o.uu);
+                const int k = lane % R0, cls = r + R0 * (lane / R0);
 #pragma unroll
-                    for (int i = 0; i < B; i++) {
-                        const int s = (lane % B) * R0 + r0, e1 = lane / B + R0 * i;
-                        u[16 * e1 + (s ^ e1)] = v[i + r0 * B];
-                    }
-                __syncwarp(half);
-                const int k = lane % R0, q = r + R0 * (lane / R0);
+                for (int a = 0; a < NV; a++) v[a] = u[xc_at(q + Q * a, lane)];
+                if constexpr (HOLD_TW) dft_q<-1, true>(v, w_3, 2 * k >= R0, qt, scr);
+                else dft_q<-1, true>(v, o.rot_3(), 2 * k >= R0, qt, scr);
+                /* output m: element cls of class k + R0 m */
 #pragma unroll
-                for (int e = 0; e < 16; e++) v[e] = u[16 * e + (lane ^ e)];
-                if constexpr (HOLD_TW) dft16<-1, true>(v, w_3, 2 * k >= R0);
-                else dft16<-1, true>(v, o.rot_3(), 2 * k >= R0);
-                /* output m: element q of class k + R0 m */
-#pragma unroll
-                for (int m = 0; m < 16; m++) {
-                    const int c = k + R0 * m;
-                    put(tb, o.f, c / Tc, (o.f * CL + o.uk2) * NP + q * Tc + c % Tc, v[m]);
+                for (int a = 0; a < NV; a++) {
+                    const int c = k + R0 * (q + Q * a);
+                    put(tb, o.f, c / Tc, (o.f * CL + o.uk2) * NP + tb_at(cls, c % Tc), v[a]);
                 }
             }
             flip(1, mask);
@@ -503,7 +620,7 @@ struct Wide {
 #pragma unroll
                 for (int j = 0; j < J; j++)
 #pragma unroll
-                    for (int c = 0; c < CL; c++) v += cabs2d(tb[(CL + c) * NP + (rk * J + j) * Tc + t2l]);
+                    for (int c = 0; c < CL; c++) v += cabs2d(tb[(CL + c) * NP + tb_at(rk * J + j, t2l)]);
                 const unsigned half = 0xFFFFu << (tid & 16);
 #pragma unroll
                 for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(half, v, o);
@@ -527,10 +644,10 @@ struct Wide {
     };
 };
 
-template <typename R, int F, int M, int CL, int P, int NTHR, int MINB>
+template <typename R, int F, int M, int CL, int P, int NTHR, int MINB, int Q>
 __global__ void __launch_bounds__(NTHR, MINB) wide_kernel(LaunchArgs a)
 {
-    drive<R, typename Wide<R, F, M, CL, P, NTHR, MINB>::Engine>(a);
+    drive<R, typename Wide<R, F, M, CL, P, NTHR, MINB, Q>::Engine>(a);
 }
 
 }  // namespace cuopo

@@ -6,22 +6,22 @@
 namespace cuopo {
 
 static const KernelEntry k_list[] = {
-    CUOPO_W(float, CUOPO_F32, 3, 512, 1, 1, 128, 1, 2.9, 4.1),
-    CUOPO_W(float, CUOPO_F32, 3, 1024, 1, 1, 256, 1, 3.9, 3.9),
-    CUOPO_W(float, CUOPO_F32, 3, 1024, 1, 4, 128, 1, 3.4, 3.8),
-    CUOPO_W(float, CUOPO_F32, 3, 2048, 1, 1, 384, 1, 7, 7),
-    CUOPO_W(float, CUOPO_F32, 3, 2048, 1, 4, 128, 1, 4, 4.3),
-    CUOPO_W(float, CUOPO_F32, 3, 2048, 1, 8, 128, 1, 3.5, 3.9),
-    CUOPO_W(float, CUOPO_F32, 3, 4096, 1, 2, 384, 1, 9.6, 9.6),
-    CUOPO_W(float, CUOPO_F32, 3, 4096, 1, 4, 256, 1, 4.5, 4.5),
-    CUOPO_W(float, CUOPO_F32, 3, 4096, 1, 16, 128, 1, 3.7, 3.9),
-    CUOPO_W(float, CUOPO_F32, 3, 4096, 2, 4, 384, 1, 9.6, 9.6),
-    CUOPO_W(float, CUOPO_F32, 3, 4096, 2, 8, 256, 1, 5.3, 5.3),
-    CUOPO_W(float, CUOPO_F32, 3, 4096, 2, 16, 256, 1, 3.8, 3.8),
-    CUOPO_W(float, CUOPO_F32, 3, 4096, 4, 8, 384, 1, 11, 11),
-    CUOPO_W(float, CUOPO_F32, 3, 4096, 4, 16, 256, 1, 6, 6),
-    CUOPO_W(float, CUOPO_F32, 3, 4096, 8, 16, 384, 1, 11.4, 11.4),
-    CUOPO_W(float, CUOPO_F32, 3, 4096, 16, 16, 384, 1, 21.6, 21.6),
+    CUOPO_W(float, CUOPO_F32, 3, 512, 1, 1, 128, 1, 1, 2.9, 4.1),
+    CUOPO_W(float, CUOPO_F32, 3, 1024, 1, 1, 256, 1, 1, 3.9, 3.9),
+    CUOPO_W(float, CUOPO_F32, 3, 1024, 1, 4, 192, 1, 4, 3.6, 3.7),
+    CUOPO_W(float, CUOPO_F32, 3, 2048, 1, 1, 384, 1, 1, 7, 7),
+    CUOPO_W(float, CUOPO_F32, 3, 2048, 1, 4, 128, 1, 1, 4, 4.3),
+    CUOPO_W(float, CUOPO_F32, 3, 2048, 1, 8, 192, 1, 4, 3.6, 3.8),
+    CUOPO_W(float, CUOPO_F32, 3, 4096, 1, 2, 384, 1, 1, 9.6, 9.6),
+    CUOPO_W(float, CUOPO_F32, 3, 4096, 1, 4, 256, 1, 1, 4.5, 4.5),
+    CUOPO_W(float, CUOPO_F32, 3, 4096, 1, 16, 128, 1, 1, 3.7, 3.9),
+    CUOPO_W(float, CUOPO_F32, 3, 4096, 2, 4, 384, 1, 1, 9.6, 9.6),
+    CUOPO_W(float, CUOPO_F32, 3, 4096, 2, 8, 256, 1, 1, 5.3, 5.3),
+    CUOPO_W(float, CUOPO_F32, 3, 4096, 2, 16, 256, 1, 1, 3.8, 3.8),
+    CUOPO_W(float, CUOPO_F32, 3, 4096, 4, 8, 384, 1, 1, 11, 11),
+    CUOPO_W(float, CUOPO_F32, 3, 4096, 4, 16, 256, 1, 1, 6, 6),
+    CUOPO_W(float, CUOPO_F32, 3, 4096, 8, 16, 384, 1, 1, 11.4, 11.4),
+    CUOPO_W(float, CUOPO_F32, 3, 4096, 16, 16, 384, 1, 1, 21.6, 21.6),
     /* more instances than fit one CTA per SM: in place, two per SM */
     CUOPO_K(float, CUOPO_F32, 3, 4096, 1, 1, 2, 13.9, 20.5),
     CUOPO_K(float, CUOPO_F32, 3, 4096, 4, 1, 2, 18, 26.7),
