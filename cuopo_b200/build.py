@@ -26,7 +26,7 @@ CC_FLAGS = ["-O2", "-fPIC", "-std=c11", "-Wall", "-Wextra", "-fvisibility=hidden
             "-I" + str(CSRC)]
 
 CU_SOURCES = ["kern_f64_3eq.cu", "kern_f64_2eq.cu", "wide_f64_3eq.cu", "wide_f64_2eq.cu",
-              "wide_f32_3eq.cu", "wide_f32_2eq.cu", "kern_f32_2eq.cu", "kern_f32_3eq.cu", "solver.cu", "noise.cu", "fft_api.cu", "probe.cu", "mlp.cu", "params_dev.cu"]
+              "wide_f32_3eq.cu", "wide_f32_2eq.cu", "kern_f32_2eq.cu", "solo_f32_2eq.cu", "kern_f32_3eq.cu", "solver.cu", "noise.cu", "fft_api.cu", "probe.cu", "mlp.cu", "params_dev.cu"]
 # per-file nvcc flags: the device set-up keeps the host's float rounding (no FMA contraction)
 CU_EXTRA = {"params_dev.cu": ["-fmad=false"]}
 C_SOURCES = ["params.c", "dat_io.c"]

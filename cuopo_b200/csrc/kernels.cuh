@@ -1,6 +1,6 @@
 /*
  * kernels.cuh -- the built kernel configurations: their launch functions and
- * the registry entries.  Each kern_*.cu (ssfm_kernel) and wide_*.cu
+ * the registry entries.  Each kern_*.cu and solo_*.cu (ssfm_kernel) and wide_*.cu
  * (wide_kernel) instantiates the configurations of one precision and number
  * of equations (separate files so that they compile in parallel); solver.cu
  * chooses among them.
@@ -91,9 +91,13 @@ struct KernelEntry {
 };
 
 #define CUOPO_K(R, PREC, F, M, CL, HM, MINB, US1, USF)                                                         \
+    CUOPO_KC(R, PREC, F, M, CL, HM, MINB, field_copies<R>(F), US1, USF)
+#define CUOPO_KC(R, PREC, F, M, CL, HM, MINB, COPIES, US1, USF)                                                \
     {PREC, F, M, CL, HM, CL, M / 16, 0, US1, USF, Ssfm<R, F, M, CL, HM>::smem_bytes(),                          \
-     &Launcher<&ssfm_kernel<R, F, M, CL, HM, MINB>, CL, M / 16, Ssfm<R, F, M, CL, HM>::smem_bytes()>::launch,    \
-     &Launcher<&ssfm_kernel<R, F, M, CL, HM, MINB>, CL, M / 16, Ssfm<R, F, M, CL, HM>::smem_bytes()>::occupancy}
+     &Launcher<&ssfm_kernel<R, F, M, CL, HM, MINB, COPIES>, CL, M / 16,                                         \
+               Ssfm<R, F, M, CL, HM>::smem_bytes()>::launch,                                                    \
+     &Launcher<&ssfm_kernel<R, F, M, CL, HM, MINB, COPIES>, CL, M / 16,                                         \
+               Ssfm<R, F, M, CL, HM>::smem_bytes()>::occupancy}
 
 /* The same arithmetic (M, CL) spread over P CTAs of NTHR threads, at least
  * MINB on an SM, Q threads per 16-point transform (wide.cuh). */
@@ -110,6 +114,7 @@ struct KernelList {
     int n;
 };
 extern const KernelList kern_f32_2eq, kern_f32_3eq, kern_f64_2eq, kern_f64_3eq;
+extern const KernelList solo_f32_2eq;
 extern const KernelList wide_f32_2eq, wide_f32_3eq, wide_f64_2eq, wide_f64_3eq;
 
 }  // namespace cuopo

@@ -129,7 +129,8 @@ static double slice_time(const KernelEntry &k, int count)
  * and CL; one that the autotuner is timing runs as it is. */
 static std::vector<const KernelEntry *> layouts(const KernelEntry *k)
 {
-    static const KernelList *const lists[] = {&wide_f32_2eq, &wide_f32_3eq, &wide_f64_2eq, &wide_f64_3eq};
+    static const KernelList *const lists[] = {&solo_f32_2eq, &wide_f32_2eq, &wide_f32_3eq, &wide_f64_2eq,
+                                              &wide_f64_3eq};
     std::vector<const KernelEntry *> v{k};
     if (!k || k == g_force || k->us1 <= 0) return v;
     for (const KernelList *l : lists)
@@ -145,14 +146,13 @@ static std::vector<const KernelEntry *> layouts(const KernelEntry *k)
  * 2^12-point instance, for example, takes 11.1 us per slice on one CTA and
  * 3.1 spread over 16, but only 14 of those clusters are resident against 296
  * CTAs, so between 15 and 33 instances 4 CTAs each are best (4.2 us), then 2
- * each (7.1) up to 74, then one.  packed: only the layouts of the fewest CTAs
- * per instance (a chip that is full anyway). */
-static const KernelEntry *pick_layout(const KernelEntry *k, int count, bool packed = false)
+ * each (7.1) up to 74, then one. */
+static const KernelEntry *pick_layout(const KernelEntry *k, int count)
 {
     const KernelEntry *best = k;
     double t = 0;
     for (const KernelEntry *w : layouts(k)) {
-        if (!w || (packed && w->wide)) continue;
+        if (!w) continue;
         const double tw = slice_time(*w, count);
         if (w == k || tw < t) {
             best = w;
@@ -162,13 +162,25 @@ static const KernelEntry *pick_layout(const KernelEntry *k, int count, bool pack
     return best;
 }
 
+/* k for launches of at most one CTA per SM (solo_f32_2eq.cu), or k itself. */
+static const KernelEntry *solo(const KernelEntry *k)
+{
+    for (int i = 0; i < solo_f32_2eq.n; i++) {
+        const KernelEntry &s = solo_f32_2eq.k[i];
+        if (s.precision == k->precision && s.F == k->F && s.M == k->M && s.CL == k->CL && !k->wide) return &s;
+    }
+    return k;
+}
+
 /* The layouts of groups that share the chip (k: their kernels, n: instances).
  * Together they finish with the slowest: while the SMs that the layouts take
  * leave room, the slowest group gets a faster one, and the groups are launched
  * one CTA per SM (side by side, kernels of two CTAs per SM pair up on some
  * SMs and leave others idle: 16 instances of 2^12..2^15 took 20 us per slice
  * that way against 17).  Where even the base kernels fill the chip every group
- * keeps the one of the least SM time. */
+ * keeps the one of the least SM time.  With at most one CTA per SM on average
+ * the kernels for that take over: 32 instances of 2^12..2^15 (138 CTAs) 16.6
+ * us per slice against 21.7. */
 static std::vector<const KernelEntry *> share_chip(const std::vector<const KernelEntry *> &k,
                                                    const std::vector<int> &n, bool &spread)
 {
@@ -186,10 +198,12 @@ static std::vector<const KernelEntry *> share_chip(const std::vector<const Kerne
         ctas += (double)n[g] * k[g]->ctas;
     }
     if (used > 1.0) {
-        for (size_t g = 0; g < k.size(); g++) pick[g] = pick_layout(k[g], (int)(ctas / k[g]->ctas), true);
+        if (ctas <= 148)
+            for (const KernelEntry *&p : pick) p = solo(p);
         return pick;
     }
     spread = true;
+    for (const KernelEntry *&p : pick) p = solo(p);
     for (;;) {
         size_t slow = 0;
         for (size_t g = 1; g < k.size(); g++)

@@ -204,8 +204,12 @@ namespace cg = cooperative_groups;
  *      passes, with one shared scratch[M] for the local transforms; for grids
  *      whose fields exceed a cluster's shared memory (3 FP64 fields of 2^17
  *      points are 6 MiB, a 16-CTA cluster has 3.6 MB).  Every access to
- *      the fields goes to L2 (ld/st .cg), ordered by the cluster barriers. */
-template <typename R, int F, int M, int CL, int HM>
+ *      the fields goes to L2 (ld/st .cg), ordered by the cluster barriers.
+ * COPIES: copies of a field's dispersion step in the code (Engine::dispersion). */
+template <typename R>
+constexpr int field_copies(int F) { return sizeof(R) == 4 && F == 2 ? F : 1; }
+
+template <typename R, int F, int M, int CL, int HM, int COPIES = field_copies<R>(F)>
 struct Ssfm {
     static constexpr bool GH = (HM == 2);
     static constexpr bool INPLACE = (HM != 0); /* one exchange buffer per local transform */
@@ -709,11 +713,13 @@ struct Ssfm {
             const C *__restrict__ disp = reinterpret_cast<const C *>(tab.disp);
             /* FP32, 2 equations: one copy of the code per field, so that one
              * field's last stores overlap the other's loads (333 instances of
-             * 2^13: 9.3 ms against 10.1 with a loop).  Elsewhere one copy:
-             * kernels that run side by side share instruction caches, and the
-             * others gain nothing (32 FP64 instances of 2^12..2^15: 31.5 us per
-             * slice against 33.8 with a copy per field). */
-            constexpr int COPIES = (sizeof(R) == 4 && F == 2) ? F : 1;
+             * 2^13: 9.3 ms against 10.1 with a loop), except in the kernels
+             * of one CTA per SM (solo_f32_2eq.cu), which run side by side
+             * with other grids' and share instruction caches (32 instances
+             * of 2^12..2^15: 18.8 us per slice against 21.7 with a copy per
+             * field).  Elsewhere one copy: the others gain nothing from more
+             * (32 FP64 instances of 2^12..2^15: 31.5 us per slice against
+             * 33.8). */
 #pragma unroll COPIES
             for (int f = 0; f < F; f++) {
                 spectral<0>(fld(f), scratch, disp + ((size_t)f * CL + rank) * M, nullptr, 0.0, 0.0, 0, tab.inv_n, tw,
@@ -945,10 +951,10 @@ static __device__ __forceinline__ void drive(const LaunchArgs &a)
     }
 }
 
-template <typename R, int F, int M, int CL, int HM, int MINB>
+template <typename R, int F, int M, int CL, int HM, int MINB, int COPIES = field_copies<R>(F)>
 __global__ void __launch_bounds__(M / 16, MINB) ssfm_kernel(LaunchArgs a)
 {
-    drive<R, typename Ssfm<R, F, M, CL, HM>::Engine>(a);
+    drive<R, typename Ssfm<R, F, M, CL, HM, COPIES>::Engine>(a);
 }
 
 }  // namespace cuopo
