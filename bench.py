@@ -663,7 +663,7 @@ def warm_start_leg(args, seed: int = 7) -> dict:
         "bf16_peak_tflops": peak, "peak_source": "MEASURED_PEAKS.json bf16_tflops (cuBLAS burst)",
         "train_frac": (train_flops / (train_ms * 1e-3) / 1e12) / peak if peak else None,
         "note": "batch 4096, 4 -> 512 x 4 (GELU) -> 512; layer 0 padded to K = 64; the training step is one "
-                "CUDA graph (14 tcgen05 GEMM launches, loss and Adam) after an input-packing kernel"}
+                "CUDA graph (5 forward and 4 dX tcgen05 GEMM launches, one for every dW, Adam) after an input-packing kernel"}
     model.close()
     return out
 

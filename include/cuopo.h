@@ -196,7 +196,10 @@ cuopo_status cuopo_plan_create(cuopo_plan **plan, const cuopo_params *p,
                                int precision);
 cuopo_status cuopo_plan_destroy(cuopo_plan *plan);
 
-/* Cluster size and threads per CTA the plan launches with. */
+/* Cluster size and threads per CTA the plan launches with: a plan runs one
+ * instance, spread over up to 16 CTAs; a batch chooses per group, by the
+ * number of instances, among layouts of the same arithmetic (equal results
+ * bit for bit). */
 cuopo_status cuopo_plan_config(const cuopo_plan *plan, int *cluster, int *threads,
                                int *smem_bytes);
 
@@ -230,8 +233,10 @@ cuopo_status cuopo_round_trips(cuopo_plan *plan, void *Ap, void *As, void *Ai,
                                void *stream);
 
 /* Reads (and with reset != 0 clears) the plan's device-side status word:
- * CUOPO_OK, or CUOPO_ENONFINITE if a launch met a NaN/Inf signal power
- * (that instance stops at the round trip where it happened).  Synchronous. */
+ * CUOPO_OK, CUOPO_ENONFINITE if a launch met a NaN/Inf signal power
+ * (that instance stops at the round trip where it happened), or
+ * CUOPO_ETIMEOUT if a wait between an instance's CTAs gave up (about 1 s).
+ * Synchronous. */
 cuopo_status cuopo_plan_status(cuopo_plan *plan, int *status, int reset);
 
 /*
@@ -314,7 +319,8 @@ cuopo_status cuopo_batch_wait(cuopo_batch *batch, void *stream);
 /* Number of instances still running (synchronous). */
 cuopo_status cuopo_batch_pending(cuopo_batch *batch, int *running, void *stream);
 /* Per-instance last signal power, round trips run and flag (0 running,
- * 1 converged, 2 round-trip limit reached, 5 non-finite) into host arrays
+ * 1 converged, 2 round-trip limit reached, 4 a wait between the CTAs gave up,
+ * 5 non-finite) into host arrays
  * (any may be NULL).  Waits for stream. */
 cuopo_status cuopo_batch_results(cuopo_batch *batch, double *ps, int *rts, int *flags, void *stream);
 
@@ -340,7 +346,9 @@ cuopo_status cuopo_autotune(const cuopo_params *base, int precision, int count, 
 cuopo_status cuopo_kernel_select(int precision, int n_eqs, int n_t, int points_per_cta, int cluster);
 /* Forgets every autotuned or selected choice (the built-in preference order applies). */
 cuopo_status cuopo_autotune_reset(void);
-/* The configuration a plan created now would use. */
+/* The configuration (points per CTA and cluster size of the transforms'
+ * decomposition, which fixes the arithmetic) that a plan created now would
+ * use; cuopo_plan_config reports the CTAs that it runs on. */
 cuopo_status cuopo_kernel_config(int precision, int n_eqs, int n_t, int *points_per_cta, int *cluster);
 
 /*
