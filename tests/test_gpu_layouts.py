@@ -6,7 +6,7 @@ bit for bit, and within the oracle's bounds (F64 1e-10, F32 5e-5 over round
 trips, as for the other layouts).
 
 Counts are chosen to cross every rung: one instance, one and two waves of the
-16-CTA clusters, the 4-, 2- and 1-CTA layouts, two per SM."""
+16-CTA clusters, the 4-, 2- and 1-CTA layouts, one CTA per SM, two per SM."""
 import numpy as np
 import pytest
 
@@ -37,8 +37,8 @@ def run(neq, n_t, prec, count, n_rt=2):
 
 
 CASES = [(2, n, cu.F32, (1, 2, 40, 150, 300)) for n in (512, 1024, 2048)] + \
-        [(2, 4096, cu.F32, (1, 12, 30, 70, 200)), (2, 8192, cu.F32, (1, 10, 30, 80)), (2, 16384, cu.F32, (1, 10, 40)),
-         (2, 32768, cu.F32, (1, 20)), (3, 512, cu.F32, (1, 200)), (3, 1024, cu.F32, (1, 60, 140)),
+        [(2, 4096, cu.F32, (1, 12, 30, 70, 100, 200)), (2, 8192, cu.F32, (1, 10, 30, 50, 80)),
+         (2, 16384, cu.F32, (1, 10, 22, 40)), (2, 32768, cu.F32, (1, 10, 20)), (3, 512, cu.F32, (1, 200)), (3, 1024, cu.F32, (1, 60, 140)),
          (3, 2048, cu.F32, (1, 20, 60, 140)), (3, 4096, cu.F32, (1, 30, 70, 140, 160)), (3, 8192, cu.F32, (1, 12, 30, 80)),
          (3, 16384, cu.F32, (1, 12, 30, 40)), (3, 32768, cu.F32, (1, 10, 17)), (3, 65536, cu.F32, (1, 9)),
          (2, 512, cu.F64, (1, 100, 200)), (2, 1024, cu.F64, (1, 60, 140)), (2, 2048, cu.F64, (1, 60, 140)),
