@@ -736,8 +736,10 @@ struct Ssfm {
 
         __device__ __forceinline__ void gdd(const Tables &tab, const Instance &I)
         {
+            /* (nothing is staged here: with CL = 1 no barrier lies between the
+             * pass before this step, where every warp reads the coefficients,
+             * and its start; the pass after it uses none) */
             const float *__restrict__ w = tab.w + (size_t)rank * M;
-            st.write(t - (T - 32), staged);
             spectral<1>(fld(1), scratch, nullptr, w, I.gdd, I.tod_s, I.use_tod_s, tab.inv_n, tw, t);
             if constexpr (F == 3)
                 spectral<1>(fld(2), scratch, nullptr, w, I.gdd, I.tod_i, I.use_tod_i, tab.inv_n, tw, t);
@@ -897,7 +899,6 @@ static __device__ __forceinline__ void drive(const LaunchArgs &a)
                 E.pass(ALL, in_y, end, I, tab, rkc, a.eom_idler, th, acc);
                 end = Ops{};
                 end.frame = -1;
-                E.stage(end, tab, false);
                 E.gdd(tab, I);
             }
             const bool save = (rt >= I.save_first && rt < I.save_first + I.save_count);
