@@ -668,7 +668,8 @@ struct Ssfm {
                     for (int e = 0; e < 16; e++)
                         home[f * M + swz<C>(t + e * T)] = gf[f][(size_t)rank * M + t + e * T];
             }
-            xsync();
+            if constexpr (GH) xsync();
+            else bar();
         }
 
         __device__ __forceinline__ void store()
@@ -842,6 +843,9 @@ static __device__ __forceinline__ void drive(const LaunchArgs &a)
             tol = a.tol;
             patience = a.patience;
         }
+        /* (load() ends in a barrier of the instance: all its threads have read
+         * the state above before the leader writes it, even if no round trip
+         * is left to run) */
         E.load(I);
 
         double ps = prev_ps, acc = 0.0;

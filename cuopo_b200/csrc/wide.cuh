@@ -400,7 +400,7 @@ struct Wide {
 #pragma unroll
             for (int q = 0; q < F; q++)
                 for (int i = tid; i < CL * NP; i += NTHR) tb[q * CL * NP + i] = gf[q][point(i % NP, i / NP)];
-            __syncthreads();
+            barrier();
         }
 
         __device__ __forceinline__ void store()
