@@ -113,6 +113,7 @@ SIGNATURES = {
     "cuopo_batch_step": (_i, [_vp, _i, _i, _d, _i, _vp]),
     "cuopo_batch_pending": (_i, [_vp, C.POINTER(_i), _vp]),
     "cuopo_batch_results": (_i, [_vp, _vp, _vp, _vp, _vp]),
+    "cuopo_batch_hold": (_i, [_vp, _i]),
     "cuopo_batch_history": (_i, [_vp, _i, _vp, _i, _vp]),
     "cuopo_batch_wait": (_i, [_vp, _vp]),
     "cuopo_probe_fp32_peak": (_i, [C.POINTER(_d), _vp]),

@@ -668,6 +668,7 @@ struct cuopo_batch {
     cuopo_noise_item *d_noise;    /* per instance: place, size and seed of its noise */
     std::vector<size_t> offset;   /* element offset of each instance's fields */
     bool spread;                  /* several groups that fit one CTA per SM: launched so */
+    int hold;                     /* cuopo_batch_hold */
     size_t total;                 /* total signal elements */
     void *d_pump;                 /* pump-field work buffers (n_t per instance) */
     void *d_signal;               /* signal fields, concatenated */
@@ -1092,10 +1093,18 @@ extern "C" cuopo_status cuopo_batch_step(cuopo_batch *b, int chunk, int max_rt, 
         a.max_rt = max_rt;
         a.tol = tol;
         a.patience = patience;
+        a.hold = b->hold;
         cuopo_status s2 = launch(g.kernel, a, g.grid, g.stream, b->spread);
         if (s2 != CUOPO_OK) return s2;
         if ((e = cudaEventRecord(g.done, g.stream)) != cudaSuccess) return cuda_fail(e, "batch_step");
     }
+    return CUOPO_OK;
+}
+
+extern "C" cuopo_status cuopo_batch_hold(cuopo_batch *b, int on)
+{
+    if (!b) return cuopo_fail(CUOPO_EINVAL, "batch_hold: NULL batch");
+    b->hold = on != 0;
     return CUOPO_OK;
 }
 

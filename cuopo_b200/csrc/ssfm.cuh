@@ -104,6 +104,8 @@ struct LaunchArgs {
     int pass_only;              /* 1: one crystal pass, no cavity map */
     int use_eom, eom_idler;
     int *status;                /* first error code (atomicCAS from 0) */
+    int hold;                   /* test hook: exchanges into the first CTA of an instance never complete, so
+                                   its bounded waits run out (wide_kernel) */
     /* batch launches: continue each running instance by up to `chunk` round
      * trips, stopping at max_rt; convergence tolerance and patience */
     int chunk, max_rt, patience;
@@ -630,7 +632,7 @@ struct Ssfm {
         Stager st;
         int t, rank;
 
-        __device__ __forceinline__ void init()
+        __device__ __forceinline__ void init(int)
         {
             extern __shared__ __align__(16) unsigned char smem_raw[];
             C *const sm = reinterpret_cast<C *>(smem_raw);
@@ -734,6 +736,8 @@ struct Ssfm {
 
         __device__ __forceinline__ int failed() const { return 0; }
         __device__ __forceinline__ int error() const { return 0; }
+        __device__ __forceinline__ void report() {}
+        __device__ __forceinline__ void drain() const {}
 
         __device__ __forceinline__ void gdd(const Tables &tab, const Instance &I)
         {
@@ -792,7 +796,7 @@ static __device__ __forceinline__ void drive(const LaunchArgs &a)
     constexpr unsigned ALL = K::ALL;
     __shared__ int next_inst;
     Engine E;
-    E.init();
+    E.init(a.hold);
     bool first = true;
     for (;;) {
         int idx;
@@ -952,7 +956,15 @@ static __device__ __forceinline__ void drive(const LaunchArgs &a)
                 *I.st_flag = flag != 0 ? flag : (rt_begin + rts >= K::rt_limit(a, I) ? (int)ST_LIMIT : 0);
             }
         }
+        E.report();
         E.barrier();
+        if (E.error()) {
+            /* this cluster's exchanges are out of step: instances that it has
+             * not taken stay as they are, for another cluster or a later
+             * launch.  Nothing may still be on its way to a CTA that exits. */
+            E.drain();
+            break;
+        }
     }
 }
 

@@ -45,8 +45,13 @@
  * stage rotations before the wait or, where registers allow, once.
  *
  * The waits are bounded (1 s of %globaltimer): one that gives up marks the
- * CTA, all its later waits return at once, and the instance ends with
- * ST_TIMEOUT after the round trip, on every CTA of the cluster.
+ * CTA, which from the next pass on takes no part in the exchanges any more.
+ * It must not: its barrier's phase is incomplete with no arrival pending, and
+ * another arrival is undefined.  Its partners miss its bytes and give up in
+ * their turn, so no CTA gets more than one exchange ahead of a barrier.  The
+ * instance ends with ST_TIMEOUT after the round trip, on every CTA of the
+ * cluster, and the cluster takes no further one: it lets the stores under way
+ * land (drain()) and exits.
  */
 #pragma once
 #include "ssfm.cuh"
@@ -262,13 +267,14 @@ struct Wide {
         typename Math::Staged *staged;
         typename Math::Stager st;
         unsigned parity;           /* bit 3 b + f: parity of that mbarrier's next phase */
+        int gone;                  /* this CTA gave up a wait before the present pass: the same in all its threads */
         int tid, rank;
         int q;                     /* thread of the transform */
         QuadTw<C> qt;              /* Q == 4 */
         C *scr;
         StageRot<C> w_t, w_1, w_2, w_3; /* HOLD_TW: this thread's rotations */
 
-        __device__ __forceinline__ void init()
+        __device__ __forceinline__ void init(int hold)
         {
             extern __shared__ __align__(16) unsigned char smem_raw[];
             __shared__ unsigned long long s_mbar[6];
@@ -280,13 +286,16 @@ struct Wide {
             dead = s_dead;
             staged = &s_staged;
             parity = 0;
+            gone = 0;
             tid = threadIdx.x;
             rank = 0;
             if constexpr (P > 1) rank = (int)cg::this_cluster().block_rank();
             if (tid <= P) s_dead[tid] = 0;
             if constexpr (P > 1) {
                 if (tid < 6)
-                    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&s_mbar[tid])) : "memory");
+                    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&s_mbar[tid])),
+                                 "r"(hold && rank == 0 ? 0xFFFFF : 1) /* one arrival per exchange; held: never enough */
+                                 : "memory");
                 asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
             }
             q = tid % Q;
@@ -325,11 +334,13 @@ struct Wide {
                          v);
         }
 
-        /* Announces this CTA's bytes of the exchange into buffer b, per field of mask. */
+        /* Announces this CTA's bytes of the exchange into buffer b, per field of
+         * mask: every earlier wait has succeeded, so the barriers' phases are
+         * complete. */
         __device__ __forceinline__ void expect(int b, unsigned mask)
         {
             if constexpr (P > 1) {
-                if (tid < F && ((mask >> tid) & 1u))
+                if (tid < F && ((mask >> tid) & 1u) && !gone)
                     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(
                                      smem_addr(mbar + 3 * b + tid)),
                                  "r"((unsigned)(CL * NP * (int)sizeof(C)))
@@ -338,29 +349,51 @@ struct Wide {
         }
 
         /* Waits for field f of the exchange into buffer b (the threads that
-         * read it; then flip() by all, for the fields of the exchange). */
-        __device__ __forceinline__ void wait(int b, int f)
+         * read it; then flip() by all, for the fields of the exchange).  false:
+         * it has not come, and nothing must be sent on. */
+        __device__ __forceinline__ bool wait(int b, int f)
         {
             if constexpr (P > 1) {
+                if (gone) return false;
                 const unsigned m = smem_addr(mbar + 3 * b + f), par = (parity >> (3 * b + f)) & 1u;
-                if (mbar_test(m, par)) return;
+                if (mbar_test(m, par)) return true;
                 unsigned long long t0, t1;
                 asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
                 while (!mbar_test(m, par)) {
                     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
                     if (*(volatile int *)dead || t1 - t0 > 1000000000ull) {
                         *(volatile int *)dead = 1;
-                        return;
+                        return false;
                     }
                 }
             }
+            return true;
         }
         __device__ __forceinline__ void flip(int b, unsigned mask) { parity ^= mask << (3 * b); }
 
         /* a wait of this CTA gave up */
         __device__ __forceinline__ int failed() const { return P > 1 ? *(volatile int *)dead : 0; }
 
-        /* a wait of any CTA gave up (the same on every CTA, after power()) */
+        /* Tells every CTA whether a wait of this one gave up; error() holds
+         * after the next barrier(). */
+        __device__ __forceinline__ void report()
+        {
+            if constexpr (P > 1) {
+                if (tid < P) *cta(&dead[1 + rank], tid) = *(volatile int *)dead;
+            }
+        }
+
+        /* 2 ms for the stores under way to land in this CTA. */
+        __device__ __forceinline__ void drain() const
+        {
+            unsigned long long t0, t1;
+            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
+            do asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
+            while (t1 - t0 < 2000000ull);
+        }
+
+        /* a wait of any CTA gave up (the same on every CTA, after report() or
+         * power() and a barrier) */
         __device__ __forceinline__ int error() const
         {
             int e = 0;
@@ -440,6 +473,7 @@ struct Wide {
                 flip(0, in_y);
             }
             __syncthreads();
+            gone = failed(); /* (no wait comes before the next barrier) */
             const typename Math::Coef co = Math::coef(staged, rkc);
             if (op.frame >= 0) Math::frame_step(op, staged->c + 6, staged->u, th);
             if (out_y) expect(1, out_y);
@@ -492,7 +526,7 @@ struct Wide {
                 }
             }
             __syncthreads();
-            if (!out_y) return;
+            if (!out_y || gone) return;
 #pragma unroll 1
             for (int task = tid / Q; task < NT; task += NTHR / Q) {
                 const Role o(task, rank);
@@ -550,7 +584,7 @@ struct Wide {
 #pragma unroll
                     for (int a = 0; a < NV; a++) d[a] = ld_now(disp + 16 * Q * a);
                 }
-                wait(1, o.f);
+                const bool come = wait(1, o.f);
                 /* stage 1 (length R0): butterfly `lane`, k = r */
 #pragma unroll
                 for (int a = 0; a < NV; a++) v[a] = u[fb_at(lane + 16 * (q + Q * a))];
@@ -588,6 +622,7 @@ struct Wide {
                 for (int a = 0; a < NV; a++) v[a] = u[xc_at(q + Q * a, lane)];
                 if constexpr (HOLD_TW) dft_q<-1, true>(v, w_3, 2 * k >= R0, qt, scr);
                 else dft_q<-1, true>(v, o.rot_3(), 2 * k >= R0, qt, scr);
+                if (!come) continue;
                 /* output m: element cls of class k + R0 m */
 #pragma unroll
                 for (int a = 0; a < NV; a++) {
@@ -627,9 +662,7 @@ struct Wide {
                 const int g = rank * (Tc / 16) + t2l / 16;
                 if ((tid & 15) < P) *cta(&red[rk * G + g], tid & 15) = v;
             }
-            if constexpr (P > 1) {
-                if (tid < P) *cta(&dead[1 + rank], tid) = *(volatile int *)dead;
-            }
+            report();
             barrier();
             double part = 0.0;
 #pragma unroll

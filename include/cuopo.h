@@ -321,8 +321,14 @@ cuopo_status cuopo_batch_pending(cuopo_batch *batch, int *running, void *stream)
 /* Per-instance last signal power, round trips run and flag (0 running,
  * 1 converged, 2 round-trip limit reached, 4 a wait between the CTAs gave up,
  * 5 non-finite) into host arrays
- * (any may be NULL).  Waits for stream. */
+ * (any may be NULL).  Waits for stream.  With flag 4 the instance's fields are
+ * lost, and the CTAs that ran it take no further instance in that step: what
+ * no other CTAs have taken keeps flag 0, and the next step continues it. */
 cuopo_status cuopo_batch_results(cuopo_batch *batch, double *ps, int *rts, int *flags, void *stream);
+/* Test hook: with on != 0, the waits between the CTAs of an instance run out
+ * (flag 4, after about 1 s) in the steps that follow; instances that run on
+ * one CTA or on the general layout have no such waits. */
+cuopo_status cuopo_batch_hold(cuopo_batch *batch, int on);
 
 /*
  * Kernel autotuner (no counterpart in the reference, which has one cuFFT plan
