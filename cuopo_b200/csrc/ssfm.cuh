@@ -670,8 +670,7 @@ struct Ssfm {
                     for (int e = 0; e < 16; e++)
                         home[f * M + swz<C>(t + e * T)] = gf[f][(size_t)rank * M + t + e * T];
             }
-            if constexpr (GH) xsync();
-            else bar();
+            xsync();
         }
 
         __device__ __forceinline__ void store()
@@ -735,8 +734,8 @@ struct Ssfm {
         }
 
         __device__ __forceinline__ int failed() const { return 0; }
+        __device__ __forceinline__ bool stopped() const { return false; }
         __device__ __forceinline__ int error() const { return 0; }
-        __device__ __forceinline__ void report() {}
         __device__ __forceinline__ void drain() const {}
 
         __device__ __forceinline__ void gdd(const Tables &tab, const Instance &I)
@@ -847,9 +846,10 @@ static __device__ __forceinline__ void drive(const LaunchArgs &a)
             tol = a.tol;
             patience = a.patience;
         }
-        /* (load() ends in a barrier of the instance: all its threads have read
-         * the state above before the leader writes it, even if no round trip
-         * is left to run) */
+        /* no round trip left: without a round trip's barriers, all threads of
+         * the instance must still have read its state before the leader
+         * writes it below */
+        if (rt_count < 1) E.barrier();
         E.load(I);
 
         double ps = prev_ps, acc = 0.0;
@@ -883,7 +883,7 @@ static __device__ __forceinline__ void drive(const LaunchArgs &a)
                 }
                 return op;
             };
-            for (int s = 0; s < a.n_z; s++) {
+            for (int s = 0; s < a.n_z && !E.stopped(); s++) {
                 E.stage(between(s), tab, false);
                 E.dispersion(tab);
                 if (s + 1 < a.n_z) {
@@ -956,9 +956,8 @@ static __device__ __forceinline__ void drive(const LaunchArgs &a)
                 *I.st_flag = flag != 0 ? flag : (rt_begin + rts >= K::rt_limit(a, I) ? (int)ST_LIMIT : 0);
             }
         }
-        E.report();
         E.barrier();
-        if (E.error()) {
+        if (E.failed() || E.error()) {
             /* this cluster's exchanges are out of step: instances that it has
              * not taken stay as they are, for another cluster or a later
              * launch.  Nothing may still be on its way to a CTA that exits. */

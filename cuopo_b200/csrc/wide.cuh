@@ -44,11 +44,13 @@
  * memory before the dispersion step (stage()), the dispersion rows and the
  * stage rotations before the wait or, where registers allow, once.
  *
- * The waits are bounded (1 s of %globaltimer): one that gives up marks the
- * CTA, which from the next pass on takes no part in the exchanges any more.
- * It must not: its barrier's phase is incomplete with no arrival pending, and
- * another arrival is undefined.  Its partners miss its bytes and give up in
- * their turn, so no CTA gets more than one exchange ahead of a barrier.  The
+ * The waits are bounded (1 s of %globaltimer).  One that gives up marks the
+ * CTA, whose other waits then give up at once.  The barrier's phase is
+ * incomplete with no arrival pending, and another arrival is undefined, so
+ * from the next pass on the CTA announces nothing any more and its slices end
+ * (stopped(): read once per pass and used at the loop's own test; tests beside
+ * the sends cost 2..4 % of a slice).  Its partners miss its bytes and give up
+ * in their turn, so none gets more than two exchanges ahead of another.  The
  * instance ends with ST_TIMEOUT after the round trip, on every CTA of the
  * cluster, and the cluster takes no further one: it lets the stores under way
  * land (drain()) and exits.
@@ -267,7 +269,7 @@ struct Wide {
         typename Math::Staged *staged;
         typename Math::Stager st;
         unsigned parity;           /* bit 3 b + f: parity of that mbarrier's next phase */
-        int gone;                  /* this CTA gave up a wait before the present pass: the same in all its threads */
+        int gone;                  /* a wait of the CTA had given up by the latest pass (the same in every thread) */
         int tid, rank;
         int q;                     /* thread of the transform */
         QuadTw<C> qt;              /* Q == 4 */
@@ -335,8 +337,7 @@ struct Wide {
         }
 
         /* Announces this CTA's bytes of the exchange into buffer b, per field of
-         * mask: every earlier wait has succeeded, so the barriers' phases are
-         * complete. */
+         * mask (every wait before has succeeded: the barriers' phases are complete). */
         __device__ __forceinline__ void expect(int b, unsigned mask)
         {
             if constexpr (P > 1) {
@@ -349,39 +350,30 @@ struct Wide {
         }
 
         /* Waits for field f of the exchange into buffer b (the threads that
-         * read it; then flip() by all, for the fields of the exchange).  false:
-         * it has not come, and nothing must be sent on. */
-        __device__ __forceinline__ bool wait(int b, int f)
+         * read it; then flip() by all, for the fields of the exchange). */
+        __device__ __forceinline__ void wait(int b, int f)
         {
             if constexpr (P > 1) {
-                if (gone) return false;
                 const unsigned m = smem_addr(mbar + 3 * b + f), par = (parity >> (3 * b + f)) & 1u;
-                if (mbar_test(m, par)) return true;
+                if (mbar_test(m, par)) return;
                 unsigned long long t0, t1;
                 asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
                 while (!mbar_test(m, par)) {
                     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
                     if (*(volatile int *)dead || t1 - t0 > 1000000000ull) {
                         *(volatile int *)dead = 1;
-                        return false;
+                        return;
                     }
                 }
             }
-            return true;
         }
         __device__ __forceinline__ void flip(int b, unsigned mask) { parity ^= mask << (3 * b); }
 
+        /* no further slices (the same in every thread of the CTA) */
+        __device__ __forceinline__ bool stopped() const { return P > 1 && gone; }
+
         /* a wait of this CTA gave up */
         __device__ __forceinline__ int failed() const { return P > 1 ? *(volatile int *)dead : 0; }
-
-        /* Tells every CTA whether a wait of this one gave up; error() holds
-         * after the next barrier(). */
-        __device__ __forceinline__ void report()
-        {
-            if constexpr (P > 1) {
-                if (tid < P) *cta(&dead[1 + rank], tid) = *(volatile int *)dead;
-            }
-        }
 
         /* 2 ms for the stores under way to land in this CTA. */
         __device__ __forceinline__ void drain() const
@@ -392,8 +384,7 @@ struct Wide {
             while (t1 - t0 < 2000000ull);
         }
 
-        /* a wait of any CTA gave up (the same on every CTA, after report() or
-         * power() and a barrier) */
+        /* a wait of any CTA gave up (the same on every CTA, after power()) */
         __device__ __forceinline__ int error() const
         {
             int e = 0;
@@ -433,7 +424,7 @@ struct Wide {
 #pragma unroll
             for (int q = 0; q < F; q++)
                 for (int i = tid; i < CL * NP; i += NTHR) tb[q * CL * NP + i] = gf[q][point(i % NP, i / NP)];
-            barrier();
+            __syncthreads();
         }
 
         __device__ __forceinline__ void store()
@@ -526,7 +517,7 @@ struct Wide {
                 }
             }
             __syncthreads();
-            if (!out_y || gone) return;
+            if (!out_y) return;
 #pragma unroll 1
             for (int task = tid / Q; task < NT; task += NTHR / Q) {
                 const Role o(task, rank);
@@ -569,6 +560,7 @@ struct Wide {
         template <int MODE>
         __device__ __forceinline__ void spectral(unsigned mask, const Tables &tab, const Instance *I)
         {
+            if (MODE == 1 && gone) return;
             expect(0, mask);
 #pragma unroll 1
             for (int task = tid / Q; task < NT; task += NTHR / Q) {
@@ -584,7 +576,7 @@ struct Wide {
 #pragma unroll
                     for (int a = 0; a < NV; a++) d[a] = ld_now(disp + 16 * Q * a);
                 }
-                const bool come = wait(1, o.f);
+                wait(1, o.f);
                 /* stage 1 (length R0): butterfly `lane`, k = r */
 #pragma unroll
                 for (int a = 0; a < NV; a++) v[a] = u[fb_at(lane + 16 * (q + Q * a))];
@@ -622,7 +614,6 @@ struct Wide {
                 for (int a = 0; a < NV; a++) v[a] = u[xc_at(q + Q * a, lane)];
                 if constexpr (HOLD_TW) dft_q<-1, true>(v, w_3, 2 * k >= R0, qt, scr);
                 else dft_q<-1, true>(v, o.rot_3(), 2 * k >= R0, qt, scr);
-                if (!come) continue;
                 /* output m: element cls of class k + R0 m */
 #pragma unroll
                 for (int a = 0; a < NV; a++) {
@@ -662,7 +653,9 @@ struct Wide {
                 const int g = rank * (Tc / 16) + t2l / 16;
                 if ((tid & 15) < P) *cta(&red[rk * G + g], tid & 15) = v;
             }
-            report();
+            if constexpr (P > 1) {
+                if (tid < P) *cta(&dead[1 + rank], tid) = *(volatile int *)dead;
+            }
             barrier();
             double part = 0.0;
 #pragma unroll
