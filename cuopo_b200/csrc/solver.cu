@@ -66,8 +66,9 @@ extern "C" const char *cuopo_version(void) { return "cuopo_b200 0.1.0 (sm_100a)"
  * entries are in order of measured batch throughput on the B200: 2-eq 2^13,
  * 2^14 and 2^15 run faster as clusters of 2, 4 and 8 4096-point CTAs, two
  * CTAs per SM, than as 1, 2 and 4 8192-point CTAs, one per SM).  The
- * single-CTA entries stay reachable for callers that need one
- * (crystal_pass_noalloc). */
+ * single-CTA entries stay reachable for the caller that needs one:
+ * crystal_pass_noalloc runs on one CTA (the entry itself, or a layout of it
+ * that has one). */
 static const KernelList *const k_lists[] = {&kern_f32_2eq, &kern_f32_3eq, &kern_f64_2eq, &kern_f64_3eq};
 
 /* Calls f(entry) for every built configuration until it returns true. */
@@ -146,13 +147,15 @@ static std::vector<const KernelEntry *> layouts(const KernelEntry *k)
  * 2^12-point instance, for example, takes 11.1 us per slice on one CTA and
  * 3.1 spread over 16, but only 14 of those clusters are resident against 296
  * CTAs, so between 15 and 33 instances 4 CTAs each are best (4.2 us), then 2
- * each (7.1) up to 74, then one. */
-static const KernelEntry *pick_layout(const KernelEntry *k, int count)
+ * each (7.1) up to 74, then one.  single_cta: among the layouts of one CTA per
+ * instance, which have no waits between CTAs (crystal_pass_noalloc, whose
+ * caller has no status to read). */
+static const KernelEntry *pick_layout(const KernelEntry *k, int count, bool single_cta = false)
 {
     const KernelEntry *best = k;
     double t = 0;
     for (const KernelEntry *w : layouts(k)) {
-        if (!w) continue;
+        if (!w || (single_cta && w->ctas != 1)) continue;
         const double tw = slice_time(*w, count);
         if (w == k || tw < t) {
             best = w;
@@ -1324,7 +1327,7 @@ extern "C" cuopo_status cuopo_crystal_pass_noalloc(const cuopo_params *p, const 
     if (p->n_z < 1 || p->n_z > CUOPO_NOALLOC_MAX_NZ)
         return cuopo_fail(CUOPO_EINVAL, "crystal_pass_noalloc: n_z must be in [1, 1024]");
     const KernelEntry *k = find_kernel(CUOPO_F32, p->n_eqs, p->n_t, true);
-    k = pick_layout(k, 1);
+    k = pick_layout(k, 1, true);
     if (!k) return cuopo_fail(CUOPO_EUNSUPPORTED, "crystal_pass_noalloc: no single-CTA kernel for n_t");
     const int N = p->n_t, F = p->n_eqs;
 
