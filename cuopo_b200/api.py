@@ -238,7 +238,8 @@ def probe_fp64_peak(stream=None) -> float:
 def autotune(base: Params, precision: int = F32, count: int = 148, n_rt: int = 2) -> dict:
     """Times every built kernel configuration for base.n_t on `count` copies of
     the CW instance `base` (n_rt round trips each) and makes the fastest the
-    one later plans and batches of this process use (cuopo_autotune)."""
+    one that later batches of this process with at least `count` such instances
+    use (cuopo_autotune)."""
     m, cl, ms = C.c_int(), C.c_int(), C.c_double()
     check(load().cuopo_autotune(C.byref(base), precision, count, n_rt, C.byref(m), C.byref(cl), C.byref(ms)))
     return {"points_per_cta": m.value, "cluster": cl.value, "ms": ms.value}
@@ -254,7 +255,7 @@ def kernel_select(n_t: int, points_per_cta: int, cluster: int, n_eqs: int = 2, p
 
 
 def kernel_config(n_t: int, n_eqs: int = 2, precision: int = F32) -> tuple[int, int]:
-    """(points per CTA, CTAs per cluster) a plan for this grid would use now."""
+    """(points per CTA, CTAs per cluster) recorded for this grid, or the built-in choice (cuopo_kernel_config)."""
     m, cl = C.c_int(), C.c_int()
     check(load().cuopo_kernel_config(precision, n_eqs, n_t, C.byref(m), C.byref(cl)))
     return m.value, cl.value

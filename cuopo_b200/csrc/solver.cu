@@ -80,24 +80,30 @@ static void each_kernel(Fn f)
             if (f(l->k[i])) return;
 }
 
-/* Autotuned choices, process-wide: (precision, F, N) -> entry. */
+/* Recorded choices, process-wide: (precision, F, N) -> entry, for launches of
+ * at least `from` instances: the number that the autotuner timed (for fewer,
+ * a decomposition that is a few percent faster on a full chip may lack the
+ * layouts that spread an instance: 8192-point CTAs have none), or 1 for a
+ * choice made by hand. */
 struct TunedChoice {
     int precision, F, N;
     const KernelEntry *k;
+    int from;
 };
 static std::mutex g_tune_mu;
 static std::vector<TunedChoice> g_tuned;
 /* set by cuopo_autotune on its own thread while it times one candidate */
 static thread_local const KernelEntry *g_force = nullptr;
 
-static const KernelEntry *find_kernel(int precision, int F, int N, bool single_cta = false)
+/* count: instances that the kernel is for. */
+static const KernelEntry *find_kernel(int precision, int F, int N, int count, bool single_cta = false)
 {
     if (!single_cta) {
         if (g_force && g_force->precision == precision && g_force->F == F && g_force->M * g_force->CL == N)
             return g_force;
         std::lock_guard<std::mutex> lock(g_tune_mu);
         for (const TunedChoice &c : g_tuned)
-            if (c.precision == precision && c.F == F && c.N == N) return c.k;
+            if (c.precision == precision && c.F == F && c.N == N && count >= c.from) return c.k;
     }
     const KernelEntry *found = nullptr;
     each_kernel([&](const KernelEntry &k) {
@@ -126,14 +132,14 @@ static double slice_time(const KernelEntry &k, int count)
 }
 
 /* Every layout of k's arithmetic (same M and CL: the same results bit for
- * bit), k first.  A kernel chosen by hand (cuopo_kernel_select) keeps its M
- * and CL; one that the autotuner is timing runs as it is. */
+ * bit), k first.  A kernel chosen by hand or by the autotuner keeps its M
+ * and CL only. */
 static std::vector<const KernelEntry *> layouts(const KernelEntry *k)
 {
     static const KernelList *const lists[] = {&solo_f32_2eq, &wide_f32_2eq, &wide_f32_3eq, &wide_f64_2eq,
                                               &wide_f64_3eq};
     std::vector<const KernelEntry *> v{k};
-    if (!k || k == g_force || k->us1 <= 0) return v;
+    if (!k || k->us1 <= 0) return v;
     for (const KernelList *l : lists)
         for (int i = 0; i < l->n; i++) {
             const KernelEntry &w = l->k[i];
@@ -408,7 +414,7 @@ static cuopo_status plan_create(cuopo_plan **out, const cuopo_params *p, const f
     if (phase32) precision = CUOPO_F32;
     if (!k) {
         /* a plan runs one instance at a time */
-        k = pick_layout(find_kernel(precision, p->n_eqs, p->n_t), 1);
+        k = pick_layout(find_kernel(precision, p->n_eqs, p->n_t, 1), 1);
     }
     if (!k) return cuopo_fail(CUOPO_EUNSUPPORTED, "no kernel built for this (precision, n_eqs, n_t)");
 
@@ -752,7 +758,7 @@ static cuopo_status batch_build(cuopo_batch **out, const std::vector<cuopo_param
             return cuopo_fail(CUOPO_EINVAL, "batch_create: bad regime");
         }
         if (p.n_eqs != 2 && p.n_eqs != 3) return cuopo_fail(CUOPO_EINVAL, "batch_create: n_eqs must be 2 or 3");
-        if (!is_pow2i(p.n_t) || !find_kernel(precision, p.n_eqs, p.n_t))
+        if (!is_pow2i(p.n_t) || !find_kernel(precision, p.n_eqs, p.n_t, 1))
             return cuopo_fail(CUOPO_EUNSUPPORTED, "batch_create: an instance has an unsupported n_t");
         if (p.n_z < 1) return cuopo_fail(CUOPO_EINVAL, "batch_create: n_z must be >= 1");
         if (!(p.Rs >= 0.0 && p.Rs <= 1.0) || !(p.Ri >= 0.0 && p.Ri <= 1.0))
@@ -859,10 +865,10 @@ static cuopo_status batch_build(cuopo_batch **out, const std::vector<cuopo_param
     std::vector<const KernelEntry *> base;
     std::vector<int> members;
     for (const std::array<int, 5> &key : keys) {
-        base.push_back(find_kernel(precision, key[0], key[1]));
         members.push_back(0);
         for (const cuopo_params &p : prm)
             members.back() += std::array<int, 5>{p.n_eqs, p.n_t, p.n_z, p.eom_idler, p.regime} == key;
+        base.push_back(find_kernel(precision, key[0], key[1], members.back()));
     }
     const std::vector<const KernelEntry *> pick = share_chip(base, members, b->spread);
     for (const std::array<int, 5> &key : keys) {
@@ -1188,7 +1194,8 @@ extern "C" cuopo_status cuopo_autotune(const cuopo_params *base, int precision, 
         if (base->regime != CUOPO_CW)
             return cuopo_fail(CUOPO_EUNSUPPORTED, "autotune: timing runs use CW 2-equation batches");
         /* `count` copies of the base instance, seeded noise, n_rt round trips
-         * with the convergence test off (fixed work), per candidate */
+         * with the convergence test off (fixed work), per candidate, on the
+         * layout that a batch of that many takes */
         std::vector<cuopo_instance> inst((size_t)count);
         for (int i = 0; i < count; i++) {
             inst[(size_t)i].n_t = N;
@@ -1242,9 +1249,10 @@ extern "C" cuopo_status cuopo_autotune(const cuopo_params *base, int precision, 
         for (TunedChoice &c : g_tuned)
             if (c.precision == precision && c.F == F && c.N == N) {
                 c.k = best;
+                c.from = count;
                 found = true;
             }
-        if (!found) g_tuned.push_back(TunedChoice{precision, F, N, best});
+        if (!found) g_tuned.push_back(TunedChoice{precision, F, N, best, count});
     }
     if (points_per_cta) *points_per_cta = best->M;
     if (cluster) *cluster = best->CL;
@@ -1266,9 +1274,10 @@ extern "C" cuopo_status cuopo_kernel_select(int precision, int n_eqs, int n_t, i
         for (TunedChoice &c : g_tuned)
             if (c.precision == precision && c.F == n_eqs && c.N == n_t) {
                 c.k = found;
+                c.from = 1;
                 return CUOPO_OK;
             }
-        g_tuned.push_back(TunedChoice{precision, n_eqs, n_t, found});
+        g_tuned.push_back(TunedChoice{precision, n_eqs, n_t, found, 1});
         return CUOPO_OK;
     }
     return cuopo_fail(CUOPO_EUNSUPPORTED, "kernel_select: no such built configuration");
@@ -1283,7 +1292,7 @@ extern "C" cuopo_status cuopo_autotune_reset(void)
 
 extern "C" cuopo_status cuopo_kernel_config(int precision, int n_eqs, int n_t, int *points_per_cta, int *cluster)
 {
-    const KernelEntry *k = find_kernel(precision, n_eqs, n_t);
+    const KernelEntry *k = find_kernel(precision, n_eqs, n_t, INT_MAX);
     if (!k) return cuopo_fail(CUOPO_EUNSUPPORTED, "kernel_config: no kernel built for this (precision, n_eqs, n_t)");
     if (points_per_cta) *points_per_cta = k->M;
     if (cluster) *cluster = k->CL;
@@ -1326,7 +1335,7 @@ extern "C" cuopo_status cuopo_crystal_pass_noalloc(const cuopo_params *p, const 
                                         "(its tables live in a fixed 384 KiB device array)");
     if (p->n_z < 1 || p->n_z > CUOPO_NOALLOC_MAX_NZ)
         return cuopo_fail(CUOPO_EINVAL, "crystal_pass_noalloc: n_z must be in [1, 1024]");
-    const KernelEntry *k = find_kernel(CUOPO_F32, p->n_eqs, p->n_t, true);
+    const KernelEntry *k = find_kernel(CUOPO_F32, p->n_eqs, p->n_t, 1, true);
     k = pick_layout(k, 1, true);
     if (!k) return cuopo_fail(CUOPO_EUNSUPPORTED, "crystal_pass_noalloc: no single-CTA kernel for n_t");
     const int N = p->n_t, F = p->n_eqs;

@@ -337,8 +337,9 @@ cuopo_status cuopo_batch_hold(cuopo_batch *batch, int on);
  * 8192) are timed on `count` copies of the CW 2-equation instance `base`
  * (its n_t, ap0, Rs, delta, gdd) for n_rt round trips each (best of two
  * runs); the built-in choice stays unless another configuration is more
- * than 3 % faster, and the result becomes the one every plan and batch
- * created afterwards in this process uses for (precision, n_eqs, n_t).
+ * than 3 % faster, and the result becomes the one that batches of at least
+ * `count` such instances created afterwards in this process use for
+ * (precision, n_eqs, n_t); plans and smaller batches keep the built-in choice.
  * The timing runs one grid size alone: in a sweep that runs several grid
  * sizes at once, configurations with one CTA per SM pack worse next to the
  * others than this timing shows.  Reports the chosen points per CTA,
@@ -347,14 +348,16 @@ cuopo_status cuopo_batch_hold(cuopo_batch *batch, int on);
  */
 cuopo_status cuopo_autotune(const cuopo_params *base, int precision, int count, int n_rt, int *points_per_cta,
                             int *cluster, double *ms);
-/* Records a built configuration as the choice for (precision, n_eqs, n_t)
- * without timing (CUOPO_EUNSUPPORTED if it was not built). */
+/* Records a built configuration as the choice for (precision, n_eqs, n_t),
+ * for plans and batches of any size, without timing (CUOPO_EUNSUPPORTED if it
+ * was not built). */
 cuopo_status cuopo_kernel_select(int precision, int n_eqs, int n_t, int points_per_cta, int cluster);
 /* Forgets every autotuned or selected choice (the built-in preference order applies). */
 cuopo_status cuopo_autotune_reset(void);
 /* The configuration (points per CTA and cluster size of the transforms'
- * decomposition, which fixes the arithmetic) that a plan created now would
- * use; cuopo_plan_config reports the CTAs that it runs on. */
+ * decomposition, which fixes the arithmetic) that a large batch created now
+ * would use, and a plan too unless an autotuned choice differs from the
+ * built-in one; cuopo_plan_config reports the CTAs that a plan runs on. */
 cuopo_status cuopo_kernel_config(int precision, int n_eqs, int n_t, int *points_per_cta, int *cluster);
 
 /*
