@@ -121,26 +121,30 @@ static int one_per_sm(const KernelEntry &k)
 }
 
 /* Measured time per slice of `count` instances on kernel k: its resident
- * clusters work through them in waves.  A wave runs at us1 while every SM
- * sub-partition has one warp: one CTA per SM, or as many as 128 threads make
- * (F64, 3 equations, 2^10 points on CTAs of 64 threads: 152..266 instances
- * 11.7 us, one to 148 10.1, a full load of 444 16.2).  With several CTAs per
- * SM these do not all end together, and the next wave starts early: a last
- * wave of one CTA per SM adds 0.6..0.85 of the time it takes alone (2^12,
- * F32: 297..444 instances 24.5 us, 296 17.2, 148 10.5).  Over 440 counts
- * around one to three full loads of every grid size this rule takes a layout
- * on average 0.2 % slower than the best and at no count slower than the general
- * one; without the two corrections 0.6 %, and up to 24 % slower (F64, 3
+ * clusters work through them in waves.  A wave of one CTA per SM takes us1;
+ * CTAs of fewer than 128 threads leave SM sub-partitions without a warp, and
+ * until each has one a wave takes little longer (F64, 3 equations, 2^10 points
+ * on CTAs of 64 threads: up to 148 instances 10.1 us, 152..266 11.7, a full
+ * load of 444 16.2): a quarter of the way to us_full at that limit.  With
+ * several CTAs per SM a wave does not end all at once, and the next starts
+ * early: a last wave of that kind adds 0.6..0.85 of the time it takes alone
+ * (2^12, F32: 297..444 instances 24.5 us, 296 17.2, 148 10.5).  Over 822 counts
+ * up to three full loads, every grid size, this rule takes a layout on average
+ * 0.24 % slower than the best and at no count more than 0.6 % slower than the
+ * general one; without the two corrections 0.64 % and up to 24 % (F64, 3
  * equations, 1110 of 2^9: 27.8 us, now 22.6). */
 static double slice_time(const KernelEntry &k, int count)
 {
     const int occ = k.occ();
     if (occ < 1 || k.us1 <= 0) return 1e30;
     const int waves = count / occ, rest = count % occ, one = one_per_sm(k);
-    double t = waves * (double)k.us_full;
-    if (rest > one * std::max(1, 128 / k.threads)) t += k.us_full;
-    else if (rest > 0) t += (waves > 0 && occ > one ? 0.88 : 1.0) * k.us1;
-    return t;
+    const int light = one * std::max(1, 128 / k.threads);
+    const double full = waves * (double)k.us_full;
+    if (rest == 0) return full;
+    if (rest > light) return full + k.us_full;
+    double last = k.us1;
+    if (rest > one) last += 0.25 * (k.us_full - k.us1) * (rest - one) / (light - one);
+    return full + (waves > 0 && occ > one ? 0.88 : 1.0) * last;
 }
 
 /* Every layout of k's arithmetic (same M and CL: the same results bit for

@@ -37,6 +37,7 @@ def kernel_blocks(call):
     (3, 1024, cu.F64, 500, 64),     # 22.1 against 25.2
     (2, 1024, cu.F64, 200, 64),     # 11.2 against 11.8
     (2, 1024, cu.F32, 200, 256),    # the spread layout where it is the faster one: 5.5 against 6.7
+    (3, 512, cu.F64, 339, 128),     # 10.0 against 11.2
     (2, 512, cu.F32, 260, 128)])    # 3.7 against 6.2
 def test_batch_takes_the_faster_layout(neq, n_t, prec, count, threads):
     p = (params_2eq if neq == 2 else params_3eq)(n_t=n_t, n_z=2, regime=cu.CW)
