@@ -337,11 +337,11 @@ struct Wide {
         }
 
         /* Announces this CTA's bytes of the exchange into buffer b, per field of
-         * mask (every wait before has succeeded: the barriers' phases are complete). */
-        __device__ __forceinline__ void expect(int b, unsigned mask)
+         * mask; go: every wait before has succeeded (the barriers' phases are complete). */
+        __device__ __forceinline__ void expect(int b, unsigned mask, bool go)
         {
             if constexpr (P > 1) {
-                if (tid < F && ((mask >> tid) & 1u) && !gone)
+                if (tid < F && ((mask >> tid) & 1u) && go)
                     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(
                                      smem_addr(mbar + 3 * b + tid)),
                                  "r"((unsigned)(CL * NP * (int)sizeof(C)))
@@ -467,7 +467,7 @@ struct Wide {
             gone = failed(); /* (no wait comes before the next barrier) */
             const typename Math::Coef co = Math::coef(staged, rkc);
             if (op.frame >= 0) Math::frame_step(op, staged->c + 6, staged->u, th);
-            if (out_y) expect(1, out_y);
+            if (out_y) expect(1, out_y, !gone);
             if constexpr (SPLIT) {
                 cross_field<-1>(in_y, twN);
                 __syncthreads();
@@ -561,7 +561,7 @@ struct Wide {
         __device__ __forceinline__ void spectral(unsigned mask, const Tables &tab, const Instance *I)
         {
             if (MODE == 1 && gone) return;
-            expect(0, mask);
+            expect(0, mask, true); /* (not reached once gone: stopped() ends the slices) */
 #pragma unroll 1
             for (int task = tid / Q; task < NT; task += NTHR / Q) {
                 const Role o(task, rank);
