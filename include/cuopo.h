@@ -199,7 +199,9 @@ cuopo_status cuopo_plan_destroy(cuopo_plan *plan);
 /* Cluster size and threads per CTA the plan launches with: a plan runs one
  * instance, spread over up to 16 CTAs; a batch chooses per group, by the
  * number of instances, among layouts of the same arithmetic (equal results
- * bit for bit). */
+ * bit for bit).  To run many instances at once use a batch: plans on several
+ * streams are each laid out as if alone (16 CTAs from 2^12 points on, 7 to
+ * 14 of which fit the GPU at once). */
 cuopo_status cuopo_plan_config(const cuopo_plan *plan, int *cluster, int *threads,
                                int *smem_bytes);
 
@@ -377,7 +379,8 @@ cuopo_status cuopo_kernel_config(int precision, int n_eqs, int n_t, int *points_
  * that array's address and keeps it for the life of the process (so the
  * library must not be used across a cudaDeviceReset of that device).  The
  * array is shared by all calls and keeps the last call's tables, so calls
- * that overlap on the GPU race -- order them on one stream.  The pass does
+ * that overlap on the GPU race -- order them on one stream.  It runs on one
+ * CTA, without the waits between CTAs that a plan's pass may have.  The pass does
  * not report non-finite fields (there is no status to read back; check the
  * fields).  w_host: the n_t angular frequencies, or NULL to build them from
  * p->t_rt.
