@@ -4,6 +4,7 @@
  */
 #include <cuda_runtime.h>
 
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -11,6 +12,7 @@
 #include <algorithm>
 #include <array>
 #include <mutex>
+#include <utility>
 #include <vector>
 
 #include "cuopo.h"
@@ -113,6 +115,17 @@ static const KernelEntry *find_kernel(int precision, int F, int N, int count, bo
     return found;
 }
 
+/* At most so many clusters of k are resident (one per SM where a full chip
+ * takes no longer than one CTA per SM), known without asking for its
+ * occupancy: that loads the kernel, some milliseconds each at its first use in
+ * a process. */
+static int resident_bound(const KernelEntry &k)
+{
+    const int by_smem = (int)(228 * 1024 / (k.smem + 1024)), by_threads = 2048 / k.threads;
+    const int per_sm = k.us_full > k.us1 ? std::min(by_smem, std::min(by_threads, 32)) : 1;
+    return 148 * std::max(per_sm, 1) / k.ctas;
+}
+
 /* Clusters of k that are resident with one CTA per SM. */
 static int one_per_sm(const KernelEntry &k)
 {
@@ -147,6 +160,37 @@ static double slice_time(const KernelEntry &k, int count)
     return full + (waves > 0 && occ > one ? 0.88 : 1.0) * last;
 }
 
+/* No more than slice_time: with as many resident clusters as can be. */
+static double slice_time_bound(const KernelEntry &k, int count)
+{
+    const int occ = resident_bound(k);
+    if (occ < 1 || k.us1 <= 0) return 1e30;
+    const int waves = count / occ, rest = count % occ;
+    return waves * (double)k.us_full + (rest == 0 ? 0.0 : (waves > 0 ? 0.88 : 1.0) * k.us1);
+}
+
+/* The entry of the least cost(entry) in v, the first one of equals.  bound(entry)
+ * is at most its cost; costs are asked for in the order of the bounds and only
+ * while one can still be the least. */
+template <typename Cost, typename Bound>
+static const KernelEntry *least(const std::vector<const KernelEntry *> &v, Cost cost, Bound bound)
+{
+    std::vector<std::pair<double, size_t>> order;
+    for (size_t i = 0; i < v.size(); i++) order.push_back({bound(*v[i]), i});
+    std::sort(order.begin(), order.end());
+    double t = 0;
+    size_t best = v.size();
+    for (const std::pair<double, size_t> &o : order) {
+        if (best < v.size() && o.first > t) break;
+        const double c = cost(*v[o.second]);
+        if (best == v.size() || c < t || (c == t && o.second < best)) {
+            t = c;
+            best = o.second;
+        }
+    }
+    return best < v.size() ? v[best] : nullptr;
+}
+
 /* Every layout of k's arithmetic (same M and CL: the same results bit for
  * bit), k first.  A kernel chosen by hand or by the autotuner keeps its M
  * and CL only. */
@@ -159,8 +203,7 @@ static std::vector<const KernelEntry *> layouts(const KernelEntry *k)
     for (const KernelList *l : lists)
         for (int i = 0; i < l->n; i++) {
             const KernelEntry &w = l->k[i];
-            if (w.precision == k->precision && w.F == k->F && w.M == k->M && w.CL == k->CL && w.occ() > 0)
-                v.push_back(&w);
+            if (w.precision == k->precision && w.F == k->F && w.M == k->M && w.CL == k->CL) v.push_back(&w);
         }
     return v;
 }
@@ -174,17 +217,12 @@ static std::vector<const KernelEntry *> layouts(const KernelEntry *k)
  * caller has no status to read). */
 static const KernelEntry *pick_layout(const KernelEntry *k, int count, bool single_cta = false)
 {
-    const KernelEntry *best = k;
-    double t = 0;
-    for (const KernelEntry *w : layouts(k)) {
-        if (!w || (single_cta && w->ctas != 1)) continue;
-        const double tw = slice_time(*w, count);
-        if (w == k || tw < t) {
-            best = w;
-            t = tw;
-        }
-    }
-    return best;
+    if (!k) return k;
+    std::vector<const KernelEntry *> v;
+    for (const KernelEntry *w : layouts(k))
+        if (w == k || !single_cta || w->ctas == 1) v.push_back(w);
+    return least(v, [&](const KernelEntry &w) { return slice_time(w, count); },
+                 [&](const KernelEntry &w) { return slice_time_bound(w, count); });
 }
 
 /* k for launches of at most one CTA per SM (solo_f32_2eq.cu), or k itself. */
@@ -233,9 +271,11 @@ static std::vector<const KernelEntry *> share_chip(const std::vector<const Kerne
         size_t slow = 0;
         for (size_t g = 1; g < k.size(); g++)
             if (pick[g]->us1 > pick[slow]->us1) slow = g;
-        const KernelEntry *next = nullptr;
+        std::vector<const KernelEntry *> faster;
         for (const KernelEntry *w : layouts(k[slow]))
-            if (w->us1 < pick[slow]->us1 && (!next || share(w, n[slow]) < share(next, n[slow]))) next = w;
+            if (w->us1 < pick[slow]->us1) faster.push_back(w);
+        const KernelEntry *next = least(faster, [&](const KernelEntry &w) { return share(&w, n[slow]); },
+                                        [&](const KernelEntry &w) { return (double)n[slow] * w.ctas / 148; });
         if (!next) return pick;
         const double then = used - share(pick[slow], n[slow]) + share(next, n[slow]);
         if (then > 1.0) return pick;
